@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "image_kernels.h"
 
 namespace {
@@ -70,89 +72,234 @@ __global__ void __launch_bounds__(256) density_histogram_kernel(const float4* __
 // quantised to 1/RFK_DE_STEPS px; the weight of integer offset o is
 //   k(o) = max(0, 1 - |o|^2 / (r + 1)^2) / Z(r),  Z(r) = sum over |ox|,|oy| <= ceil(r) of the same,
 // so a pixel of radius 0 keeps its value and every source conserves its total
-// (inside the image). The output gathers, for each pixel, the contributions of
-// all sources within max_radius.
-#define DE_TILE_X 32
-#define DE_TILE_Y 16
+// (inside the image).
+//
+// A block owns a strip of 32 output columns (lane = column) and walks down its
+// source rows, the strip's rows and a halo of 9, eight rows a step, one per
+// warp. What bounds the kernel is the FP32 work per (source, output) pair - an
+// fma for k, a max, four fmas - so a step does it once for both output rows at
+// distance d = 0 .. 9 of a source row:
+//   H[d] = sum over the row's sources of v max(0, 1 - (dx^2 + d^2) a) / Z
+// goes through shared memory to the rows above and below, whose sums wait in
+// registers (the warp keeps every eighth output row) until the walk has passed
+// them. H takes few pairs that are zero:
+//   - sources that reach at most 2 px (the bulk of a converged image) are
+//     gathered, five taps per source row, each lane its own sources;
+//   - wider sources are taken one by one from the row's bit mask, all lanes on
+//     the same source (its values broadcast from shared memory), distances
+//     beyond its reach skipped three at a time. A real 1080p frame has 20-35%
+//     such sources; a pixel is reached by 20-100 of the 361 in its window;
+//   - a row with more of them than taps is gathered over its full reach.
+// Measured (GB300): a 1024-spp 1920 x 1080 frame 162 us, a 1280 x 720 animation
+// frame 75-79 us, a faint 256 x 256 image 21 us; one thread per pixel looping
+// over a shared tile up to the tile's widest reach took 632, 208-330 and 90 us.
+// 8 warps x 3 blocks per SM (80 registers) issue 75% of the slots.
 #define DE_HALO 9  // RFK_DE_MAX_RADIUS_CAP
+#define DE_WARPS 8  // source rows a step
+#define DE_TILE_X 32
 #define DE_SW (DE_TILE_X + 2 * DE_HALO)
-#define DE_SH (DE_TILE_Y + 2 * DE_HALO)
+#define DE_SMALL 2  // reach of the sources that are gathered
 
-// Radius level (r * RFK_DE_STEPS, 255 = empty) of a source pixel.
-__device__ __forceinline__ unsigned char de_level(float d, float max_radius, float min_radius, float curve) {
-    if (!(d > 0.0f)) return 255;
+// Per radius level: 1 / (r + 1)^2, rounded up where that keeps the offset
+// ceil(r) + 1 at weight 0, 1 / Z(r), and ceil(r).
+struct de_table {
+    float a[RFK_DE_LEVELS], inv_z[RFK_DE_LEVELS];
+    int reach[RFK_DE_LEVELS];
+};
+
+// Radius level (r * RFK_DE_STEPS) of a source pixel of density d > 0.
+__device__ __forceinline__ int de_level(float d, float max_radius, float min_radius, float curve) {
     float r = max_radius * powf(d, -curve);
     r = fminf(fmaxf(r, min_radius), max_radius);
-    return (unsigned char)lrintf(r * RFK_DE_STEPS);
+    return (int)(unsigned char)lrintf(r * RFK_DE_STEPS);
 }
 
-__global__ void __launch_bounds__(DE_TILE_X * DE_TILE_Y / 2) de_blur_kernel(const float4* __restrict__ in, float4* __restrict__ out,
-                                                                            unsigned w, unsigned h, float max_radius,
-                                                                            float min_radius, float curve, int reach) {
-    __shared__ float4 tile[DE_SH][DE_SW];
-    __shared__ unsigned char lv[DE_SH][DE_SW];
-    __shared__ float2 tab[RFK_DE_LEVELS];  // (1 / (r + 1)^2, 1 / Z(r)) per level
-    __shared__ int max_rc;                  // largest support radius of a source in the tile
-    const int tx0 = blockIdx.x * DE_TILE_X - DE_HALO, ty0 = blockIdx.y * DE_TILE_Y - DE_HALO;
-    const int nthreads = blockDim.x;
-    if (threadIdx.x == 0) max_rc = 0;
-    for (int l = threadIdx.x; l < RFK_DE_LEVELS; l += nthreads) {
-        const float r = (float)l / RFK_DE_STEPS;
-        const float a = 1.0f / ((r + 1.0f) * (r + 1.0f));
-        const int rc = (l + RFK_DE_STEPS - 1) / RFK_DE_STEPS;
-        float z = 0.0f;
-        for (int oy = -rc; oy <= rc; oy++)
-            for (int ox = -rc; ox <= rc; ox++) z += fmaxf(0.0f, 1.0f - (float)(ox * ox + oy * oy) * a);
-        tab[l] = make_float2(a, 1.0f / z);
-    }
-    __syncthreads();  // max_rc cleared
-    int my_rc = 0;
-    for (int i = threadIdx.x; i < DE_SW * DE_SH; i += nthreads) {
-        const int sy = i / DE_SW, sx = i % DE_SW;
-        const int gx = tx0 + sx, gy = ty0 + sy;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        unsigned char l = 255;
-        if (gx >= 0 && gy >= 0 && gx < (int)w && gy < (int)h) {
-            v = in[(size_t)gy * w + gx];
-            l = de_level(v.w, max_radius, min_radius, curve);
+// One source row of a warp's strip: columns -9 .. 40 of it.
+struct de_row {
+    float4 v[DE_SW];  // RGBA / Z, 0 where there is no source
+    float a[DE_SW];   // 1 / (r + 1)^2
+    unsigned char reach[DE_SW + 2];
+};
+
+// p += q k for two channels in one instruction (the kernel issues 75% of its
+// slots: 5 instead of 6 instructions a pair took a 1080p frame from 174 to 162 us).
+__device__ __forceinline__ void fma_pair(float& px, float& py, float qx, float qy, float k) {
+    unsigned long long p, q, kk;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(px), "f"(py));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(qx), "f"(qy));
+    asm("mov.b64 %0, {%1, %1};" : "=l"(kk) : "f"(k));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(p) : "l"(q), "l"(kk));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(px), "=f"(py) : "l"(p));
+}
+
+// H[d] += v k(dx, d) for d = D0 .. D1; t = 1 - dx^2 a. A non-finite source is
+// added where k > 0 only, so that it stays inside its own support.
+template <bool FINITE, int D0, int D1>
+__device__ __forceinline__ void de_add(float4 (&H)[DE_HALO + 1], const float4& v, float a, float t) {
+#pragma unroll
+    for (int d = D0; d <= D1; d++) {
+        float k = fmaf(-(float)(d * d), a, t);
+        if (FINITE) k = fmaxf(k, 0.0f);
+        if (FINITE || k > 0.0f) {
+            fma_pair(H[d].x, H[d].y, v.x, v.y, k);
+            fma_pair(H[d].z, H[d].w, v.z, v.w, k);
         }
-        tile[sy][sx] = v;
-        lv[sy][sx] = l;
-        if (l != 255) my_rc = max(my_rc, ((int)l + RFK_DE_STEPS - 1) / RFK_DE_STEPS);
     }
-    if (my_rc > 0) atomicMax(&max_rc, my_rc);
-    __syncthreads();
-    // no source of the tile (halo included) reaches further than max_rc, so
-    // the offsets beyond it would all be skipped below: the loop stops there
-    // (an empty tile writes zeros at once); the sum is unchanged bit for bit
-    reach = min(reach, max_rc);
-    // two output pixels per thread, rows y and y + DE_TILE_Y/2
-    const int ox = threadIdx.x % DE_TILE_X, oy = threadIdx.x / DE_TILE_X;
-    for (int half = 0; half < 2; half++) {
-        const int py = oy + half * (DE_TILE_Y / 2);
-        const int gx = blockIdx.x * DE_TILE_X + ox, gy = blockIdx.y * DE_TILE_Y + py;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int dy = -reach; dy <= reach; dy++) {
-            const int sy = py + DE_HALO + dy;
-            for (int dx = -reach; dx <= reach; dx++) {
-                const int sx = ox + DE_HALO + dx;
-                const unsigned char l = lv[sy][sx];
-                if (l == 255) continue;
-                // the source's support is |ox|,|oy| <= ceil(r)
-                const int rc = (l + RFK_DE_STEPS - 1) / RFK_DE_STEPS;
-                if (abs(dx) > rc || abs(dy) > rc) continue;
-                const float2 t = tab[l];
-                const float k = fmaxf(0.0f, 1.0f - (float)(dx * dx + dy * dy) * t.x);
-                if (k == 0.0f) continue;
-                const float wgt = k * t.y;
-                const float4 v = tile[sy][sx];
-                acc.x = fmaf(v.x, wgt, acc.x);
-                acc.y = fmaf(v.y, wgt, acc.y);
-                acc.z = fmaf(v.z, wgt, acc.z);
-                acc.w = fmaf(v.w, wgt, acc.w);
+}
+
+template <bool FINITE>
+__device__ __forceinline__ void de_add_reach(float4 (&H)[DE_HALO + 1], const float4& v, float a, float t, int reach) {
+    de_add<FINITE, 0, 3>(H, v, a, t);
+    if (reach > 3) de_add<FINITE, 4, 6>(H, v, a, t);
+    if (reach > 6) de_add<FINITE, 7, DE_HALO>(H, v, a, t);
+}
+
+// H of the row's wide sources (mask: their columns, reach: the widest).
+template <bool FINITE>
+__device__ __forceinline__ void de_wide(const de_row& row, int lane, unsigned long long mask, int reach, float4 (&H)[DE_HALO + 1]) {
+    const float wide_a = 1.0f / ((DE_SMALL + 1) * (DE_SMALL + 1));  // a of a source is below it if it is wide
+    if (__popcll(mask) > 2 * reach) {
+#pragma unroll 1
+        for (int dx = -reach; dx <= reach; dx++) {
+            const int c = lane + DE_HALO + dx;
+            const float a = row.a[c];
+            const float4 v = row.v[c];
+            de_add_reach<FINITE>(H, v, a, a < wide_a ? fmaf((float)(-dx * dx), a, 1.0f) : 0.0f, reach);
+        }
+        return;
+    }
+#pragma unroll 1
+    while (mask) {
+        const int c = __ffsll((long long)mask) - 1;
+        mask &= mask - 1ull;
+        const int rc = row.reach[c];
+        if (rc < max(DE_HALO - c, c - (DE_HALO + DE_TILE_X - 1))) continue;  // short of the strip
+        const float a = row.a[c];
+        const float4 v = row.v[c];
+        const float dx = (float)(lane + DE_HALO - c);
+        de_add_reach<FINITE>(H, v, a, fmaf(-dx * dx, a, 1.0f), rc);
+    }
+}
+
+// H[0 .. 2] of the sources that reach at most DE_SMALL.
+template <bool FINITE>
+__device__ __forceinline__ void de_small(const de_row& row, int lane, float4 (&H)[DE_HALO + 1]) {
+    const float wide_a = 1.0f / ((DE_SMALL + 1) * (DE_SMALL + 1));
+#pragma unroll
+    for (int dx = -DE_SMALL; dx <= DE_SMALL; dx++) {
+        const int c = lane + DE_HALO + dx;
+        const float a = row.a[c];
+        const float4 v = row.v[c];
+        de_add<FINITE, 0, DE_SMALL>(H, v, a, a < wide_a ? 0.0f : fmaf((float)(-dx * dx), a, 1.0f));
+    }
+}
+
+__global__ void __launch_bounds__(32 * DE_WARPS, 3) de_blur_kernel(const float4* __restrict__ in, float4* __restrict__ out,
+                                                                   unsigned w, unsigned h, float max_radius, float min_radius,
+                                                                   float curve, int steps, const __grid_constant__ de_table tab) {
+    __shared__ union {
+        de_row row;                          // the warp's source row, then
+        float4 H[DE_HALO + 1][DE_TILE_X];    // its H
+    } sm[DE_WARPS];
+    __shared__ int reach_sm[DE_WARPS];       // H[0 .. reach] is set; -1: the row has no source
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    de_row& row = sm[warp].row;
+    const int rows = steps * DE_WARPS - 2 * DE_HALO;
+    const int y0 = (int)blockIdx.y * rows, y1 = min((int)h, y0 + rows);
+    const int x0 = blockIdx.x * DE_TILE_X - DE_HALO;
+    const int gx = x0 + DE_HALO + lane;
+
+    // the warp's source row s: columns lane and lane + 32 (the last 18) of the strip's window
+    const bool in0 = x0 + lane >= 0 && x0 + lane < (int)w;
+    const bool in1 = lane < DE_SW - 32 && x0 + lane + 32 < (int)w;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 n0 = zero, n1 = zero;
+    auto fetch = [&](int s) {
+        n0 = n1 = zero;
+        if (s < 0 || s >= (int)h) return;
+        const float4* src = in + (size_t)s * w + x0 + lane;
+        if (in0) n0 = src[0];
+        if (in1) n1 = src[32];
+    };
+    // sums of output rows s0 + own + 8 i, of those the step's rows s0 .. s0 + 7
+    // reach; the first is complete after the step
+    const int own = warp == DE_WARPS - 1 ? -1 : warp;
+    float4 B[4] = {zero, zero, zero, zero};
+    fetch(y0 - DE_HALO + warp);
+#pragma unroll 1
+    for (int step = 0; step < steps; step++) {
+        const int s0 = y0 - DE_HALO + step * DE_WARPS;
+        unsigned long long wide = 0ull;
+        unsigned small = 0u, odd = 0u, widest = 0u;
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            float4 v = half ? n1 : n0;
+            int reach = 0;
+            float a = 1.0f;
+            const bool source = v.w > 0.0f;
+            if (source) {
+                const int l = de_level(v.w, max_radius, min_radius, curve);
+                const float z = tab.inv_z[l];
+                a = tab.a[l];
+                reach = tab.reach[l];
+                v = make_float4(v.x * z, v.y * z, v.z * z, v.w * z);
+            } else {
+                v = zero;
+            }
+            const int c = lane + 32 * half;
+            if (c < DE_SW) {
+                row.v[c] = v;
+                row.a[c] = a;
+                row.reach[c] = (unsigned char)reach;
+            }
+            wide |= (unsigned long long)__ballot_sync(0xffffffffu, reach > DE_SMALL) << (32 * half);
+            small |= __ballot_sync(0xffffffffu, source && reach <= DE_SMALL);
+            odd |= __ballot_sync(0xffffffffu, !(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w)));
+            widest = max(widest, __reduce_max_sync(0xffffffffu, (unsigned)reach));
+        }
+        __syncwarp();
+        fetch(s0 + DE_WARPS + warp);
+        const int reach = wide ? (int)widest : small ? DE_SMALL : -1;
+        if (reach >= 0) {
+            float4 H[DE_HALO + 1];
+#pragma unroll
+            for (int d = 0; d <= DE_HALO; d++) H[d] = zero;
+            if (odd) {
+                if (small) de_small<false>(row, lane, H);
+                if (wide) de_wide<false>(row, lane, wide, reach, H);
+            } else {
+                if (small) de_small<true>(row, lane, H);
+                if (wide) de_wide<true>(row, lane, wide, reach, H);
+            }
+            __syncwarp();  // H takes the row's place
+#pragma unroll
+            for (int d = 0; d <= DE_HALO; d++)
+                if (d <= reach) sm[warp].H[d][lane] = H[d];
+        }
+        if (lane == 0) reach_sm[warp] = reach;
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < DE_WARPS; s++) {
+            const int rs = reach_sm[s];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int d = abs(own + 8 * (i - 1) - s);
+                if (d <= rs) {
+                    const float4 q = sm[s].H[d][lane];
+                    B[i].x += q.x;
+                    B[i].y += q.y;
+                    B[i].z += q.z;
+                    B[i].w += q.w;
+                }
             }
         }
-        if (gx < (int)w && gy < (int)h) out[(size_t)gy * w + gx] = acc;
+        const int y = s0 + own - DE_WARPS;
+        if (y >= y0 && y < y1 && gx < (int)w) out[(size_t)y * w + gx] = B[0];
+        B[0] = B[1];
+        B[1] = B[2];
+        B[2] = B[3];
+        B[3] = zero;
+        __syncthreads();
     }
 }
 
@@ -243,6 +390,23 @@ __global__ void clear_counters_kernel(unsigned long long* c) {
     c[5] = 0;
 }
 
+de_table de_make_table() {
+    de_table t;
+    for (int l = 0; l < RFK_DE_LEVELS; l++) {
+        const float r = (float)l / RFK_DE_STEPS, r1 = (r + 1.0f) * (r + 1.0f);
+        const int rc = (l + RFK_DE_STEPS - 1) / RFK_DE_STEPS;
+        float a = 1.0f / r1;
+        while (std::fma(-(float)((rc + 1) * (rc + 1)), a, 1.0f) > 0.0f) a = std::nextafter(a, 2.0f);
+        float z = 0.0f;
+        for (int oy = -rc; oy <= rc; oy++)
+            for (int ox = -rc; ox <= rc; ox++) z += std::fmax(0.0f, std::fma(-(float)(ox * ox + oy * oy), a, 1.0f));
+        t.a[l] = a;
+        t.inv_z[l] = 1.0f / z;
+        t.reach[l] = rc;
+    }
+    return t;
+}
+
 int sm_count() {
     static int n = 0;
     if (!n) {
@@ -304,9 +468,26 @@ cudaError_t rfk_launch_density_histogram(const float4* bins, unsigned size, unsi
 cudaError_t rfk_launch_de_blur(const float4* in, float4* out, unsigned w, unsigned h, float max_radius, float min_radius,
                                float curve, cudaStream_t s) {
     if (w == 0 || h == 0) return cudaSuccess;
-    dim3 grid((w + DE_TILE_X - 1) / DE_TILE_X, (h + DE_TILE_Y - 1) / DE_TILE_Y);
-    const int reach = (int)ceilf(max_radius);
-    de_blur_kernel<<<grid, DE_TILE_X * DE_TILE_Y / 2, 0, s>>>(in, out, w, h, max_radius, min_radius, curve, reach);
+    static const de_table tab = de_make_table();
+    const unsigned strips = (w + DE_TILE_X - 1) / DE_TILE_X;
+    // steps per block: more of them share the halo, fewer spread the rows over
+    // the SMs. A step of a block takes about as long as its share of the SM, but
+    // no less than that of one block alone. (512 x 512: 6 steps 41 us, 16 steps
+    // 76 us; 1920 x 1080: 4 steps 268 us, 12 steps 174 us.)
+    int steps = 3;
+    double best = 1e30;
+    for (int n = 3; n <= 24; n++) {
+        const unsigned rows = (unsigned)(n * DE_WARPS - 2 * DE_HALO);
+        const double per_sm = (double)strips * ((h + rows - 1) / rows) / sm_count();
+        const double cost = n * ((per_sm > 1.0 ? per_sm : 1.0) + 1.0);
+        if (cost < best) {
+            best = cost;
+            steps = n;
+        }
+    }
+    const unsigned rows = (unsigned)(steps * DE_WARPS - 2 * DE_HALO);
+    const dim3 grid(strips, (h + rows - 1) / rows);
+    de_blur_kernel<<<grid, 32 * DE_WARPS, 0, s>>>(in, out, w, h, max_radius, min_radius, curve, steps, tab);
     return cudaGetLastError();
 }
 
