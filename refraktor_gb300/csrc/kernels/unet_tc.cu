@@ -54,6 +54,7 @@ struct conv_args {
     const bf16* mask;
     int mask_cstride, mask_coff;
     int accumulate;
+    int tma_out;  // bf16 output through shared memory and TMA stores
     int* err;
 };
 
@@ -74,7 +75,8 @@ template <int BK, int BN, int MODE>
 struct conv_cfg {
     // R image rows per tile (R accumulators of 128 x BN): small-N layers move
     // R times the bytes per pipeline stage, so the stage round trip is shared
-    static constexpr int R = BN >= 128 ? 1 : 128 / BN;
+    // (128 channels: two rows share each weight tile)
+    static constexpr int R = BN == 128 && MODE == 1 ? 2 : BN >= 96 ? 1 : 128 / BN;
     static constexpr int A_PIX = MODE ? 136 : 128;                // pixel lines per image row
     static constexpr int A_ROWS = MODE == 2 ? R + 2 : R;           // image rows per A box
     static constexpr uint32_t A_ROW = (uint32_t)A_PIX * BK * 2u;   // one image row segment
@@ -87,12 +89,15 @@ struct conv_cfg {
     static constexpr uint32_t LOAD_BYTES = A_BYTES + NB * B_TILE;  // bytes the TMA writes per stage
     static constexpr uint32_t STAGE_BYTES = (LOAD_BYTES + 1023u) & ~1023u;
     static constexpr int TAPS = MODE == 2 ? 1 : (MODE == 1 ? 3 : 9);  // K blocks per input channel block
+    // output staging: two tiles of 128 pixels x OC channels
+    static constexpr int OC = BN % 64 == 0 ? 64 : 32;
+    static constexpr uint32_t OUT_TILE = 128u * OC * 2u;
     // one persistent CTA per SM: as many stages as fit in ~208 KB, at most 8
-    static constexpr uint32_t BUDGET = 212992u;
+    static constexpr uint32_t BUDGET = 229376u - 2u * OUT_TILE;
     static constexpr int STAGES = ((BUDGET - B_RES) / STAGE_BYTES > 8) ? 8 : (int)((BUDGET - B_RES) / STAGE_BYTES);
-    static constexpr uint32_t SMEM = B_RES + STAGES * STAGE_BYTES + 1024u;
-    static constexpr uint32_t TMEM_COLS = 2u * R * BN;  // two sets of R accumulators
-    static_assert(MODE == 0 || (A_ROW % 512u == 0 && A_BYTES % 1024u == 0 && B_TILE % 1024u == 0 && B_RES % 1024u == 0),
+    static constexpr uint32_t SMEM = B_RES + STAGES * STAGE_BYTES + 2u * OUT_TILE + 1024u;
+    static constexpr uint32_t TMEM_COLS = BN == 96 ? 256u : 2u * R * BN;  // two sets of R accumulators
+    static_assert(MODE == 0 || (A_ROW % 512u == 0 && A_BYTES % (16u * BK) == 0 && B_TILE % 1024u == 0 && B_RES % 1024u == 0),
                   "tap-reuse tiles must stay swizzle-aligned");
     static_assert(STAGES >= 2, "at least two stages");
 };
@@ -129,6 +134,152 @@ __device__ __forceinline__ void load_bf16x16(const bf16* src, float (&v)[16]) {
 
 constexpr int kEpiWarps = 8;  // two warps per TMEM lane quarter, each half of the columns
 
+// Bias, ReLU and ReLU-derivative mask of N consecutive output channels of one pixel.
+template <int N>
+__device__ __forceinline__ void conv_activate(const conv_args& p, float (&v)[N], int ch, size_t pix, bool valid) {
+    if (p.bias) {
+        const float4* bb = reinterpret_cast<const float4*>(p.bias + ch);
+#pragma unroll
+        for (int q = 0; q < N / 4; q++) {
+            const float4 f = __ldg(bb + q);
+            v[4 * q] += f.x;
+            v[4 * q + 1] += f.y;
+            v[4 * q + 2] += f.z;
+            v[4 * q + 3] += f.w;
+        }
+    }
+    if (p.relu) {
+#pragma unroll
+        for (int j = 0; j < N; j++) v[j] = fmaxf(v[j], 0.0f);
+    }
+    if (p.mask && valid) {
+#pragma unroll
+        for (int g = 0; g < N; g += 16) {
+            float m[16];
+            load_bf16x16(p.mask + pix * p.mask_cstride + p.mask_coff + ch + g, m);
+#pragma unroll
+            for (int j = 0; j < 16; j++) v[g + j] = m[j] > 0.0f ? v[g + j] : 0.0f;
+        }
+    }
+}
+
+// Drains R accumulator rows of 128 x BN (TMEM columns from acc on) into the
+// output: image rows y0 + r, pixels xt * 128 ..; warp (quarter, half) reads
+// TMEM lanes 32 quarter .. 32 quarter + 31 = pixels, columns of its half.
+// f32 and accumulating outputs: each lane stores its pixel's channels.
+template <int R, int BN>
+__device__ __forceinline__ void conv_epilogue(const conv_args& p, uint32_t acc, int img, int y0, int xt, int n0, int quarter,
+                                              int half, int lane) {
+    const int x = xt * 128 + quarter * 32 + lane;
+#pragma unroll 1
+    for (int r = 0; r < R; r++) {
+        const int y = y0 + r;
+        const bool valid = x < p.w && y < p.h;
+        const size_t pix = ((size_t)img * p.h + (valid ? y : 0)) * p.w + (valid ? x : 0);
+#pragma unroll 1
+        for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 16) {
+            float v[16];
+            tc::tmem_ld16(acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(r * BN + c), v);
+            const int ch = n0 + c;
+            if (!valid) continue;
+            if (p.bias) {
+                const float4* bb = reinterpret_cast<const float4*>(p.bias + ch);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const float4 f = __ldg(bb + q);
+                    v[4 * q] += f.x;
+                    v[4 * q + 1] += f.y;
+                    v[4 * q + 2] += f.z;
+                    v[4 * q + 3] += f.w;
+                }
+            }
+            if (p.relu) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.0f);
+            }
+            if (p.mask) {
+                float m[16];
+                load_bf16x16(p.mask + pix * p.mask_cstride + p.mask_coff + ch, m);
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] = m[j] > 0.0f ? v[j] : 0.0f;
+            }
+            const size_t at = pix * p.out_cstride + p.out_coff + ch;
+            if (p.out_f32) {
+                float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at);
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float4 o = p.accumulate ? dst[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    dst[q] = make_float4(v[4 * q] + o.x, v[4 * q + 1] + o.y, v[4 * q + 2] + o.z, v[4 * q + 3] + o.w);
+                }
+            } else {
+                bf16* dst = static_cast<bf16*>(p.out) + at;
+                if (p.accumulate) {
+                    float o[16];
+                    load_bf16x16(dst, o);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] += o[j];
+                }
+                store_bf16x16(dst, v);
+            }
+        }
+    }
+}
+
+// As conv_epilogue, for bf16 outputs: a row's 128 pixels x OC channels are
+// assembled in shared memory (128- or 64-byte rows, swizzled as the tensor map
+// has it, so the lanes' 16-byte writes meet no bank twice) and leave as one TMA
+// store, or four with up2 (the 2 x 2 pixels of each). A lane storing its own
+// pixel's 32-byte pieces touches 32 lines per instruction: for a 1080p image the
+// 64-channel layer with up2 took 141 us that way and takes 66, the 128-channel one
+// 88 and 45, a plain 32 -> 64 layer 47 and 39.
+// Two staging tiles; `flip` counts the tiles written so far.
+template <int R, int BN, int OC>
+__device__ __forceinline__ void conv_epilogue_tma(const conv_args& p, const CUtensorMap* map, uint8_t* outbuf, uint32_t acc, int img,
+                                                  int y0, int xt, int n0, int quarter, int half, int lane, uint32_t& flip) {
+    constexpr int W = OC / 2;  // channels of a warp's half
+    const int px = quarter * 32 + lane, x = xt * 128 + px;
+    const bool leader = threadIdx.x == 0;
+#pragma unroll 1
+    for (int r = 0; r < R && y0 + r < p.h; r++) {
+        const int y = y0 + r;
+        const bool valid = x < p.w;
+        const size_t pix = ((size_t)img * p.h + y) * p.w + (valid ? x : 0);
+#pragma unroll 1
+        for (int c = 0; c < BN; c += OC, flip++) {
+            float v[W];
+            const uint32_t at = acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(r * BN + c + half * W);
+            if constexpr (W == 32) tc::tmem_ld32(at, v);
+            else tc::tmem_ld16(at, v);
+            conv_activate<W>(p, v, n0 + c + half * W, pix, valid);
+            uint8_t* tile = outbuf + (flip & 1u) * (128u * OC * 2u);
+            // the tile's previous store has read it
+            if (leader) tc::tma_store_wait_read<1>();
+            tc::named_barrier(1, 32 * kEpiWarps);
+#pragma unroll
+            for (int q = 0; q < W / 8; q++) {
+                __nv_bfloat162 hh[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) hh[j] = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
+                const uint32_t k = (uint32_t)(half * (W / 8) + q);  // 16-byte piece of the pixel
+                const uint32_t sw = OC == 64 ? (k ^ ((uint32_t)px & 7u)) : (k ^ (((uint32_t)px >> 1) & 3u));
+                *reinterpret_cast<uint4*>(tile + px * (OC * 2) + sw * 16) = *reinterpret_cast<uint4*>(hh);
+            }
+            tc::fence_async();
+            tc::named_barrier(2, 32 * kEpiWarps);
+            if (leader) {
+                const int ch = p.out_coff + n0 + c, row = img * p.h + y;
+                if (p.up2) {
+#pragma unroll
+                    for (int d = 0; d < 4; d++) tc::tma_store_5d(map, tile, ch, d & 1, xt * 128, d >> 1, row);
+                } else {
+                    tc::tma_store_3d(map, tile, ch, xt * 128, row);
+                }
+                tc::tma_store_commit();
+            }
+        }
+    }
+}
+
 // Persistent: one CTA per SM walks the tiles (R rows x 128-pixel segment x BN
 // output channels) t = blockIdx.x, blockIdx.x + gridDim.x, ...
 // Warps 0-7: epilogue (warp w reads TMEM lane quarter w % 4, column half
@@ -137,7 +288,8 @@ constexpr int kEpiWarps = 8;  // two warps per TMEM lane quarter, each half of t
 // i + 1 run while the epilogue drains tile i (acc_full / acc_empty barriers).
 template <int BK, int BN, int MODE>
 __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUtensorMap tmA,
-                                                     const __grid_constant__ CUtensorMap tmB, conv_args p) {
+                                                     const __grid_constant__ CUtensorMap tmB,
+                                                     const __grid_constant__ CUtensorMap tmO, conv_args p) {
     using C = conv_cfg<BK, BN, MODE>;
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -147,6 +299,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint8_t* const res = base;                   // resident weights (MODE 2)
     uint8_t* const stages = base + C::B_RES;
+    uint8_t* const outbuf = stages + C::STAGES * C::STAGE_BYTES;
 
     const int ntn = p.cout / BN;                           // N tiles
     const int rows_t = (p.h + C::R - 1) / C::R;            // row groups per image
@@ -277,11 +430,12 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
         // epilogue: warps 0-7; TMEM lane 32 * (warp % 4) + lane = tile row,
         // columns [half * BN / 2, (half + 1) * BN / 2)
         const int quarter = warp & 3, half = warp >> 2;
+        uint32_t flip = 0;
         int i = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, i++) {
             const int b = i & 1;
-            bool got = tc::mbar_wait(&acc_full[b], (i >> 1) & 1);
-            got = __all_sync(0xffffffffu, got);
+            // all epilogue warps go on or stop together (they meet at barriers below)
+            const bool got = tc::named_barrier_all(1, 32 * kEpiWarps, tc::mbar_wait(&acc_full[b], (i >> 1) & 1));
             if (!got) {
                 if (lane == 0) atomicExch(&s_fail, 1);
                 break;
@@ -291,72 +445,17 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
             const int xt = mt % p.tiles_x;
             const int y0 = ((mt / p.tiles_x) % rows_t) * C::R;
             const int img = mt / (p.tiles_x * rows_t);
-            const int x = xt * 128 + quarter * 32 + lane;
-#pragma unroll 1
-            for (int r = 0; r < C::R; r++) {
-                const int y = y0 + r;
-                const bool valid = x < p.w && y < p.h;
-                const size_t pix = ((size_t)img * p.h + (valid ? y : 0)) * p.w + (valid ? x : 0);
-#pragma unroll 1
-                for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 16) {
-                    float v[16];
-                    tc::tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((b * C::R + r) * BN + c), v);
-                    const int ch = n0 + c;
-                    if (!valid) continue;
-                    if (p.bias) {
-                        const float4* bb = reinterpret_cast<const float4*>(p.bias + ch);
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const float4 f = __ldg(bb + q);
-                            v[4 * q] += f.x;
-                            v[4 * q + 1] += f.y;
-                            v[4 * q + 2] += f.z;
-                            v[4 * q + 3] += f.w;
-                        }
-                    }
-                    if (p.relu) {
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.0f);
-                    }
-                    if (p.mask) {
-                        float m[16];
-                        load_bf16x16(p.mask + pix * p.mask_cstride + p.mask_coff + ch, m);
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = m[j] > 0.0f ? v[j] : 0.0f;
-                    }
-                    const size_t at = pix * p.out_cstride + p.out_coff + ch;
-                    if (p.out_f32) {
-                        float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at);
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            float4 o = p.accumulate ? dst[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            dst[q] = make_float4(v[4 * q] + o.x, v[4 * q + 1] + o.y, v[4 * q + 2] + o.z, v[4 * q + 3] + o.w);
-                        }
-                    } else if (p.up2) {
-                        // nearest 2x upsampling: the four pixels (2x + dx, 2y + dy) of the
-                        // output image, which is (2h, 2w)
-#pragma unroll
-                        for (int d = 0; d < 4; d++) {
-                            const size_t pix2 = ((size_t)img * 2 * p.h + 2 * y + (d >> 1)) * (2 * (size_t)p.w) + 2 * x + (d & 1);
-                            store_bf16x16(static_cast<bf16*>(p.out) + pix2 * p.out_cstride + p.out_coff + ch, v);
-                        }
-                    } else {
-                        bf16* dst = static_cast<bf16*>(p.out) + at;
-                        if (p.accumulate) {
-                            float o[16];
-                            load_bf16x16(dst, o);
-#pragma unroll
-                            for (int j = 0; j < 16; j++) v[j] += o[j];
-                        }
-                        store_bf16x16(dst, v);
-                    }
-                }
-            }
+            if (p.tma_out)
+                conv_epilogue_tma<C::R, BN, C::OC>(p, &tmO, outbuf, tmem + (uint32_t)(b * C::R * BN), img, y0, xt, n0, quarter, half,
+                                                   lane, flip);
+            else
+                conv_epilogue<C::R, BN>(p, tmem + (uint32_t)(b * C::R * BN), img, y0, xt, n0, quarter, half, lane);
             // the accumulator may be overwritten once all epilogue warps have read it
             tc::fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[b]);
         }
+        if (threadIdx.x == 0) tc::tma_store_wait<0>();
     }
     tc::fence_before();
     __syncthreads();
@@ -554,7 +653,7 @@ bool make_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims
               const cuuint32_t* box, CUtensorMapSwizzle sw) {
     encode_fn fn = encoder();
     if (!fn) return false;
-    cuuint32_t es[4] = {1, 1, 1, 1};
+    cuuint32_t es[5] = {1, 1, 1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides_bytes, box, es,
               CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -577,7 +676,7 @@ int sm_count_cached() {
 }
 
 template <int BK, int BN, int MODE>
-cudaError_t launch_conv(const CUtensorMap& a, const CUtensorMap& b, const conv_args& p, cudaStream_t s) {
+cudaError_t launch_conv(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& o, const conv_args& p, cudaStream_t s) {
     using C = conv_cfg<BK, BN, MODE>;
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
@@ -586,7 +685,7 @@ cudaError_t launch_conv(const CUtensorMap& a, const CUtensorMap& b, const conv_a
     const long long tiles = (long long)p.n_img * ((p.h + C::R - 1) / C::R) * p.tiles_x * (p.cout / BN);
     if (tiles > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     const int grid = (int)std::min<long long>(tiles, sm_count_cached());
-    conv3x3_tc<BK, BN, MODE><<<grid, 32 * (kEpiWarps + 2), C::SMEM, s>>>(a, b, p);
+    conv3x3_tc<BK, BN, MODE><<<grid, 32 * (kEpiWarps + 2), C::SMEM, s>>>(a, b, o, p);
     return cudaGetLastError();
 }
 
@@ -621,13 +720,16 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
         return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weights) | reinterpret_cast<uintptr_t>(out)) & 63)
         return cudaErrorMisalignedAddress;
-    const int bn = pick_bn(cout);
+    const int bn = cout == 96 ? 96 : pick_bn(cout);
     // tap reuse: 32 output channels (4 rows per tile) load each input channel
     // block once for all nine taps (MODE 2, 32-channel K blocks so that three
-    // 70 KB stages fit); 64 (2 rows) once per tap row (MODE 1); wider tiles
-    // (1 row) once per tap (MODE 0)
-    // MODE 2 keeps one output tile's weights resident: cout == 32, at most 3 input blocks
-    const int mode = (bn == 32 && cout == 32 && cin <= 32 * 3) ? 2 : (bn <= 64 ? 1 : 0);
+    // 70 KB stages fit; it keeps one output tile's weights resident: cout == 32,
+    // at most 3 input blocks); up to 128 (1 or 2 rows) once per tap row (MODE 1),
+    // 256 (1 row) once per tap (MODE 0: three 32 KB weight tiles and the row leave
+    // one stage). 128 channels at 480 x 270: 384 -> 128 80 us with two rows per tile
+    // and tap rows, 135 with one row and taps; 96 channels (1080p) 189 us as one
+    // tile, 522 as three of 32.
+    const int mode = (bn == 32 && cout == 32 && cin <= 32 * 3) ? 2 : (bn <= 128 ? 1 : 0);
     const int bk = (mode != 2 && cin % 64 == 0 && in_coff % 64 == 0) ? 64 : 32;
     CUtensorMap ma, mb;
     const CUtensorMapSwizzle sw = bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
@@ -635,7 +737,7 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
         cuuint64_t dims[4] = {(cuuint64_t)in_cstride, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n_img};
         cuuint64_t str[3] = {(cuuint64_t)in_cstride * 2, (cuuint64_t)w * in_cstride * 2, (cuuint64_t)h * w * in_cstride * 2};
         // image rows and pixel lines of an A box, as conv_cfg<BK, BN, MODE>
-        const cuuint32_t rows = (bn >= 128 ? 1u : (cuuint32_t)(128 / bn)) + (mode == 2 ? 2u : 0u);
+        const cuuint32_t rows = (bn == 128 ? 2u : bn >= 96 ? 1u : (cuuint32_t)(128 / bn)) + (mode == 2 ? 2u : 0u);
         cuuint32_t box[4] = {(cuuint32_t)bk, mode ? 136u : 128u, rows, 1};
         if (!make_map(&ma, in, 4, dims, str, box, sw)) return cudaErrorInvalidValue;
     }
@@ -666,19 +768,44 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
     p.mask_coff = mask_coff;
     p.accumulate = accumulate;
     p.err = err;
+    p.tma_out = !p.out_f32 && !accumulate;
+    CUtensorMap mo{};
+    if (p.tma_out) {
+        // output rows of all images one after another; with up2 as (channel, x
+        // parity, x, y parity, y) of the (2h, 2w) image. Boxes of 128 pixels x 64 or
+        // 32 channels, as conv_cfg::OC; pixels past the width are clipped.
+        const cuuint32_t oc = bn % 64 == 0 ? 64u : 32u;
+        const CUtensorMapSwizzle osw = oc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+        const cuuint64_t pitch = (cuuint64_t)out_cstride * 2, rows_n = (cuuint64_t)n_img * h;
+        bool good;
+        if (p.up2) {
+            cuuint64_t dims[5] = {(cuuint64_t)out_cstride, 2, (cuuint64_t)w, 2, rows_n};
+            cuuint64_t str[4] = {pitch, 2 * pitch, 2 * (cuuint64_t)w * pitch, 4 * (cuuint64_t)w * pitch};
+            cuuint32_t box[5] = {oc, 1, 128, 1, 1};
+            good = make_map(&mo, out, 5, dims, str, box, osw);
+        } else {
+            cuuint64_t dims[3] = {(cuuint64_t)out_cstride, (cuuint64_t)w, rows_n};
+            cuuint64_t str[2] = {pitch, (cuuint64_t)w * pitch};
+            cuuint32_t box[3] = {oc, 128, 1};
+            good = make_map(&mo, out, 3, dims, str, box, osw);
+        }
+        if (!good) return cudaErrorInvalidValue;
+    }
     if (bk == 64) {
         switch (bn) {
-        case 256: return launch_conv<64, 256, 0>(ma, mb, p, s);
-        case 128: return launch_conv<64, 128, 0>(ma, mb, p, s);
-        case 64: return launch_conv<64, 64, 1>(ma, mb, p, s);
-        default: return launch_conv<64, 32, 1>(ma, mb, p, s);
+        case 256: return launch_conv<64, 256, 0>(ma, mb, mo, p, s);
+        case 128: return launch_conv<64, 128, 1>(ma, mb, mo, p, s);
+        case 96: return launch_conv<64, 96, 1>(ma, mb, mo, p, s);
+        case 64: return launch_conv<64, 64, 1>(ma, mb, mo, p, s);
+        default: return launch_conv<64, 32, 1>(ma, mb, mo, p, s);
         }
     }
     switch (bn) {
-    case 256: return launch_conv<32, 256, 0>(ma, mb, p, s);
-    case 128: return launch_conv<32, 128, 0>(ma, mb, p, s);
-    case 64: return launch_conv<32, 64, 1>(ma, mb, p, s);
-    default: return mode == 2 ? launch_conv<32, 32, 2>(ma, mb, p, s) : launch_conv<32, 32, 1>(ma, mb, p, s);
+    case 256: return launch_conv<32, 256, 0>(ma, mb, mo, p, s);
+    case 128: return launch_conv<32, 128, 1>(ma, mb, mo, p, s);
+    case 96: return launch_conv<32, 96, 1>(ma, mb, mo, p, s);
+    case 64: return launch_conv<32, 64, 1>(ma, mb, mo, p, s);
+    default: return mode == 2 ? launch_conv<32, 32, 2>(ma, mb, mo, p, s) : launch_conv<32, 32, 1>(ma, mb, mo, p, s);
     }
 }
 
