@@ -182,7 +182,7 @@ struct rfk_denoiser {
     void forward(workspace& s, cudaStream_t st, bool infer = false) {
         const int n = s.n, H = s.h, W = s.w;
         const int H2 = H / 2, W2 = W / 2, H3 = H / 4, W3 = W / 4, H4 = H / 8, W4 = W / 8;
-        const int R = RFK_UNET_RELU;
+        const int A = infer ? RFK_UNET_ANY_ORDER : 0, R = RFK_UNET_RELU | A;
         conv(L_IN, s.x, H, W, n, 32, 0, s.a1, 32, 0, R, st);
         conv(E1B, s.a1, H, W, n, 32, 0, s.cat1, 96, 64, R, st);
         cuda_check(rfk_unet_avgpool(s.cat1, n, H, W, 96, 64, 32, s.p1, st), "pool");
@@ -216,7 +216,7 @@ struct rfk_denoiser {
         }
         conv(D1A, s.cat1, H, W, n, 96, 0, s.e1, 32, 0, R, st);
         conv(D1B, s.e1, H, W, n, 32, 0, s.d1, 32, 0, R, st);
-        conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 32, 0, RFK_UNET_F32OUT, st);
+        conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 32, 0, RFK_UNET_F32OUT | A, st);
     }
 
     // Gradients of layer l from dY (dense, cout channels, pre-activation) and
@@ -229,7 +229,7 @@ struct rfk_denoiser {
         cuda_check(rfk_unet_bias_grad(dy, P, y.d.cout, y.bg, st), "bias grad");
         cuda_check(rfk_unet_wgrad3x3(dy, x, x_cstride, x_coff, n, h, w, y.d.cout, y.d.cin, y.g, d_err, st), "wgrad");
         if (dx)
-            cuda_check(rfk_unet_conv3x3(dy, n, h, w, y.d.cout, 0, y.d.cout, y.wb, y.d.cin, nullptr, 0, dx, dx_cstride, dx_coff,
+            cuda_check(rfk_unet_conv3x3(dy, n, h, w, y.d.cout, 0, y.d.cout, y.wb, y.d.cin, nullptr, RFK_UNET_ANY_ORDER, dx, dx_cstride, dx_coff,
                                         mask, y.d.cin, 0, 0, d_err, st),
                        "dgrad");
     }

@@ -53,10 +53,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Bounded wait for the phase with the given parity; false after the limit.
+// The usual wait ends within a few polls; %globaltimer is read only after 64 of
+// them, for reading it takes longer than such a wait.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    if (mbar_try_wait(bar, parity)) return true;
+    for (int i = 0; i < 64; i++)
+        if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = now_ns();
-    for (uint32_t i = 0; i < kWaitIters; i++) {
+    for (uint32_t i = 1; i < kWaitIters; i++) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 63u) == 0 && now_ns() - t0 > kWaitNs) return false;
     }
@@ -106,17 +109,24 @@ __device__ __forceinline__ void tma_store_wait() {
     asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// Barrier `id` (1-15) among `threads` threads of the block.
+// Barrier `id` (1-15) among `threads` threads of the block, whole warps. The
+// warp is brought together before and after it: lanes come here from polling
+// loops and single-lane branches, and what follows are .aligned instructions.
 __device__ __forceinline__ void named_barrier(int id, int threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+    __syncwarp();
+    asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+    __syncwarp();
 }
+
 // As named_barrier; whether `ok` holds in all of its threads.
 __device__ __forceinline__ bool named_barrier_all(int id, int threads, bool ok) {
     uint32_t r;
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n bar.red.and.pred q, %1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
+    __syncwarp();
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n barrier.cta.red.and.pred q, %1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
                  : "=r"(r)
                  : "r"(id), "r"(threads), "r"((uint32_t)ok)
                  : "memory");
+    __syncwarp();
     return r != 0;
 }
 
@@ -135,22 +145,42 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// tcgen05.mma and commit take their operands from uniform registers. In a branch
+// that one lane takes, the compiler keeps descriptors in per-lane registers and
+// moves them over before every instruction, which made an MMA of 45-56 cycles
+// take 120-160 to issue. So a whole warp runs the issuing loop, with warp-uniform
+// operands and control flow (waits through all_lanes), and the instruction
+// itself is predicated: `one` is nonzero in the issuing lane only.
+// The descriptors' high words are constants of the layout and only the low words
+// (start address, leading offset) are passed, for the same reason.
 // D[tmem] (+)= A[smem] * B[smem]^T, bf16 inputs, f32 accumulator.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+template <uint32_t AHI, uint32_t BHI>
+__device__ __forceinline__ void mma_bf16(uint32_t one, uint32_t d_tmem, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                         uint32_t accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n .reg .pred p, q;\n .reg .b64 da, db;\n mov.b64 da, {%1, %6};\n mov.b64 db, {%2, %7};\n"
+        " setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(one), "n"(AHI), "n"(BHI)
         : "memory");
 }
 
-// Arrives on `bar` once every tcgen05.mma issued so far by this thread is done.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// Arrives on `bar` once every tcgen05.mma issued so far by the issuing lane is done.
+__device__ __forceinline__ void mma_commit(uint32_t one, uint64_t* bar) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+        " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)),
+        "r"(one)
+        : "memory");
 }
+
+// A wait of every lane of the warp; the same answer in all of them.
+__device__ __forceinline__ bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
 
 // 32 consecutive f32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,"
         "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -164,9 +194,29 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// As tmem_ld32 for the raw bits, without waiting: tmem_ld_wait() before use.
+__device__ __forceinline__ void tmem_ld32_start(uint32_t taddr, uint32_t (&r)[32]) {
+    __syncwarp();
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,"
+        "%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+// Waits for this thread's TMEM loads; the registers named are their results.
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[32], uint32_t (&b)[32], uint32_t (&c)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; i++) asm volatile("" : "+r"(a[i]), "+r"(b[i]), "+r"(c[i]));
+}
+
 // 16 consecutive f32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
@@ -177,44 +227,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// K-major operand tile in shared memory written by TMA with a row of
-// `row_bytes` (128 or 64) and the matching swizzle; rows are `row_bytes`
-// apart, 8-row groups (the swizzle atom) `8 * row_bytes` apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t row_bytes) {
-    const uint64_t layout = (row_bytes == 128) ? 2ull : 4ull;
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)1u << 16;                                // leading byte offset (unused when swizzled)
-    d |= (uint64_t)(((8u * row_bytes) >> 4) & 0x3FFFu) << 32;  // stride byte offset: 8-row group
-    d |= (uint64_t)1u << 46;                                // descriptor version
-    d |= layout << 61;
-    return d;
+// Descriptor of an operand tile in shared memory that TMA wrote with a row of
+// `row_bytes` (128 or 64) and the matching swizzle, as two words: the high word
+// depends on the layout only, the low word on the start address.
+// K-major: rows are `row_bytes` apart, 8-row groups (the swizzle atom)
+// 8 * row_bytes apart (the stride byte offset; the leading one is unused).
+// MN-major (the M or N index contiguous; boxes of row_bytes x K rows, one per
+// group of row_bytes / 2 M or N elements, `group_stride` bytes apart): the
+// stride byte offset is the 8-row K group, the leading byte offset the group
+// stride (checked on the GPU against a reference product for both swizzles and
+// one to four groups).
+// A start address may lie inside a tile that was written from a 1024-byte
+// aligned base: whole rows (pixel lines) past it, plus 32-byte K steps within a
+// row. The swizzle pattern is taken from the address bits of each access, as TMA
+// applied it, so the matrix base offset field stays 0.
+__host__ __device__ constexpr uint32_t desc_hi(uint32_t row_bytes) {
+    return ((8u * row_bytes) >> 4) | (1u << 14) | ((row_bytes == 128 ? 2u : 4u) << 29);
 }
-
-// As smem_desc, for a start address anywhere inside a tile that TMA wrote
-// from a 1024-byte aligned base: whole pixel lines (rows) past the base, plus
-// 32-byte K steps within a line. The swizzle pattern is taken from the
-// address bits of each access, as TMA applied it, so the matrix base offset
-// field stays 0.
-__device__ __forceinline__ uint64_t smem_desc_at(uint32_t saddr, uint32_t row_bytes) {
-    return smem_desc(saddr, row_bytes);
-}
-
-// MN-major operand tile (the M or N index contiguous) that TMA wrote as
-// boxes of `row_bytes` (128 or 64, with the matching swizzle) x K rows, one
-// box per group of row_bytes / 2 M or N elements, `group_stride` bytes apart:
-// the stride byte offset is the 8-row K group, the leading byte offset the
-// group stride (checked on the GPU against a reference product for both
-// swizzles and one to four groups).
-__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t row_bytes, uint32_t group_stride) {
-    const uint64_t layout = (row_bytes == 128) ? 2ull : 4ull;
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((group_stride >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)(((8u * row_bytes) >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1u << 46;
-    d |= layout << 61;
-    return d;
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr >> 4) & 0x3FFFu) | (1u << 16); }
+__device__ __forceinline__ uint32_t desc_lo_mn(uint32_t saddr, uint32_t group_stride) {
+    return ((saddr >> 4) & 0x3FFFu) | (((group_stride >> 4) & 0x3FFFu) << 16);
 }
 
 // bf16 x bf16 -> f32, both operands K-major, M x N tile.

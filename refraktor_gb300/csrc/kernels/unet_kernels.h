@@ -12,6 +12,8 @@
 #define RFK_UNET_F32OUT 2  // conv epilogue: store f32 instead of bf16
 #define RFK_UNET_UP2 4     // conv epilogue: store each output pixel at its 2x2 pixels of a (2h, 2w) output
                            // (nearest upsampling into the next level's concatenation; bf16, no accumulate)
+#define RFK_UNET_ANY_ORDER 8  // conv: the f32 sums may be ordered and split as is fastest (inference and input
+                              // gradients); without it the order is fixed, so that a training loss is reproducible
 
 #ifdef __cplusplus
 extern "C" {

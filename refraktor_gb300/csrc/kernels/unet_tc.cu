@@ -10,11 +10,12 @@
 // TMA box of the NHWC input at the tile's offset - the padding comes from
 // TMA's zero fill outside the image - and the B tiles boxes (BK x BN) of the
 // weights [cout][9][cin]. A producer warp (one lane) issues the TMA loads into
-// a ring of shared-memory stages, an MMA warp (one lane) issues tcgen05.mma
+// a ring of shared-memory stages, an MMA warp issues tcgen05.mma
 // (M 128, N BN, K 16 per instruction) and frees each stage with
 // tcgen05.commit; eight epilogue warps read the accumulator rows from TMEM
 // (two per lane quarter) and apply the epilogue: bias, ReLU, a
-// ReLU-derivative mask, accumulation into the output, bf16 or f32 store.
+// ReLU-derivative mask, then bf16 rows by TMA store, or f32 or accumulating
+// stores. conv3x3_rows streams image rows through narrow layers.
 // The input gradient of a conv is the same kernel on the output gradient with
 // the weights transposed and the taps flipped ([cin][9][cout]).
 //
@@ -55,6 +56,7 @@ struct conv_args {
     int mask_cstride, mask_coff;
     int accumulate;
     int tma_out;  // bf16 output through shared memory and TMA stores
+    int band;     // conv3x3_rows: output rows per task
     int* err;
 };
 
@@ -76,7 +78,7 @@ struct conv_cfg {
     // R image rows per tile (R accumulators of 128 x BN): small-N layers move
     // R times the bytes per pipeline stage, so the stage round trip is shared
     // (128 channels: two rows share each weight tile)
-    static constexpr int R = BN == 128 && MODE == 1 ? 2 : BN >= 96 ? 1 : 128 / BN;
+    static constexpr int R = BN == 128 ? 2 : BN == 256 ? 1 : 128 / BN;
     static constexpr int A_PIX = MODE ? 136 : 128;                // pixel lines per image row
     static constexpr int A_ROWS = MODE == 2 ? R + 2 : R;           // image rows per A box
     static constexpr uint32_t A_ROW = (uint32_t)A_PIX * BK * 2u;   // one image row segment
@@ -96,14 +98,38 @@ struct conv_cfg {
     static constexpr uint32_t BUDGET = 229376u - 2u * OUT_TILE;
     static constexpr int STAGES = ((BUDGET - B_RES) / STAGE_BYTES > 8) ? 8 : (int)((BUDGET - B_RES) / STAGE_BYTES);
     static constexpr uint32_t SMEM = B_RES + STAGES * STAGE_BYTES + 2u * OUT_TILE + 1024u;
-    static constexpr uint32_t TMEM_COLS = BN == 96 ? 256u : 2u * R * BN;  // two sets of R accumulators
-    static_assert(MODE == 0 || (A_ROW % 512u == 0 && A_BYTES % (16u * BK) == 0 && B_TILE % 1024u == 0 && B_RES % 1024u == 0),
+    static constexpr uint32_t TMEM_COLS = 2u * R * BN;  // two sets of R accumulators
+    static_assert(MODE == 0 || (A_ROW % 512u == 0 && A_BYTES % 1024u == 0 && B_TILE % 1024u == 0 && B_RES % 1024u == 0),
                   "tap-reuse tiles must stay swizzle-aligned");
     static_assert(STAGES >= 2, "at least two stages");
 };
 
+// conv3x3_rows: input channel blocks of BK, tiles of 32 output channels whose
+// weights stay in shared memory; a pipeline stage is CPS channel blocks of an input row.
+template <int BK, int CPS>
+struct rows_cfg {
+    static constexpr uint32_t A_ROW = 136u * BK * 2u;  // pixels x0 - 1 .. x0 + 134 of an input row
+    static constexpr uint32_t STAGE_BYTES = CPS * A_ROW;
+    static constexpr uint32_t B_TILE = 32u * BK * 2u;
+    static constexpr int SLOTS = 5;                    // accumulators of 128 x 96 in TMEM
+    static constexpr int MAX_STAGES = 16, MIN_STAGES = 4;
+    static constexpr uint32_t OUT_TILE = 128u * 32u * 2u;  // two per epilogue group
+    static constexpr uint32_t BUDGET = 229376u - 4u * OUT_TILE;
+    static __host__ __device__ constexpr uint32_t res_bytes(int kpt) { return (uint32_t)kpt * 9u * B_TILE; }
+    static __host__ __device__ constexpr int stages(int kpt) {
+        if (res_bytes(kpt) >= BUDGET) return 0;
+        const int n = (int)((BUDGET - res_bytes(kpt)) / STAGE_BYTES);
+        return n > MAX_STAGES ? MAX_STAGES : n;
+    }
+    static_assert(A_ROW % 512u == 0 && B_TILE % 1024u == 0, "tiles must stay swizzle-aligned");
+};
+
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(n) : "memory");
 }
 
 __device__ __forceinline__ void store_bf16x16(bf16* dst, const float (&v)[16]) {
@@ -134,20 +160,22 @@ __device__ __forceinline__ void load_bf16x16(const bf16* src, float (&v)[16]) {
 
 constexpr int kEpiWarps = 8;  // two warps per TMEM lane quarter, each half of the columns
 
-// Bias, ReLU and ReLU-derivative mask of N consecutive output channels of one pixel.
+// Bias; ReLU and ReLU-derivative mask of N consecutive output channels of one pixel.
+template <int N>
+__device__ __forceinline__ void conv_bias(const conv_args& p, float (&v)[N], int ch) {
+    if (!p.bias) return;
+    const float4* bb = reinterpret_cast<const float4*>(p.bias + ch);
+#pragma unroll
+    for (int q = 0; q < N / 4; q++) {
+        const float4 f = __ldg(bb + q);
+        v[4 * q] += f.x;
+        v[4 * q + 1] += f.y;
+        v[4 * q + 2] += f.z;
+        v[4 * q + 3] += f.w;
+    }
+}
 template <int N>
 __device__ __forceinline__ void conv_activate(const conv_args& p, float (&v)[N], int ch, size_t pix, bool valid) {
-    if (p.bias) {
-        const float4* bb = reinterpret_cast<const float4*>(p.bias + ch);
-#pragma unroll
-        for (int q = 0; q < N / 4; q++) {
-            const float4 f = __ldg(bb + q);
-            v[4 * q] += f.x;
-            v[4 * q + 1] += f.y;
-            v[4 * q + 2] += f.z;
-            v[4 * q + 3] += f.w;
-        }
-    }
     if (p.relu) {
 #pragma unroll
         for (int j = 0; j < N; j++) v[j] = fmaxf(v[j], 0.0f);
@@ -161,6 +189,57 @@ __device__ __forceinline__ void conv_activate(const conv_args& p, float (&v)[N],
             for (int j = 0; j < 16; j++) v[g + j] = m[j] > 0.0f ? v[g + j] : 0.0f;
         }
     }
+}
+
+// f32 and accumulating outputs: a lane stores its pixel's N channels.
+template <int N>
+__device__ __forceinline__ void store_direct(const conv_args& p, float (&v)[N], size_t at) {
+    if (p.out_f32) {
+        float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at);
+#pragma unroll
+        for (int q = 0; q < N / 4; q++) {
+            const float4 o = p.accumulate ? dst[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            dst[q] = make_float4(v[4 * q] + o.x, v[4 * q + 1] + o.y, v[4 * q + 2] + o.z, v[4 * q + 3] + o.w);
+        }
+        return;
+    }
+#pragma unroll
+    for (int g = 0; g < N; g += 16) {
+        bf16* dst = static_cast<bf16*>(p.out) + at + g;
+        float o[16];
+        load_bf16x16(dst, o);
+#pragma unroll
+        for (int j = 0; j < 16; j++) o[j] += v[g + j];
+        store_bf16x16(dst, o);
+    }
+}
+
+// N channels of pixel px, from channel c0 of a tile of 128 pixels x OC
+// channels in shared memory, swizzled as the output's tensor map has it
+// (128- or 64-byte rows), so that the lanes' 16-byte writes meet no bank twice.
+template <int OC, int N>
+__device__ __forceinline__ void stage_bf16(uint8_t* tile, int px, int c0, const float (&v)[N]) {
+#pragma unroll
+    for (int q = 0; q < N / 8; q++) {
+        __nv_bfloat162 hh[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) hh[j] = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
+        const uint32_t k = (uint32_t)(c0 / 8 + q);  // 16-byte piece of the pixel
+        const uint32_t sw = OC == 64 ? (k ^ ((uint32_t)px & 7u)) : (k ^ (((uint32_t)px >> 1) & 3u));
+        *reinterpret_cast<uint4*>(tile + px * (OC * 2) + sw * 16) = *reinterpret_cast<uint4*>(hh);
+    }
+}
+
+// One thread: the staged tile to channels ch .. of pixels xt * 128 .. of a row
+// (with up2 to the 2 x 2 pixels of each).
+__device__ __forceinline__ void store_row(const conv_args& p, const CUtensorMap* map, const uint8_t* tile, int ch, int xt, int row) {
+    if (p.up2) {
+#pragma unroll
+        for (int d = 0; d < 4; d++) tc::tma_store_5d(map, tile, ch, d & 1, xt * 128, d >> 1, row);
+    } else {
+        tc::tma_store_3d(map, tile, ch, xt * 128, row);
+    }
+    tc::tma_store_commit();
 }
 
 // Drains R accumulator rows of 128 x BN (TMEM columns from acc on) into the
@@ -180,55 +259,16 @@ __device__ __forceinline__ void conv_epilogue(const conv_args& p, uint32_t acc, 
         for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 16) {
             float v[16];
             tc::tmem_ld16(acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(r * BN + c), v);
-            const int ch = n0 + c;
             if (!valid) continue;
-            if (p.bias) {
-                const float4* bb = reinterpret_cast<const float4*>(p.bias + ch);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float4 f = __ldg(bb + q);
-                    v[4 * q] += f.x;
-                    v[4 * q + 1] += f.y;
-                    v[4 * q + 2] += f.z;
-                    v[4 * q + 3] += f.w;
-                }
-            }
-            if (p.relu) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) v[j] = fmaxf(v[j], 0.0f);
-            }
-            if (p.mask) {
-                float m[16];
-                load_bf16x16(p.mask + pix * p.mask_cstride + p.mask_coff + ch, m);
-#pragma unroll
-                for (int j = 0; j < 16; j++) v[j] = m[j] > 0.0f ? v[j] : 0.0f;
-            }
-            const size_t at = pix * p.out_cstride + p.out_coff + ch;
-            if (p.out_f32) {
-                float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float4 o = p.accumulate ? dst[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    dst[q] = make_float4(v[4 * q] + o.x, v[4 * q + 1] + o.y, v[4 * q + 2] + o.z, v[4 * q + 3] + o.w);
-                }
-            } else {
-                bf16* dst = static_cast<bf16*>(p.out) + at;
-                if (p.accumulate) {
-                    float o[16];
-                    load_bf16x16(dst, o);
-#pragma unroll
-                    for (int j = 0; j < 16; j++) v[j] += o[j];
-                }
-                store_bf16x16(dst, v);
-            }
+            conv_bias<16>(p, v, n0 + c);
+            conv_activate<16>(p, v, n0 + c, pix, true);
+            store_direct<16>(p, v, pix * p.out_cstride + p.out_coff + n0 + c);
         }
     }
 }
 
 // As conv_epilogue, for bf16 outputs: a row's 128 pixels x OC channels are
-// assembled in shared memory (128- or 64-byte rows, swizzled as the tensor map
-// has it, so the lanes' 16-byte writes meet no bank twice) and leave as one TMA
-// store, or four with up2 (the 2 x 2 pixels of each). A lane storing its own
+// assembled in shared memory and leave as one TMA store, or four with up2. A lane storing its own
 // pixel's 32-byte pieces touches 32 lines per instruction: for a 1080p image the
 // 64-channel layer with up2 took 141 us that way and takes 66, the 128-channel one
 // 88 and 45, a plain 32 -> 64 layer 47 and 39.
@@ -250,32 +290,16 @@ __device__ __forceinline__ void conv_epilogue_tma(const conv_args& p, const CUte
             const uint32_t at = acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(r * BN + c + half * W);
             if constexpr (W == 32) tc::tmem_ld32(at, v);
             else tc::tmem_ld16(at, v);
+            conv_bias<W>(p, v, n0 + c + half * W);
             conv_activate<W>(p, v, n0 + c + half * W, pix, valid);
             uint8_t* tile = outbuf + (flip & 1u) * (128u * OC * 2u);
             // the tile's previous store has read it
             if (leader) tc::tma_store_wait_read<1>();
             tc::named_barrier(1, 32 * kEpiWarps);
-#pragma unroll
-            for (int q = 0; q < W / 8; q++) {
-                __nv_bfloat162 hh[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) hh[j] = __floats2bfloat162_rn(v[8 * q + 2 * j], v[8 * q + 2 * j + 1]);
-                const uint32_t k = (uint32_t)(half * (W / 8) + q);  // 16-byte piece of the pixel
-                const uint32_t sw = OC == 64 ? (k ^ ((uint32_t)px & 7u)) : (k ^ (((uint32_t)px >> 1) & 3u));
-                *reinterpret_cast<uint4*>(tile + px * (OC * 2) + sw * 16) = *reinterpret_cast<uint4*>(hh);
-            }
+            stage_bf16<OC, W>(tile, px, half * W, v);
             tc::fence_async();
             tc::named_barrier(2, 32 * kEpiWarps);
-            if (leader) {
-                const int ch = p.out_coff + n0 + c, row = img * p.h + y;
-                if (p.up2) {
-#pragma unroll
-                    for (int d = 0; d < 4; d++) tc::tma_store_5d(map, tile, ch, d & 1, xt * 128, d >> 1, row);
-                } else {
-                    tc::tma_store_3d(map, tile, ch, xt * 128, row);
-                }
-                tc::tma_store_commit();
-            }
+            if (leader) store_row(p, map, tile, p.out_coff + n0 + c, xt, img * p.h + y);
         }
     }
 }
@@ -296,7 +320,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
     __shared__ uint64_t full[C::STAGES], empty[C::STAGES], acc_full[2], acc_empty[2], wbar;
     __shared__ uint32_t tmem_base;
     __shared__ int s_fail;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     uint8_t* const res = base;                   // resident weights (MODE 2)
     uint8_t* const stages = base + C::B_RES;
     uint8_t* const outbuf = stages + C::STAGES * C::STAGE_BYTES;
@@ -324,7 +348,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
 
     if (warp == kEpiWarps) {
         if (lane == 0) {
@@ -379,15 +403,17 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
             if (MODE == 2 && !tc::mbar_wait(&wbar, 0)) atomicExch(&s_fail, 1);
         }
     } else if (warp == kEpiWarps + 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = tc::idesc_bf16(128, BN);
+        // the whole warp, see tc::mma_bf16
+        const uint32_t one = lane == 0;
+        {
+            constexpr uint32_t idesc = tc::idesc_bf16(128, BN), HI = tc::desc_hi(BK * 2);
             uint32_t g = 0;
-            bool ok = MODE != 2 || tc::mbar_wait(&wbar, 0);
+            bool ok = MODE != 2 || tc::all_lanes(tc::mbar_wait(&wbar, 0));
             const uint32_t sres = tc::smem_u32(res);
             int i = 0;
             for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x, i++) {
                 const int b = i & 1;
-                if (i >= 2 && !tc::mbar_wait(&acc_empty[b], ((i >> 1) - 1) & 1)) {
+                if (i >= 2 && !tc::all_lanes(tc::mbar_wait(&acc_empty[b], ((i >> 1) - 1) & 1))) {
                     ok = false;
                     break;
                 }
@@ -395,7 +421,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
                 const uint32_t acc = tmem + (uint32_t)(b * C::R * BN);
                 for (int kb = 0; kb < nk; kb++, g++) {
                     const uint32_t s = g % C::STAGES;
-                    if (!tc::mbar_wait(&full[s], (g / C::STAGES) & 1)) {
+                    if (!tc::all_lanes(tc::mbar_wait(&full[s], (g / C::STAGES) & 1))) {
                         ok = false;
                         break;
                     }
@@ -406,7 +432,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
                     // descriptors of the stage's first tiles; the others differ only in the
                     // start address field (bits 0-13, 16-byte units; shared memory < 256 KB,
                     // so adding the compile-time offset cannot carry out of it)
-                    const uint64_t a0 = tc::smem_desc_at(sa, BK * 2), b0 = tc::smem_desc(sb, BK * 2);
+                    const uint32_t a0 = tc::desc_lo(sa), b0 = tc::desc_lo(sb);
 #pragma unroll
                     for (int r = 0; r < C::R; r++)
 #pragma unroll
@@ -415,14 +441,14 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
                             const int dy = MODE == 2 ? t / 3 : 0, dx = MODE == 2 ? t % 3 : t;
 #pragma unroll
                             for (int kk = 0; kk < BK / 16; kk++)
-                                tc::mma_bf16(acc + (uint32_t)(r * BN),
-                                             a0 + (uint64_t)(((r + dy) * C::A_ROW + dx * (BK * 2) + kk * 32) >> 4),
-                                             b0 + (uint64_t)((t * C::B_TILE + kk * 32) >> 4), idesc,
-                                             (kb | t | kk) != 0 ? 1u : 0u);
+                                tc::mma_bf16<HI, HI>(one, acc + (uint32_t)(r * BN),
+                                                     a0 + (uint32_t)(((r + dy) * C::A_ROW + dx * (BK * 2) + kk * 32) >> 4),
+                                                     b0 + (uint32_t)((t * C::B_TILE + kk * 32) >> 4), idesc,
+                                                     (kb | t | kk) != 0 ? 1u : 0u);
                         }
-                    tc::mma_commit(&empty[s]);
+                    tc::mma_commit(one, &empty[s]);
                 }
-                tc::mma_commit(&acc_full[b]);  // also on failure: arrives once the issued MMAs are done
+                tc::mma_commit(one, &acc_full[b]);  // also on failure: arrives once the issued MMAs are done
             }
             if (!ok) atomicExch(&s_fail, 1);
         }
@@ -435,7 +461,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x, i++) {
             const int b = i & 1;
             // all epilogue warps go on or stop together (they meet at barriers below)
-            const bool got = tc::named_barrier_all(1, 32 * kEpiWarps, tc::mbar_wait(&acc_full[b], (i >> 1) & 1));
+            const bool got = tc::named_barrier_all(1, 32 * kEpiWarps, tc::all_lanes(tc::mbar_wait(&acc_full[b], (i >> 1) & 1)));
             if (!got) {
                 if (lane == 0) atomicExch(&s_fail, 1);
                 break;
@@ -461,6 +487,221 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
     __syncthreads();
     if (threadIdx.x == 0 && s_fail) atomicExch(p.err, 1);
     if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
+}
+
+// Row-streaming convolution for layers of 32, 64 or 96 output channels. An MMA
+// of such a layer is bound by its A tile: M 128 x K 16 takes 45 cycles at N 32
+// and 56 at N 96 (math: 16 and 48), so the three tap rows go into N: the
+// weights of a column tap lie stacked as [dy 0 | dy 1 | dy 2], 32 output
+// channels each, and the MMAs of an input row leave its three partial products
+// side by side in a TMEM slot of 96 columns. Output row q is dy 0 of input row
+// q - 1, dy 1 of row q and dy 2 of row q + 1, summed in f32 by the epilogue; five
+// slots let two input rows run ahead. A CTA walks down bands of a 128-pixel
+// column, an input row (136 pixels, one stage per channel block) being read
+// once per band and 32 output channels; the tile's weights are loaded once.
+// Two epilogue groups of four warps (one per TMEM lane quarter) take output rows
+// in turn; each output row arrives once at its three slots, the first and last
+// row of a band also for the rows that do not exist.
+template <int BK, int CPS>
+__global__ void __launch_bounds__(320, 1) conv3x3_rows(const __grid_constant__ CUtensorMap tmA,
+                                                       const __grid_constant__ CUtensorMap tmB,
+                                                       const __grid_constant__ CUtensorMap tmO, conv_args p) {
+    using C = rows_cfg<BK, CPS>;
+    extern __shared__ uint8_t smem_dyn[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[C::MAX_STAGES], empty[C::MAX_STAGES], slot_full[C::SLOTS], slot_empty[C::SLOTS], wbar;
+    __shared__ uint32_t tmem_base;
+    __shared__ int s_fail;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int kpt = p.cin / BK;
+    const uint32_t nst = (uint32_t)C::stages(kpt);
+    uint8_t* const res = base;
+    uint8_t* const outbuf = base + C::res_bytes(kpt);
+    uint8_t* const stages = outbuf + 4 * C::OUT_TILE;
+    // this CTA's 32 output channels, and its tasks among those of the CTAs that share them
+    const int ntn = p.cout / 32, n0 = ((int)blockIdx.x % ntn) * 32;
+    const int bands = (p.h + p.band - 1) / p.band;
+    const int ntasks = p.n_img * bands * p.tiles_x, first = (int)blockIdx.x / ntn;
+    const int step = ((int)gridDim.x - (int)blockIdx.x % ntn + ntn - 1) / ntn;
+
+    if (warp == 0) tc::tmem_alloc(&tmem_base, 512u);
+    if (threadIdx.x == 32) {
+        for (uint32_t s = 0; s < nst; s++) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < C::SLOTS; s++) {
+            tc::mbar_init(&slot_full[s], 1);
+            tc::mbar_init(&slot_empty[s], 3 * 4);  // three output rows, four warps each
+        }
+        tc::mbar_init(&wbar, 1);
+        s_fail = 0;
+        tc::mbar_fence_init();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+
+    if (warp == kEpiWarps) {
+        if (lane == 0) {
+            // producer: the weights once, then a stage per (input row, channel block)
+            tc::mbar_expect_tx(&wbar, C::res_bytes(kpt));
+            for (int cb = 0; cb < kpt; cb++)
+                for (int dx = 0; dx < 3; dx++)
+                    for (int dy = 0; dy < 3; dy++)
+                        tc::tma_load_2d(res + (uint32_t)((cb * 3 + dx) * 3 + dy) * C::B_TILE, &tmB, &wbar,
+                                        (dy * 3 + dx) * p.cin + cb * BK, n0);
+            uint32_t s = 0, round = 0, issued = 0;
+            bool ok = true;
+            for (int t = first; ok && t < ntasks; t += step) {
+                const int xt = t % p.tiles_x, y0 = ((t / p.tiles_x) % bands) * p.band, img = t / (p.tiles_x * bands);
+                const int rows_in = min(p.band, p.h - y0) + 2;
+                for (int i = 0; ok && i < rows_in; i++)
+                    for (int cb = 0; cb < kpt; cb += CPS) {
+                        if (round > 0 && !tc::mbar_wait(&empty[s], (round - 1) & 1)) {
+                            ok = false;
+                            break;
+                        }
+                        tc::mbar_expect_tx(&full[s], C::STAGE_BYTES);
+#pragma unroll
+                        for (int c = 0; c < CPS; c++)
+                            tc::tma_load_4d(stages + s * C::STAGE_BYTES + (uint32_t)c * C::A_ROW, &tmA, &full[s],
+                                            p.cin_off + (cb + c) * BK, xt * 128 - 1, y0 + i - 1, img);
+                        issued++;
+                        if (++s == nst) {
+                            s = 0;
+                            round++;
+                        }
+                    }
+            }
+            if (!ok) {
+                atomicExch(&s_fail, 1);
+                // let the copies in flight land before the CTA exits (bounded)
+                for (uint32_t q = issued >= nst ? issued - nst : 0; q < issued; q++) tc::mbar_wait(&full[q % nst], (q / nst) & 1);
+            }
+            if (!tc::mbar_wait(&wbar, 0)) atomicExch(&s_fail, 1);
+        }
+    } else if (warp == kEpiWarps + 1) {
+        const uint32_t one = lane == 0;
+        {
+            constexpr uint32_t idesc = tc::idesc_bf16(128, 96), HI = tc::desc_hi(BK * 2);
+            const uint32_t b0 = tc::desc_lo(tc::smem_u32(res));
+            uint32_t s = 0, round = 0, slot = 0, use = 0;  // use: how often the slot ring has gone round
+            bool ok = tc::all_lanes(tc::mbar_wait(&wbar, 0));
+            for (int t = first; ok && t < ntasks; t += step) {
+                const int y0 = ((t / p.tiles_x) % bands) * p.band;
+                const int rows_in = min(p.band, p.h - y0) + 2;
+                for (int i = 0; ok && i < rows_in; i++) {
+                    if (use > 0 && !tc::all_lanes(tc::mbar_wait(&slot_empty[slot], (use - 1) & 1))) {
+                        ok = false;
+                        break;
+                    }
+                    tc::fence_after();
+                    const uint32_t acc = tmem + slot * 96u;
+                    for (int cb = 0; cb < kpt; cb += CPS) {
+                        if (!tc::all_lanes(tc::mbar_wait(&full[s], round & 1))) {
+                            ok = false;
+                            break;
+                        }
+                        tc::fence_after();
+                        const uint32_t a0 = tc::desc_lo(tc::smem_u32(stages + s * C::STAGE_BYTES));
+                        const uint32_t bc = b0 + (((uint32_t)cb * 9u * C::B_TILE) >> 4);
+#pragma unroll
+                        for (int c = 0; c < CPS; c++)
+#pragma unroll
+                            for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                                for (int kk = 0; kk < BK / 16; kk++)
+                                    tc::mma_bf16<HI, HI>(one, acc, a0 + (uint32_t)((c * C::A_ROW + dx * (BK * 2) + kk * 32) >> 4),
+                                                         bc + (uint32_t)(((c * 9 + dx * 3) * C::B_TILE + kk * 32) >> 4), idesc,
+                                                         (cb | c | dx | kk) != 0 ? 1u : 0u);
+                        tc::mma_commit(one, &empty[s]);
+                        if (++s == nst) {
+                            s = 0;
+                            round++;
+                        }
+                    }
+                    tc::mma_commit(one, &slot_full[slot]);  // also on failure: arrives once the issued MMAs are done
+                    if (++slot == C::SLOTS) {
+                        slot = 0;
+                        use++;
+                    }
+                }
+            }
+            if (!ok) atomicExch(&s_fail, 1);
+        }
+    } else {
+        // epilogue: the groups take the CTA's output rows in turn. A group waits
+        // for the last input row of an output row only (the others were committed
+        // before it); a parity tells neighbouring uses of a slot apart, so these
+        // waits may be SLOTS input rows apart at most: 2, or 4 across the end of a
+        // band, as every band has at least two rows.
+        const int quarter = warp & 3, group = warp >> 2;
+        const bool leader = (threadIdx.x & 127) == 0;
+        const int px = quarter * 32 + lane;
+        const uint32_t lane_acc = tmem + ((uint32_t)(quarter * 32) << 16);
+        float bias[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++) bias[j] = p.bias ? __ldg(p.bias + n0 + j) : 0.0f;
+        uint32_t g0 = 0, n = 0, flip = 0;  // input rows and output rows before this band; staged rows of the group
+        bool ok = true;
+        for (int t = first; ok && t < ntasks; t += step) {
+            const int xt = t % p.tiles_x, y0 = ((t / p.tiles_x) % bands) * p.band, img = t / (p.tiles_x * bands);
+            const int rows = min(p.band, p.h - y0);
+            const int x = xt * 128 + px;
+            const bool valid = x < p.w;
+            for (int q = (int)((n ^ (uint32_t)group) & 1u); q < rows; q += 2) {
+                const uint32_t g = g0 + (uint32_t)q;
+                const uint32_t s0 = g % C::SLOTS, s1 = (g + 1) % C::SLOTS, s2 = (g + 2) % C::SLOTS;
+                ok = tc::named_barrier_all(1 + group, 128,
+                                           __all_sync(0xffffffffu, tc::mbar_wait(&slot_full[s2], ((g + 2) / C::SLOTS) & 1)));
+                if (!ok) {
+                    if (lane == 0) atomicExch(&s_fail, 1);
+                    break;
+                }
+                tc::fence_after();
+                uint32_t d0[32], d1[32], d2[32];
+                tc::tmem_ld32_start(lane_acc + s0 * 96u, d0);
+                tc::tmem_ld32_start(lane_acc + s1 * 96u + 32u, d1);
+                tc::tmem_ld32_start(lane_acc + s2 * 96u + 64u, d2);
+                tc::tmem_ld_wait(d0, d1, d2);
+                tc::fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    const uint32_t lo = q == 0 ? 1u : 0u, hi = q == rows - 1 ? 1u : 0u;
+                    mbar_arrive_n(&slot_empty[s0], 1u + 2u * lo);
+                    mbar_arrive_n(&slot_empty[s1], 1u + lo + hi);
+                    mbar_arrive_n(&slot_empty[s2], 1u + 2u * hi);
+                }
+                float v[32];
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    v[j] = ((__uint_as_float(d0[j]) + __uint_as_float(d1[j])) + __uint_as_float(d2[j])) + bias[j];
+                const int y = y0 + q;
+                const size_t pix = ((size_t)img * p.h + y) * p.w + (valid ? x : 0);
+                conv_activate<32>(p, v, n0, pix, valid);
+                if (p.tma_out) {
+                    // two staging tiles per group: the store before last has read this one
+                    uint8_t* const tile = outbuf + (2 * group + (int)(flip++ & 1u)) * C::OUT_TILE;
+                    stage_bf16<32, 32>(tile, px, 0, v);
+                    tc::fence_async();
+                    if (leader) tc::tma_store_wait_read<0>();
+                    tc::named_barrier(1 + group, 128);
+                    if (leader) store_row(p, &tmO, tile, p.out_coff + n0, xt, img * p.h + y);
+                } else if (valid) {
+                    store_direct<32>(p, v, pix * p.out_cstride + p.out_coff + n0);
+                }
+            }
+            g0 += (uint32_t)rows + 2u;
+            n += (uint32_t)rows;
+        }
+        if (leader) tc::tma_store_wait<0>();
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && s_fail) atomicExch(p.err, 1);
+    if (warp == 0) tc::tmem_dealloc(tmem, 512u);
 }
 
 // ----------------------------------------------------------------- wgrad ----
@@ -518,7 +759,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
     __shared__ uint64_t full[C::STAGES], empty[C::STAGES], done;
     __shared__ uint32_t tmem_base;
     __shared__ int s_fail;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
     const int ntiles = p.cin / BN;
     const int m0 = (blockIdx.y / ntiles) * 128;
@@ -543,7 +784,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
-    const uint32_t tmem = tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
 
     if (warp == 0 && lane == 0) {
         int issued = 0;
@@ -580,12 +821,13 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
             for (int kb = issued - C::STAGES < 0 ? 0 : issued - C::STAGES; kb < issued; kb++)
                 tc::mbar_wait(&full[kb % C::STAGES], (kb / C::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
+        const uint32_t one = lane == 0;
         constexpr uint32_t idesc = tc::idesc_bf16_bmn(128, C::NB) | (1u << 15);  // A MN-major too
         bool ok = true;
         for (int kb = 0; kb < nk; kb++) {
             const int s = kb % C::STAGES, r = kb / C::STAGES;
-            if (!tc::mbar_wait(&full[s], r & 1)) {
+            if (!tc::all_lanes(tc::mbar_wait(&full[s], r & 1))) {
                 ok = false;
                 break;
             }
@@ -593,13 +835,12 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
             const uint32_t sa = tc::smem_u32(base + (size_t)s * C::STAGE_BYTES), sb = sa + C::A_BYTES;
 #pragma unroll
             for (int kk = 0; kk < 4; kk++)
-                tc::mma_bf16(tmem, tc::smem_desc_mn(sa + kk * 16 * A_ROW, A_ROW, A_GROUP),
-                             tc::smem_desc_mn(sb + kk * 16 * C::B_ROW, C::B_ROW, C::B_GROUP),
-                             idesc,
-                             (kb | kk) != 0 ? 1u : 0u);
-            tc::mma_commit(&empty[s]);
+                tc::mma_bf16<tc::desc_hi(A_ROW), tc::desc_hi(C::B_ROW)>(one, tmem, tc::desc_lo_mn(sa + kk * 16 * A_ROW, A_GROUP),
+                                                                        tc::desc_lo_mn(sb + kk * 16 * C::B_ROW, C::B_GROUP), idesc,
+                                                                        (kb | kk) != 0 ? 1u : 0u);
+            tc::mma_commit(one, &empty[s]);
         }
-        tc::mma_commit(&done);
+        tc::mma_commit(one, &done);
         if (!ok) atomicExch(&s_fail, 1);
     }
     __syncwarp();
@@ -689,6 +930,35 @@ cudaError_t launch_conv(const CUtensorMap& a, const CUtensorMap& b, const CUtens
     return cudaGetLastError();
 }
 
+template <int BK, int CPS>
+cudaError_t launch_rows(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& o, conv_args p, cudaStream_t s) {
+    using C = rows_cfg<BK, CPS>;
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [] { attr = raise_smem(conv3x3_rows<BK, CPS>, C::BUDGET + 4u * C::OUT_TILE + 1024u); });
+    if (attr != cudaSuccess) return attr;
+    const int ntn = p.cout / 32, sms = sm_count_cached(), kpt = p.cin / BK;
+    // rows per band: the least rows of the busiest CTA, each band's two halo rows
+    // included; no band of one row
+    const long long strips = (long long)p.n_img * p.tiles_x, ctas = std::max(1, sms / ntn);
+    if (strips * p.h > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+    long long best = -1;
+    for (long long nb = 1; nb <= 4 * ctas / strips + 4 && nb <= (p.h + 1) / 2; nb++) {
+        const int band = (int)((p.h + nb - 1) / nb);
+        if (p.h % band == 1 || band < 2) continue;
+        const long long tasks = strips * ((p.h + band - 1) / band), cost = (tasks + ctas - 1) / ctas * (band + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            p.band = band;
+        }
+    }
+    const long long tasks = strips * ((p.h + p.band - 1) / p.band);
+    const int grid = (int)std::min<long long>(tasks, ctas) * ntn;
+    const uint32_t smem = C::res_bytes(kpt) + (uint32_t)C::stages(kpt) * C::STAGE_BYTES + 4u * C::OUT_TILE + 1024u;
+    conv3x3_rows<BK, CPS><<<grid, 32 * (kEpiWarps + 2), smem, s>>>(a, b, o, p);
+    return cudaGetLastError();
+}
+
 template <int BN, bool PACK, bool DXP>
 cudaError_t launch_wgrad(const CUtensorMap& a, const CUtensorMap& b, const wgrad_args& p, int splits, cudaStream_t s) {
     using C = wgrad_cfg<BN, DXP>;
@@ -720,25 +990,39 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
         return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weights) | reinterpret_cast<uintptr_t>(out)) & 63)
         return cudaErrorMisalignedAddress;
-    const int bn = cout == 96 ? 96 : pick_bn(cout);
+    const bool wide_k = cin % 64 == 0 && in_coff % 64 == 0;
+    // Order of the sums. Without RFK_UNET_ANY_ORDER an accumulator adds its
+    // products in one order, whichever sizes: channel block, tap (32 output
+    // channels), tap row, channel block, column tap (64), or tap, channel block
+    // (128, 256). Another order changes a few bf16 roundings per layer: 1e-5 of a
+    // training loss, nothing in a denoised image (half-float steps are coarser).
+    const bool any = (flags & RFK_UNET_ANY_ORDER) != 0;
+    // Up to 96 output channels with weights that leave room for four input rows
+    // in shared memory: conv3x3_rows (1080p U-Net, against the tiles below: 32 ->
+    // 32 63 / 72 us, 96 -> 32 95 / 174, 32 -> 96 176 / 211, 192 -> 64 100 / 111, 64 -> 64
+    // with up2 56 / 63), except 64 output channels from at most 64 without up2
+    // (32 -> 64 37 / 33).
+    const bool up2 = (flags & RFK_UNET_UP2) != 0;
+    const bool rows = any && cout <= 96 && h >= 2 && (cout != 64 || cin > 64 || up2) &&
+                      (wide_k ? rows_cfg<64, 1>::stages(cin / 64) : rows_cfg<32, 1>::stages(cin / 32)) >= rows_cfg<32, 1>::MIN_STAGES;
+    const int bn = rows ? 32 : pick_bn(cout);
     // tap reuse: 32 output channels (4 rows per tile) load each input channel
     // block once for all nine taps (MODE 2, 32-channel K blocks so that three
-    // 70 KB stages fit; it keeps one output tile's weights resident: cout == 32,
-    // at most 3 input blocks); up to 128 (1 or 2 rows) once per tap row (MODE 1),
-    // 256 (1 row) once per tap (MODE 0: three 32 KB weight tiles and the row leave
-    // one stage). 128 channels at 480 x 270: 384 -> 128 80 us with two rows per tile
-    // and tap rows, 135 with one row and taps; 96 channels (1080p) 189 us as one
-    // tile, 522 as three of 32.
-    const int mode = (bn == 32 && cout == 32 && cin <= 32 * 3) ? 2 : (bn <= 128 ? 1 : 0);
-    const int bk = (mode != 2 && cin % 64 == 0 && in_coff % 64 == 0) ? 64 : 32;
+    // 52 KB stages fit; it keeps one output tile's weights resident: cout == 32,
+    // at most 3 input blocks); 64 (2 rows) once per tap row (MODE 1); 128 (2 rows
+    // sharing each weight tile) once per tap row where the order allows it, 256 (1
+    // row) once per tap (MODE 0: three 32 KB weight tiles and the row leave one stage).
+    const int mode2 = !rows && cout == 32 && cin <= 32 * 3;
+    const int bk = !mode2 && wide_k ? 64 : 32;
+    const int mode = rows ? 1 : mode2 ? 2 : bn <= 64 ? 1 : bn == 128 && (any || cin == bk) ? 1 : 0;
     CUtensorMap ma, mb;
     const CUtensorMapSwizzle sw = bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     {
         cuuint64_t dims[4] = {(cuuint64_t)in_cstride, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n_img};
         cuuint64_t str[3] = {(cuuint64_t)in_cstride * 2, (cuuint64_t)w * in_cstride * 2, (cuuint64_t)h * w * in_cstride * 2};
-        // image rows and pixel lines of an A box, as conv_cfg<BK, BN, MODE>
-        const cuuint32_t rows = (bn == 128 ? 2u : bn >= 96 ? 1u : (cuuint32_t)(128 / bn)) + (mode == 2 ? 2u : 0u);
-        cuuint32_t box[4] = {(cuuint32_t)bk, mode ? 136u : 128u, rows, 1};
+        // image rows and pixel lines of an A box, as rows_cfg and conv_cfg<BK, BN, MODE>
+        const cuuint32_t box_rows = rows || bn == 256 ? 1u : bn == 128 ? 2u : (cuuint32_t)(128 / bn) + (mode == 2 ? 2u : 0u);
+        cuuint32_t box[4] = {(cuuint32_t)bk, mode ? 136u : 128u, box_rows, 1};
         if (!make_map(&ma, in, 4, dims, str, box, sw)) return cudaErrorInvalidValue;
     }
     {
@@ -761,7 +1045,7 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
     p.bias = bias;
     p.relu = flags & RFK_UNET_RELU;
     p.out_f32 = (flags & RFK_UNET_F32OUT) ? 1 : 0;
-    p.up2 = (flags & RFK_UNET_UP2) ? 1 : 0;
+    p.up2 = up2;
     if (p.up2 && (p.out_f32 || accumulate)) return cudaErrorInvalidValue;
     p.mask = static_cast<const bf16*>(mask);
     p.mask_cstride = mask_cstride;
@@ -791,19 +1075,21 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
         }
         if (!good) return cudaErrorInvalidValue;
     }
+    if (rows) {
+        if (bk == 64) return launch_rows<64, 1>(ma, mb, mo, p, s);
+        return cin == 96 ? launch_rows<32, 3>(ma, mb, mo, p, s) : launch_rows<32, 1>(ma, mb, mo, p, s);
+    }
     if (bk == 64) {
         switch (bn) {
         case 256: return launch_conv<64, 256, 0>(ma, mb, mo, p, s);
-        case 128: return launch_conv<64, 128, 1>(ma, mb, mo, p, s);
-        case 96: return launch_conv<64, 96, 1>(ma, mb, mo, p, s);
+        case 128: return mode ? launch_conv<64, 128, 1>(ma, mb, mo, p, s) : launch_conv<64, 128, 0>(ma, mb, mo, p, s);
         case 64: return launch_conv<64, 64, 1>(ma, mb, mo, p, s);
         default: return launch_conv<64, 32, 1>(ma, mb, mo, p, s);
         }
     }
     switch (bn) {
     case 256: return launch_conv<32, 256, 0>(ma, mb, mo, p, s);
-    case 128: return launch_conv<32, 128, 1>(ma, mb, mo, p, s);
-    case 96: return launch_conv<32, 96, 1>(ma, mb, mo, p, s);
+    case 128: return mode ? launch_conv<32, 128, 1>(ma, mb, mo, p, s) : launch_conv<32, 128, 0>(ma, mb, mo, p, s);
     case 64: return launch_conv<32, 64, 1>(ma, mb, mo, p, s);
     default: return mode == 2 ? launch_conv<32, 32, 2>(ma, mb, mo, p, s) : launch_conv<32, 32, 1>(ma, mb, mo, p, s);
     }

@@ -1,6 +1,7 @@
 """The convolution's output path at the edges of its tiles: widths that end inside
-a 128-pixel store, odd row counts, the 96-channel tile and two-row 128-channel
-tiles, into a channel slice of a wider tensor with guard rows behind it."""
+a 128-pixel store, odd row counts, two-row 128-channel tiles and (any summation
+order) bands of the row-streaming kernel, several per CTA and with a short last
+one, into a channel slice of a wider tensor with guard rows behind it."""
 import ctypes as C
 
 import numpy as np
@@ -15,9 +16,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("up", [False, True])
+@pytest.mark.parametrize("any_order", [False, True])
 @pytest.mark.parametrize("n,h,w,cin,cout", [(2, 5, 200, 32, 96), (1, 1, 8, 64, 96), (1, 3, 130, 128, 128), (2, 7, 127, 64, 128),
-                                            (1, 9, 129, 32, 32), (1, 5, 72, 64, 64), (2, 1, 257, 128, 256)])
-def test_conv_stores_only_its_slice(n, h, w, cin, cout, up):
+                                            (1, 9, 129, 32, 32), (1, 5, 72, 64, 64), (2, 1, 257, 128, 256),
+                                            (1, 2, 136, 32, 32), (3, 67, 300, 96, 32), (1, 41, 640, 192, 64),
+                                            (2, 33, 129, 384, 128)])
+def test_conv_stores_only_its_slice(n, h, w, cin, cout, any_order, up):
     L = _lib.lib()
     L.rfk_unet_conv3x3.restype = C.c_int
     L.rfk_unet_conv3x3.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int,
@@ -33,7 +37,7 @@ def test_conv_stores_only_its_slice(n, h, w, cin, cout, up):
     buf = torch.randn(px + guard, wide, device="cuda", generator=g).to(torch.bfloat16)
     before = buf.clone()
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
-    rc = L.rfk_unet_conv3x3(x.data_ptr(), n, h, w, cin, 0, cin, wt.data_ptr(), cout, b.data_ptr(), 5 if up else 1, buf.data_ptr(),
+    rc = L.rfk_unet_conv3x3(x.data_ptr(), n, h, w, cin, 0, cin, wt.data_ptr(), cout, b.data_ptr(), (5 if up else 1) | (8 if any_order else 0), buf.data_ptr(),
                             wide, off, None, 0, 0, 0, err.data_ptr(), None)
     torch.cuda.synchronize()
     assert rc == 0 and int(err.item()) == 0
