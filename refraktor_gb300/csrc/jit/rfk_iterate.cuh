@@ -505,10 +505,10 @@ __device__ __forceinline__ void rfk_cache_add(rfk_cache& cc, float4* __restrict_
 // are summed in shared memory and go out as one red.global.add.v4.f32 per hot
 // pixel and check interval; every other draw is one red.v4 after a single
 // 16-byte table load, with no warp-wide matching of pixels.
-//   discovery  in the first RFK_DISC_PASSES passes of every check interval,
-//              the draws of one chain in RFK_CPT (RFK_DISC below) are counted
-//              per pixel in a hash table (linear probing, at most
-//              RFK_DISC_PROBES places);
+//   discovery  in the first RFK_DISC_PASSES drawing passes of every cycle, the
+//              draws of one chain in RFK_CPT (RFK_DISC below) are counted per
+//              pixel in a hash table (linear probing, at most RFK_DISC_PROBES
+//              places);
 //   rebuild    after those passes (all threads, between barriers): the old
 //              sums are flushed, and every pixel counted RFK_HOT_MIN times or
 //              more becomes hot (at most RFK_HOT_MAX, the first two free ways
@@ -516,16 +516,20 @@ __device__ __forceinline__ void rfk_cache_add(rfk_cache& cc, float4* __restrict_
 //   draw       a draw to a hot pixel adds to its sums (RFK_HOT_COPIES copies,
 //              picked by lane, so that lanes on one pixel rarely wait on the
 //              same shared-memory word), any other draw is one red.v4.
-// The sums are also flushed at the end of every check interval, so they
-// always go to the histogram of the unit whose draws they hold.
+// A cycle is a check interval in rfk_bin and rfk_bin_tm, which flush at its end
+// too; where every pass is checked no table could ever be used, and nothing is
+// counted (a 64-spp 1280 x 720 frame of 4 temporal samples: DISC_MS ms of
+// rfk_bin_tm, 2.75 with the counting). In rfk_bin_batch it is RFK_MAX_CHECK
+// drawing passes of the block on one unit, whatever the unit's check interval;
+// the sums are flushed when the block turns to another unit and at the end.
 // The sums are fixed point, value * 2^RFK_HOT_SHIFT in one u32 per (slot,
 // copy, channel), added with integer shared-memory atomics: on GB300 these
 // take 0.87x the time of the chain step with float shared-memory atomics on
 // the 1080p bench genome. A copy sums the draws of RFK_BLOCK * RFK_CPT /
-// RFK_HOT_COPIES chains over at most RFK_MAX_CHECK passes between flushes,
-// each channel at most 1 (a draw with opacity above 1, which only a spline
-// overshoot gives, goes out as a red.v4), so the shift below keeps every sum
-// under 2^31. One quantum is 2^-17 at the bench's launch shape: 7.6e-6 per
+// RFK_HOT_COPIES chains over at most RFK_MAX_CHECK + RFK_DISC_PASSES passes
+// between flushes, each channel at most 1 (a draw with opacity above 1, which
+// only a spline overshoot gives, goes out as a red.v4), so the shift below,
+// which keeps RFK_MAX_CHECK passes under 2^31, keeps every sum under 2^32. One quantum is 2^-17 at the bench's launch shape: 7.6e-6 per
 // draw against colour contributions of up to the opacity; an opacity of 1 is
 // exact.
 #define RFK_HOT_MAX 64
@@ -804,19 +808,20 @@ __device__ __forceinline__ void rfk_store_chains(const rfk_pass_smem& sm, const 
 #define RFK_CACHE_ARG
 #endif
 
-// Flush 4: the discovery passes of a check interval sample one chain in
-// RFK_CPT, spread over the whole sorted chain order (slot q of the threads
-// whose index is q modulo RFK_CPT: the sort puts the chains of the first
-// xforms in the low slots, so one slot alone would see only those xforms'
-// pixels); after the last of them the block rebuilds its hot-pixel table.
-// Both depend only on the pass number within the interval (block-uniform).
+// Flush 4: the discovery passes of a cycle sample one chain in RFK_CPT, spread
+// over the whole sorted chain order (slot q of the threads whose index is q
+// modulo RFK_CPT: the sort puts the chains of the first xforms in the low
+// slots, so one slot alone would see only those xforms' pixels); after the last
+// of them the block rebuilds its hot-pixel table. `age` is the block's drawing
+// pass within the cycle (block-uniform), RFK_NO_AGE or more: nothing is counted.
+#define RFK_NO_AGE 64u
 #if RFK_FLUSH == 4
-#define RFK_DISC(it, q) ((it) < RFK_DISC_PASSES && threadIdx.x % RFK_CPT == (unsigned)(q))
-#define RFK_HOT_PASS_END(it, bins) \
-    if ((it) + 1 == RFK_DISC_PASSES) rfk_hot_rebuild(sm.hot, (bins));
+#define RFK_DISC(age, q) ((age) < RFK_DISC_PASSES && threadIdx.x % RFK_CPT == (unsigned)(q))
+#define RFK_HOT_PASS_END(age, bins) \
+    if ((age) + 1 == RFK_DISC_PASSES) rfk_hot_rebuild(sm.hot, (bins));
 #else
-#define RFK_DISC(it, q) false
-#define RFK_HOT_PASS_END(it, bins)
+#define RFK_DISC(age, q) false
+#define RFK_HOT_PASS_END(age, bins)
 #endif
 
 // One pass over this thread's RFK_CPT chains, in two parts with the loop over
@@ -909,7 +914,8 @@ __device__ __forceinline__ void rfk_move_slot(int q, unsigned chain, rfk_pass_sm
 // with a barrier after which s_hits / s_draws hold the block's sums and the
 // hot-pixel cache is flushed.
 __device__ __forceinline__ void rfk_block_totals(unsigned& my_hits, unsigned& my_draws, unsigned long long* s_hits,
-                                                 unsigned long long* s_draws, rfk_pass_smem& sm, float4* bins) {
+                                                 unsigned long long* s_draws, rfk_pass_smem& sm, float4* bins,
+                                                 bool hot) {
     unsigned wh = __reduce_add_sync(0xffffffffu, my_hits);
     unsigned wd = __reduce_add_sync(0xffffffffu, my_draws);
     my_hits = 0;
@@ -922,11 +928,19 @@ __device__ __forceinline__ void rfk_block_totals(unsigned& my_hits, unsigned& my
 #if RFK_FLUSH == 2 || RFK_FLUSH == 3
     rfk_cache_flush(sm.cache, bins);
 #elif RFK_FLUSH == 4
-    rfk_hot_flush(sm.hot, bins, false);
+    if (hot) rfk_hot_flush(sm.hot, bins, false);
 #else
     (void)sm;
     (void)bins;
 #endif
+    (void)hot;
+}
+
+// Whether the `n` passes up to `pass` hold one whose number is a multiple of
+// 16: the bailout checks read the clock and the host's stop flag (pinned host
+// memory, about a microsecond away) only then, and always after 16 or more.
+__device__ __forceinline__ bool rfk_poll(unsigned long long pass, unsigned n) {
+    return n == 0 || (pass >> 4) != ((pass - n) >> 4);
 }
 
 #ifdef RFK_MINB
@@ -959,20 +973,23 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin(rfk_bin_args a) {
 
     unsigned long long pass = 0;
     unsigned my_hits = 0, my_draws = 0;
+    const unsigned age0 = a.check > 1u ? 0u : RFK_NO_AGE;
+    (void)age0;
 #pragma unroll 1
     for (;;) {
+        unsigned n = 0;
 #pragma unroll 1
-        for (unsigned it = 0; it < min(a.check, RFK_MAX_CHECK) && (a.max_passes == 0 || pass < a.max_passes); it++) {
+        for (; n < min(a.check, RFK_MAX_CHECK) && (a.max_passes == 0 || pass < a.max_passes); n++) {
             rfk_pick_sort(sm, P, lane_stream, a.call_id, pass, a.seed, a.salt);
 #pragma unroll 1
             for (int q = 0; q < RFK_CPT; q++)
                 rfk_move_slot(q, chain0 + (unsigned)q * cstride, sm, P, a.bins, a.w, a.h, a.call_id, pass, a.seed,
-                              a.salt, true, RFK_DISC(it, q), my_hits, my_draws);
+                              a.salt, true, RFK_DISC(age0 + n, q), my_hits, my_draws);
             pass++;
-            RFK_HOT_PASS_END(it, a.bins)
+            RFK_HOT_PASS_END(age0 + n, a.bins)
         }
         // bailout check: block totals -> global counters -> decision
-        rfk_block_totals(my_hits, my_draws, &s_hits, &s_draws, sm, a.bins);
+        rfk_block_totals(my_hits, my_draws, &s_hits, &s_draws, sm, a.bins, true);
         if (threadIdx.x == 0) {
             unsigned long long q = atomicAdd(&a.counters->quality, s_hits) + s_hits;
             atomicAdd(&a.counters->draws, s_draws);
@@ -981,12 +998,9 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin(rfk_bin_args a) {
             unsigned bail = 0;
             if (a.quality_target && q >= a.quality_target) bail |= RFK_ST_QUALITY;
             if (a.max_passes && pass >= a.max_passes) bail |= RFK_ST_ITERS;
-            if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
-            if (a.stop && *a.stop) bail |= RFK_ST_STOP;
-            if (!bail && a.quality_target) {
-                // another block may have met the target already
-                unsigned long long gq = *((volatile unsigned long long*)&a.counters->quality);
-                if (gq >= a.quality_target) bail |= RFK_ST_QUALITY;
+            if (rfk_poll(pass, n)) {
+                if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
+                if (a.stop && *a.stop) bail |= RFK_ST_STOP;
             }
             s_bail = bail;
         }
@@ -1091,6 +1105,8 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_tm(rfk_bin_args a) {
     unsigned long long pass = 0, total = 0;
     unsigned in_slice = 0;
     unsigned my_hits = 0, my_draws = 0;
+    const unsigned age0 = a.check > 1u ? 0u : RFK_NO_AGE;
+    (void)age0;
 #pragma unroll 1
     for (;;) {
         unsigned n = 0;
@@ -1101,13 +1117,13 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_tm(rfk_bin_args a) {
 #pragma unroll 1
             for (int q = 0; q < RFK_CPT; q++)
                 rfk_move_slot(q, chain0 + (unsigned)q * cstride, sm, P, a.bins, a.w, a.h, a.call_id, pass, a.seed,
-                              a.salt, true, RFK_DISC(n, q), my_hits, my_draws);
+                              a.salt, true, RFK_DISC(age0 + n, q), my_hits, my_draws);
             pass++;
             total++;
-            RFK_HOT_PASS_END(n, a.bins)
+            RFK_HOT_PASS_END(age0 + n, a.bins)
         }
         in_slice += n;
-        rfk_block_totals(my_hits, my_draws, &s_hits, &s_draws, sm, a.bins);
+        rfk_block_totals(my_hits, my_draws, &s_hits, &s_draws, sm, a.bins, true);
         if (threadIdx.x == 0) {
             atomicAdd(&a.counters->quality, s_hits);
             atomicAdd(&a.counters->draws, s_draws);
@@ -1120,8 +1136,10 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_tm(rfk_bin_args a) {
             unsigned bail = 0;
             if (done == (T >= 32 ? 0xFFFFFFFFu : ((1u << T) - 1u))) bail |= RFK_ST_QUALITY;
             if (a.max_passes && total >= a.max_passes) bail |= RFK_ST_ITERS;
-            if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
-            if (a.stop && *a.stop) bail |= RFK_ST_STOP;
+            if (rfk_poll(total, n)) {
+                if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
+                if (a.stop && *a.stop) bail |= RFK_ST_STOP;
+            }
             s_bail = bail;
             int nxt = cur;
             if (!bail && ((done >> cur) & 1u || in_slice >= a.slice)) {
@@ -1238,6 +1256,8 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
     unsigned long long total_passes = 0;
     unsigned status = 0;
     unsigned my_hits = 0, my_draws = 0;
+    unsigned age = 0;  // drawing passes in the hot-pixel cycle (flush 4)
+    (void)age;
 #pragma unroll 1
     for (;;) {
         __syncthreads();  // everyone is done with the previous item's parameters
@@ -1278,6 +1298,17 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
         __syncthreads();
         unsigned warm = 0;
         if (u != cur) {
+#if RFK_FLUSH == 4
+            // the last unit's sums go out (its draws were done before the barriers
+            // above), and the new unit finds its own hot pixels
+            if (cur >= 0) {
+                rfk_hot_flush(sm.hot, a.units[cur].bins, false);
+                __syncthreads();
+                rfk_hot_clear(sm.hot);
+                __syncthreads();
+            }
+            age = 0;
+#endif
 #pragma unroll
             for (int q = 0; q < RFK_CPT; q++) {
                 Rng r0;
@@ -1304,12 +1335,17 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
 #pragma unroll 1
                 for (int q = 0; q < RFK_CPT; q++)
                     rfk_move_slot(q, chain0 + (unsigned)q * cstride, sm, P, U.bins, U.w, U.h, call_id, pass, a.seed,
-                                  a.salt, draw, RFK_DISC(it, q), my_hits, my_draws);
+                                  a.salt, draw, RFK_DISC(age, q), my_hits, my_draws);
                 pass++;
-                RFK_HOT_PASS_END(it, U.bins)
+#if RFK_FLUSH == 4
+                if (draw) {
+                    if (++age == RFK_DISC_PASSES) rfk_hot_rebuild(sm.hot, U.bins);
+                    else if (age == RFK_MAX_CHECK) age = 0;
+                }
+#endif
             }
             done += n;
-            rfk_block_totals(my_hits, my_draws, &s_hits, &s_draws, sm, U.bins);
+            rfk_block_totals(my_hits, my_draws, &s_hits, &s_draws, sm, U.bins, false);
             if (threadIdx.x == 0) {
                 const unsigned long long q = atomicAdd(&a.uc[u].quality, s_hits) + s_hits;
                 atomicAdd(&a.uc[u].draws, s_draws);
@@ -1318,8 +1354,10 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
                 s_draws = 0;
                 unsigned bail = 0;
                 if (q >= U.quality_target) bail |= RFK_ST_QUALITY;
-                if (a.stop && *a.stop) bail |= RFK_ST_STOP;
-                if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
+                if (rfk_poll(pass, n)) {
+                    if (a.stop && *a.stop) bail |= RFK_ST_STOP;
+                    if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
+                }
                 s_bail = bail;
                 // a new jitter for the next interval: the other threads wait at
                 // the barrier below and read P only after it
@@ -1336,6 +1374,9 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
             break;
         }
     }
+#if RFK_FLUSH == 4
+    if (cur >= 0) rfk_hot_flush(sm.hot, a.units[cur].bins, false);  // after the barrier that follows the last draw
+#endif
     if (threadIdx.x == 0) {
         atomicAdd(&a.counters->passes, total_passes * (unsigned long long)(RFK_BLOCK * RFK_CPT));
         atomicOr(&a.counters->status, status);
