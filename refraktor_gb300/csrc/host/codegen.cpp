@@ -1,5 +1,7 @@
 #include "codegen.h"
 
+#include <map>
+#include <set>
 #include <sstream>
 
 namespace rfk {
@@ -118,7 +120,89 @@ struct emitter {
         return info;
     }
     size_t end = 0;
+
+    // One function for all standard xforms (see shared_layout): `X` is an
+    // xform's block in shared memory.
+    void shared_fn(std::ostringstream& out, const std::vector<std::string>& names) const {
+        out << "RFK_FN R rfk_xf_shared(V2& pt, R& col, const PT* RFK_RESTRICT X, Rng& rng) {\n";
+        out << "    const rfk_u32 live = __float_as_uint(X[0]);\n";
+        out << "    const R aff_a = X[4], aff_d = X[5], aff_b = X[6], aff_e = X[7], aff_c = X[8], aff_f = X[9];\n";
+        out << "    (void)aff_a; (void)aff_b; (void)aff_c; (void)aff_d; (void)aff_e; (void)aff_f;\n";
+        out << "    V2 p = fl_vec2(fl_fma(aff_a, pt.x, fl_fma(aff_b, pt.y, aff_c)), "
+               "fl_fma(aff_d, pt.x, fl_fma(aff_e, pt.y, aff_f)));\n";
+        out << "    V2 r_ = fl_vec2(R(0), R(0));\n";
+        // a common value is evaluated when a live variation reads it
+        std::map<std::string, unsigned> readers;
+        std::set<std::string> direct;
+        for (size_t v = 0; v < names.size(); v++) {
+            const auto& use = db.get_variation(names[v]).apply_usage.commons;
+            for (auto& c : db.common_closure(std::set<std::string>(use.begin(), use.end()))) {
+                readers[c] |= 1u << v;
+                direct.insert(c);
+            }
+        }
+        for (auto& cn : db.common_closure(direct)) {
+            dsl::emit_env cenv;
+            cenv.variation = "common." + cn;
+            out << "    R c_" << cn << " = R(0);\n    if (live & " << readers[cn] << "u) c_" << cn << " = "
+                << dsl::emit_expression(db.common_ast(cn), cenv) << ";\n";
+        }
+        size_t off = 10;
+        for (size_t v = 0; v < names.size(); v++) {
+            const auto& def = db.get_variation(names[v]);
+            dsl::emit_env env;
+            env.variation = names[v];
+            env.aff_prefix = "aff_";
+            out << "    if (live & " << (1u << v) << "u) { // " << names[v] << "\n";
+            out << "        const R w_ = X[" << off++ << "];\n";
+            for (auto& ps : {def.plain_params(), def.precalc_params()})
+                for (auto& pn : ps) {
+                    env.param_expr[pn] = "P_" + pn;
+                    out << "        const R P_" << pn << " = X[" << off++ << "]; (void)P_" << pn << ";\n";
+                }
+            out << indent(dsl::emit_body(*def.apply_ast, env), 2);
+            out << "    }\n";
+        }
+        out << "    pt = r_;\n";
+        out << "    col = col * (R(1) - X[2]) + X[1] * X[2];\n";
+        out << "    return X[3];\n}\n\n";
+    }
 };
+
+// A union-of-variations kernel repeats the code of nearly every variation in
+// every xform, more than the instruction cache holds while the warps of a block
+// run different xforms: half of its time goes into instruction fetch. If the
+// standard xforms (one vlink each) hold the variations of their union twice
+// over or more, and 24 bodies at least, they share one function instead, and
+// each xform's parameters are laid out alike in shared memory:
+//   live mask (bit v: the weight of the union's variation v is not 0), colour,
+//   colour speed, opacity, affine (6), then per variation its weight, parameters
+//   and precalculated parameters (0 where the xform lacks it).
+// 64 heterogeneous flames and the denoiser's sets qualify; a flame of its own, with one to
+// three variations per xform, does not, and keeps a function per xform with
+// compile-time offsets. Returns the union's names, empty if not shared.
+std::vector<std::string> shared_layout(const flamedb& db, const flame& f, size_t& stride) {
+    std::map<std::string, const vardata*> all;
+    size_t bodies = 0;
+    for (auto& xf : f.xforms) {
+        if (xf.vchain.size() != 1) return {};
+        for (auto& [vn, vd] : xf.vchain[0].variations) {
+            all[vn] = &vd;
+            bodies++;
+        }
+    }
+    if (f.xforms.size() < 2 || all.size() > 32 || bodies < 24 || bodies < 2 * all.size()) return {};
+    stride = 10;
+    std::vector<std::string> names;
+    for (auto& [vn, vd] : all) {
+        const auto& def = db.get_variation(vn);
+        names.push_back(vn);
+        stride += 1 + def.plain_params().size() + def.precalc_params().size();
+    }
+    stride |= 1;  // odd: the xforms' blocks start in different banks
+    if (stride * f.xforms.size() > shared_block_floats) return {};
+    return names;
+}
 
 }  // namespace
 
@@ -163,12 +247,49 @@ generated_flame generate_flame_code(const flamedb& db, const flame& f) {
     s << "rfk_xf_base[" << g.xforms.size() << "] = {";
     for (size_t i = 0; i < g.xforms.size(); i++) s << (i ? ", " : "") << g.xforms[i].base;
     s << "};\n\n";
+    size_t stride = 0;
+    const std::vector<std::string> names = shared_layout(db, f, stride);
+    g.shared = !names.empty();
+    s << "#define RFK_SHARED " << (g.shared ? 1 : 0) << "\n";
+    if (g.shared) {
+        s << "#ifndef RFK_HOST_TWIN\n#define RFK_SX_STRIDE " << stride << "\n#define RFK_SX_VARS " << names.size() << "\n";
+        // source of each float of the shared-memory blocks in the packed reals
+        // (-1: none), and of each variation's weight in a block
+        s << "__device__ const short rfk_sx_src[RFK_NX * RFK_SX_STRIDE] = {";
+        std::vector<size_t> weight_at;
+        for (size_t i = 0; i < g.num_xforms; i++) {
+            std::vector<long> row = {-1, (long)g.xforms[i].base + 1, (long)g.xforms[i].base + 2, (long)g.xforms[i].base + 3};
+            size_t at = g.xforms[i].base + 4;
+            for (int j = 0; j < 6; j++) row.push_back((long)at++);
+            weight_at.clear();
+            const auto& vars = f.xforms[i].vchain[0].variations;  // sorted by name, as the union is
+            for (auto& vn : names) {
+                const auto& def = db.get_variation(vn);
+                const size_t n = 1 + def.plain_params().size() + def.precalc_params().size();
+                weight_at.push_back(row.size());
+                const bool has = vars.count(vn) > 0;
+                for (size_t j = 0; j < n; j++) row.push_back(has ? (long)at++ : -1);
+            }
+            row.resize(stride, -1);
+            for (size_t j = 0; j < stride; j++) s << (i + j ? ", " : "") << row[j];
+        }
+        s << "};\n__device__ const short rfk_sx_weight[RFK_SX_VARS] = {";
+        for (size_t v = 0; v < weight_at.size(); v++) s << (v ? ", " : "") << weight_at[v];
+        s << "};\n";
+        em.shared_fn(s, names);
+        if (g.has_final) {
+            // the final xform keeps its own function
+            s << em.fn.str().substr(em.fn.str().rfind("RFK_FN R rfk_xf_"));
+        }
+        s << "#else\n";
+    }
     s << em.fn.str();
     s << "RFK_FN R rfk_dispatch(int k, V2& pt, R& col, const PT* RFK_RESTRICT P, Rng& rng) {\n";
     s << "    switch (k) {\n";
     for (size_t i = 1; i < g.num_xforms; i++) s << "    case " << i << ": return rfk_xf_" << i << "(pt, col, P, rng);\n";
     s << "    default: return rfk_xf_0(pt, col, P, rng);\n";
     s << "    }\n}\n\n";
+    if (g.shared) s << "#endif\n";
     if (g.has_final) {
         s << "RFK_FN R rfk_final(V2& pt, R& col, const PT* RFK_RESTRICT P, Rng& rng) {\n";
         s << "    return rfk_xf_" << g.num_xforms << "(pt, col, P, rng);\n}\n\n";

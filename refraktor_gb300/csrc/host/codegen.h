@@ -31,9 +31,14 @@ struct generated_flame {
     size_t num_xforms = 0;
     bool has_final = false;
     bool chaos = false;
+    bool shared = false;      // the standard xforms share one function (union kernels)
     std::vector<size_t> affine_indices;
     std::vector<xform_info> xforms;  // standard xforms, then the final xform
 };
+
+// Floats of a block's shared memory that the shared form's xform blocks may take
+// (the unused half of the palette's region, RFK_SX_BASE of rfk_iterate.cuh).
+constexpr size_t shared_block_floats = 512;
 
 generated_flame generate_flame_code(const flamedb& db, const flame& f);
 

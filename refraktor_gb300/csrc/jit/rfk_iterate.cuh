@@ -4,7 +4,9 @@
 // which defines:
 //   RFK_NX, RFK_HAS_FINAL, RFK_CHAOS, RFK_SIZE_REALS, RFK_NUM_AFFINES,
 //   rfk_affine_idx[], rfk_xf_base[] (offset of each xform's weight),
-//   R rfk_dispatch(int k, V2& p, R& c, const float* P, Rng& rng)   (standard xforms)
+//   R rfk_dispatch(int k, V2& p, R& c, const float* P, Rng& rng)   (standard xforms),
+//   or, with RFK_SHARED, R rfk_xf_shared(V2& p, R& c, const float* X, Rng& rng) for
+//   all of them with RFK_SX_STRIDE, RFK_SX_VARS, rfk_sx_src[], rfk_sx_weight[]
 //   R rfk_final(V2& p, R& c, const float* P, Rng& rng)              (if RFK_HAS_FINAL)
 //   void rfk_precalc(float* P, Rng& rng)                             (variation precalc)
 // and the launch shape: RFK_BLOCK (threads per block), RFK_CPT (chains per
@@ -53,6 +55,7 @@
 #define RFK_OFF_PAL_RAW (RFK_OFF_CALIAS + (RFK_CHAOS ? 2 * RFK_NX * RFK_NX : 0))
 #define RFK_OFF_PAL (((RFK_OFF_PAL_RAW) + 3) / 4 * 4)
 #define RFK_SAMPLE_FLOATS (RFK_OFF_PAL + 1024)
+#define RFK_SX_BASE (RFK_OFF_PAL + 512)
 
 // Passes between the bailout checks of the bin kernels, at most (the host
 // computes at most 32; the kernels clamp it again).
@@ -256,11 +259,37 @@ __device__ __forceinline__ unsigned rfk_rgb8(float4 c) {
 // refactor.cu:128-140): a draw reads both ends of its colour interval with one
 // 8-byte load from a 2 KB table instead of two 16-byte loads from 4 KB, which
 // cuts the shared-memory wavefronts of the random palette reads.
-__device__ __forceinline__ void rfk_load_params(float* P, const float* __restrict__ src) {
-    for (unsigned i = threadIdx.x; i < RFK_OFF_PAL; i += RFK_BLOCK) P[i] = src[i];
+// With RFK_SHARED the second half takes the xforms' blocks in the layout that
+// their common function reads. `threads`: of the block.
+__device__ __forceinline__ void rfk_load_params(float* P, const float* __restrict__ src, unsigned threads) {
+    for (unsigned i = threadIdx.x; i < RFK_OFF_PAL; i += threads) P[i] = src[i];
     uint2* pal = reinterpret_cast<uint2*>(P + RFK_OFF_PAL);
     const float4* sp = reinterpret_cast<const float4*>(src + RFK_OFF_PAL);
-    for (unsigned i = threadIdx.x; i < 256; i += RFK_BLOCK) pal[i] = make_uint2(rfk_rgb8(sp[i]), rfk_rgb8(sp[min(i + 1, 255u)]));
+    for (unsigned i = threadIdx.x; i < 256; i += threads) pal[i] = make_uint2(rfk_rgb8(sp[i]), rfk_rgb8(sp[min(i + 1, 255u)]));
+#if RFK_SHARED
+    for (unsigned i = threadIdx.x; i < RFK_NX * RFK_SX_STRIDE; i += threads) {
+        const int at = rfk_sx_src[i];
+        float v = at >= 0 ? src[at] : 0.0f;
+        if (i % RFK_SX_STRIDE == 0) {
+            unsigned live = 0u;
+            for (int k = 0; k < RFK_SX_VARS; k++) {
+                const int wt = rfk_sx_src[i + rfk_sx_weight[k]];
+                if (wt >= 0 && src[wt] != 0.0f) live |= 1u << k;
+            }
+            v = __uint_as_float(live);
+        }
+        P[RFK_SX_BASE + i] = v;
+    }
+#endif
+}
+
+// Applies standard xform k; P is the parameter block as rfk_load_params laid it out.
+__device__ __forceinline__ R rfk_apply_xform(int k, V2& p, R& c, const float* __restrict__ P, Rng& rng) {
+#if RFK_SHARED
+    return rfk_xf_shared(p, c, P + RFK_SX_BASE + k * RFK_SX_STRIDE, rng);
+#else
+    return rfk_dispatch(k, p, c, P, rng);
+#endif
 }
 
 // ------------------------------------------------------------- chain step --
@@ -284,7 +313,7 @@ __device__ __forceinline__ int rfk_move(int k, float& x, float& y, float& c, Rng
                                         unsigned w, unsigned h, float4& contrib, unsigned& hit) {
     V2 p = fl_vec2(x, y);
     R col = c;
-    R op = rfk_dispatch(k, p, col, P, rng);
+    R op = rfk_apply_xform(k, p, col, P, rng);
     if (rfk_badvalue(p.x) || rfk_badvalue(p.y)) {
         p.x = rng.u01() * 2.0f - 1.0f;
         p.y = rng.u01() * 2.0f - 1.0f;
@@ -518,7 +547,7 @@ __device__ __forceinline__ void rfk_cache_add(rfk_cache& cc, float4* __restrict_
 //              same shared-memory word), any other draw is one red.v4.
 // A cycle is a check interval in rfk_bin and rfk_bin_tm, which flush at its end
 // too; where every pass is checked no table could ever be used, and nothing is
-// counted (a 64-spp 1280 x 720 frame of 4 temporal samples: DISC_MS ms of
+// counted (a 64-spp 1280 x 720 frame of 4 temporal samples: 2.72 ms of
 // rfk_bin_tm, 2.75 with the counting). In rfk_bin_batch it is RFK_MAX_CHECK
 // drawing passes of the block on one unit, whatever the unit's check interval;
 // the sums are flushed when the block turns to another unit and at the end.
@@ -958,7 +987,7 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin(rfk_bin_args a) {
     rfk_pass_smem_init(sm);
     const unsigned lane_stream = blockIdx.x * RFK_BLOCK + threadIdx.x;
     const float* src = a.samples + (size_t)blockIdx.x * RFK_SAMPLE_FLOATS;
-    rfk_load_params(P, src);
+    rfk_load_params(P, src, RFK_BLOCK);
     if (threadIdx.x == 0) {
         s_hits = 0;
         s_draws = 0;
@@ -1029,7 +1058,7 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_warmup(const float* __restrict__ s
     __shared__ rfk_pass_smem sm;
     rfk_pass_smem_init(sm);
     const float* src = samples + (size_t)blockIdx.x * RFK_SAMPLE_FLOATS;
-    rfk_load_params(P, src);
+    rfk_load_params(P, src, RFK_BLOCK);
     __syncthreads();
     const unsigned total = gridDim.x * RFK_BLOCK * RFK_CPT;
     const unsigned lane_stream = blockIdx.x * RFK_BLOCK + threadIdx.x;
@@ -1098,7 +1127,7 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_tm(rfk_bin_args a) {
     unsigned smp = blockIdx.x;
     // chain of slot q of temporal sample smp: smp * RFK_BLOCK + t + q * cstride
     const unsigned cstride = S * RFK_BLOCK;
-    rfk_load_params(P, a.samples + (size_t)smp * RFK_SAMPLE_FLOATS);
+    rfk_load_params(P, a.samples + (size_t)smp * RFK_SAMPLE_FLOATS, RFK_BLOCK);
     rfk_load_chains(sm, a.st, smp * RFK_BLOCK + threadIdx.x, cstride);
     __syncthreads();
 
@@ -1162,7 +1191,7 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_tm(rfk_bin_args a) {
             rfk_store_chains(sm, a.st, smp * RFK_BLOCK + threadIdx.x, cstride);
             cur = nxt;
             smp = blockIdx.x + gridDim.x * (unsigned)cur;
-            rfk_load_params(P, a.samples + (size_t)smp * RFK_SAMPLE_FLOATS);
+            rfk_load_params(P, a.samples + (size_t)smp * RFK_SAMPLE_FLOATS, RFK_BLOCK);
             rfk_load_chains(sm, a.st, smp * RFK_BLOCK + threadIdx.x, cstride);
             in_slice = 0;
             __syncthreads();
@@ -1292,7 +1321,7 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
         if (u < 0) break;
         const unsigned long long item = s_item;
         const rfk_unit U = a.units[u];
-        rfk_load_params(P, U.params);
+        rfk_load_params(P, U.params, RFK_BLOCK);
         __syncthreads();
         if (threadIdx.x == 0) rfk_batch_jitter(P, U.params, item, call_id, pass, a.seed, a.salt);
         __syncthreads();
@@ -1392,6 +1421,14 @@ extern "C" __global__ void __launch_bounds__(256) rfk_apply(const float* __restr
                                                             const float* __restrict__ in, float* __restrict__ out,
                                                             unsigned n, unsigned seed) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+#if RFK_SHARED
+    __shared__ __align__(16) float sp[RFK_SAMPLE_FLOATS];
+    rfk_load_params(sp, params, blockDim.x);
+    __syncthreads();
+    const float* P = sp;
+#else
+    const float* P = params;
+#endif
     if (i >= n) return;
     Rng rng;
     rng.start(i, 0xFFFCu, 0ull, seed, 0u);
@@ -1400,10 +1437,10 @@ extern "C" __global__ void __launch_bounds__(256) rfk_apply(const float* __restr
     R op = 0.0f;
     if (xform < 0) {
 #if RFK_HAS_FINAL
-        op = rfk_final(p, c, params, rng);
+        op = rfk_final(p, c, P, rng);
 #endif
     } else {
-        op = rfk_dispatch(xform, p, c, params, rng);
+        op = rfk_apply_xform(xform, p, c, P, rng);
     }
     out[4 * i] = p.x;
     out[4 * i + 1] = p.y;
