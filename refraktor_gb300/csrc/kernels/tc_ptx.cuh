@@ -236,7 +236,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // group of row_bytes / 2 M or N elements, `group_stride` bytes apart): the
 // stride byte offset is the 8-row K group, the leading byte offset the group
 // stride (checked on the GPU against a reference product for both swizzles and
-// one to four groups).
+// one to four groups; a group stride of one row makes the groups the same rows
+// from one pixel line later each, as the weight gradients' column taps).
 // A start address may lie inside a tile that was written from a 1024-byte
 // aligned base: whole rows (pixel lines) past it, plus 32-byte K steps within a
 // row. The swizzle pattern is taken from the address bits of each access, as TMA

@@ -19,14 +19,13 @@
 // The input gradient of a conv is the same kernel on the output gradient with
 // the weights transposed and the taps flipped ([cin][9][cout]).
 //
-// wgrad3x3_tc (weight gradient): dW[n, t, c] = sum over pixels p of
-// dY[p, n] * X[p + t, c], a GEMM with M = cout (up to 128 per tile), N = BN
-// input channels, K = pixels; a K block is 64 pixels of one image row (W a
-// multiple of 64). A is K-major from a channel-major copy of dY; B is read
-// MN-major straight from the NHWC input: boxes of 32 or 64 channels x 64
-// pixels at the tap's offset, the column offset dx being a pixel coordinate
-// (not the innermost one, so any value is fine; zero fill outside the image).
-// CTAs split K and add their partial sums into dW (f32) atomically.
+// wgrad3x3_rows and wgrad3x3_cols (weight gradient): dW[n, t, c] = sum over
+// pixels p of dY[p, n] * X[p + t, c], GEMMs with K = pixels (64 of an image row at
+// a time, W a multiple of 64), M = output channels, and stacked on them tap rows
+// where they are few, N = input channels times the three column taps. Both
+// operands are read MN-major straight from NHWC; a column tap is the same box
+// from one pixel line further on, a tap row another row of dY (zero fill outside
+// the image). CTAs split K and add their partial sums into dW (f32) atomically.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -709,51 +708,61 @@ struct wgrad_args {
     int n_img, h, w;
     int cout, cin;
     int x_coff;     // first input channel in the NHWC tensor of X
-    int dx;         // tap column offset of this launch
-    int kpc;        // K blocks (64-pixel row segments) per CTA
-    int total_kb;   // all row segments
-    int a_rows;     // output channels an A box loads (rows of the 128-row A tile; the rest is not read)
+    int kpc;        // stages (wgrad3x3_rows) or rows (wgrad3x3_cols) of a 64-pixel segment per CTA
+    int total;      // all of them
     float* dw;      // [cout][9][cin]
+    int vec;        // dw is 16-byte aligned
     int* err;
 };
 
-// DXP (input channel tiles of at most 64): the three column taps share one
-// launch as three B blocks of BN channels (X at pixel offsets -1, 0, +1), so
-// the MMA's N is 3 BN.
-template <int BN, bool DXP>
-struct wgrad_cfg {
-    static constexpr int NB = DXP ? 3 * BN : BN;  // MMA N
-    static constexpr uint32_t A_BYTES = 128u * 64u * 2u;
-    static constexpr uint32_t B_BYTES = (uint32_t)NB * 64u * 2u;
-    // B: groups of G channels (64-byte rows, 64-byte swizzle, for 32-channel
-    // tiles; else 128-byte rows), each a 64-pixel box
-    static constexpr int G = BN == 32 ? 32 : 64;
-    static constexpr uint32_t B_ROW = (uint32_t)G * 2u;
-    static constexpr uint32_t B_GROUP = B_ROW * 64u;
-    static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-    // two CTAs per SM of ~96 KB; packed column taps (bigger stages): one CTA
-    // with a deeper ring
-    static constexpr uint32_t BUDGET = DXP ? 196608u : 98304u;
-    static constexpr int STAGES = BN == 256 ? 4 : (BUDGET / STAGE_BYTES > 8 ? 8 : (int)(BUDGET / STAGE_BYTES));
+// Adds 32 sums to 32 consecutive weights; `vec`: 16-byte aligned.
+__device__ __forceinline__ void wgrad_add(float* dst, const float (&v)[32], int vec) {
+    if (vec) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + j), "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]),
+                         "f"(v[j + 3])
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++) atomicAdd(dst + j, v[j]);
+    }
+}
+
+// Weight gradient of layers with few channels (CO = 32 or 64 output channels,
+// input channel tiles of BN = 32 or 64). A stage holds R image rows of a 64-pixel
+// segment: R rows of X, 72 pixels from x0 - 1 on, and R + 2 rows of dY, one TMA box
+// each. All nine taps read them from there: the three tap rows are dY rows r,
+// r + 1 and r + 2 of the stage against X row r (sum_y dY[y] X[y + dy] =
+// sum_y' dY[y' - dy] X[y']), stacked in M; the three column taps are N groups
+// that start one pixel line after another. With a box for each tap's rows and
+// columns a segment row took 24 KB (32 -> 32 channels) or 96 KB (64 -> 64, a launch
+// per tap row), which the L2 delivers at 5.4 TB/s (64-byte rows) or 9.2 TB/s; here
+// it is 13 or 26 KB. 16 images of 512 x 512, 32 -> 32: 124 us, before 277; 96 -> 32:
+// 246 and 720; 256 x 256, 32 -> 64: 60 and 191; 64 -> 64: 74 and 224; 192 -> 64:
+// 169 and 515.
+template <int CO, int BN>
+struct wgrad_rows_cfg {
+    static constexpr int R = 2;
+    static constexpr int NB = 3 * BN;  // MMA N
+    static constexpr uint32_t A_ROW = CO * 2u, A_GROUP = A_ROW * 64u;
+    static constexpr uint32_t B_ROW = BN * 2u, B_GROUP = B_ROW * 72u;
+    static constexpr uint32_t A_BYTES = (R + 2) * A_GROUP, STAGE_BYTES = A_BYTES + R * B_GROUP;
+    // 32 channels leave room for three CTAs on an SM (128 TMEM columns each), or two
+    static constexpr int CTAS = CO == 64 ? 1 : BN == 64 ? 2 : 3;
+    static constexpr int STAGES = (int)((225u * 1024u / CTAS - 2048u) / STAGE_BYTES);
     static constexpr uint32_t SMEM = STAGES * STAGE_BYTES + 1024u;
-    static constexpr uint32_t TMEM_COLS = NB <= 32 ? 32u : NB <= 64 ? 64u : NB <= 128 ? 128u : 256u;
-    static_assert(!DXP || BN <= 64, "column taps packed only for tiles of at most 64 channels");
+    // CO = 64: tap rows 2 and 1 in one accumulator of 128 rows, 0 in another
+    static constexpr int ACCS = CO == 64 ? 2 : 1;
+    static constexpr uint32_t ACC_COLS = NB <= 128 ? 128u : 256u;
+    static_assert(STAGES >= 2, "a ring");
+    static_assert(R * B_GROUP >= A_GROUP, "the unused fourth (CO = 64: second) row group of the last MMA is inside the stage");
 };
 
-// grid: x = K split, y = m tile * (cin / BN) + n tile, z = tap row (dy + 1).
-// PACK (32 output channels): the three tap rows share one launch, rows
-// 32 d .. 32 d + 31 of the A tile holding dY at image row yy - dy (dy = d - 1)
-// against X at row yy, since sum_y dY[y] X[y + dy] = sum_y' dY[y' - dy] X[y']
-// (rows outside the image are TMA zero fill); the A map is then 4D over
-// (x, y, image, channel). Rows of the A tile that no box writes hold stale
-// data; they only reach accumulator rows the epilogue does not read.
-template <int BN, bool PACK, bool DXP>
-__global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUtensorMap tmA,
-                                                   const __grid_constant__ CUtensorMap tmB, wgrad_args p) {
-    using C = wgrad_cfg<BN, DXP>;
-    // A (dY, MN-major from NHWC): groups of 32 output channels (64-byte rows)
-    // when packed, else of 64 (128-byte rows); the 128-row tile is 16 KB
-    constexpr uint32_t A_ROW = PACK ? 64u : 128u, A_GROUP = A_ROW * 64u;
+template <int CO, int BN>
+__global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUtensorMap tmA,
+                                                     const __grid_constant__ CUtensorMap tmB, wgrad_args p) {
+    using C = wgrad_rows_cfg<CO, BN>;
     extern __shared__ uint8_t smem_dyn[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[C::STAGES], empty[C::STAGES], done;
@@ -761,17 +770,14 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
     __shared__ int s_fail;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
-    const int ntiles = p.cin / BN;
-    const int m0 = (blockIdx.y / ntiles) * 128;
-    const int c0 = (blockIdx.y % ntiles) * BN;
-    const int dy = (int)blockIdx.z - 1;
-    const int segs_x = p.w / 64;
+    const int c0 = blockIdx.y * BN;
+    const int segs_x = p.w / 64, bands = (p.h + C::R - 1) / C::R;
     const int kb0 = blockIdx.x * p.kpc;
-    int nk = p.total_kb - kb0;
+    int nk = p.total - kb0;
     if (nk > p.kpc) nk = p.kpc;
     if (nk < 0) nk = 0;
 
-    if (warp == 0) tc::tmem_alloc(&tmem_base, C::TMEM_COLS);
+    if (warp == 0) tc::tmem_alloc(&tmem_base, C::ACCS * C::ACC_COLS);
     if (threadIdx.x == 32) {
         for (int s = 0; s < C::STAGES; s++) {
             tc::mbar_init(&full[s], 1);
@@ -796,24 +802,14 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
                 break;
             }
             const int seg = kb0 + kb;
-            const int xs = seg % segs_x;
-            const int yy = (seg / segs_x) % p.h;
-            const int im = seg / (segs_x * p.h);
+            const int x0 = seg % segs_x * 64;
+            const int y0 = seg / segs_x % bands * C::R;
+            const int im = seg / (segs_x * bands);
             uint8_t* sa = base + (size_t)s * C::STAGE_BYTES;
             // whole boxes count, zero fill included
-            tc::mbar_expect_tx(&full[s], (PACK ? 3u : (uint32_t)(p.a_rows + 63) / 64u) * A_GROUP + C::B_BYTES);
-            if (PACK) {
-#pragma unroll
-                for (int d = 0; d < 3; d++) tc::tma_load_4d(sa + d * A_GROUP, &tmA, &full[s], 0, xs * 64, yy - (d - 1), im);
-            } else {
-                for (int j = 0; j * 64 < p.a_rows; j++) tc::tma_load_4d(sa + j * A_GROUP, &tmA, &full[s], m0 + j * 64, xs * 64, yy, im);
-            }
-#pragma unroll
-            for (int xi = 0; xi < (DXP ? 3 : 1); xi++)
-#pragma unroll
-                for (int j = 0; j < BN / C::G; j++)
-                    tc::tma_load_4d(sa + C::A_BYTES + (xi * (BN / C::G) + j) * C::B_GROUP, &tmB, &full[s],
-                                    p.x_coff + c0 + j * C::G, xs * 64 + (DXP ? xi - 1 : p.dx), PACK ? yy : yy + dy, im);
+            tc::mbar_expect_tx(&full[s], C::STAGE_BYTES);
+            tc::tma_load_4d(sa, &tmA, &full[s], 0, x0, y0 - 1, im);
+            tc::tma_load_4d(sa + C::A_BYTES, &tmB, &full[s], p.x_coff + c0, x0 - 1, y0, im);
             issued++;
         }
         if (!ok) {
@@ -825,6 +821,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
         const uint32_t one = lane == 0;
         constexpr uint32_t idesc = tc::idesc_bf16_bmn(128, C::NB) | (1u << 15);  // A MN-major too
         bool ok = true;
+        uint32_t acc = 0;
         for (int kb = 0; kb < nk; kb++) {
             const int s = kb % C::STAGES, r = kb / C::STAGES;
             if (!tc::all_lanes(tc::mbar_wait(&full[s], r & 1))) {
@@ -833,11 +830,19 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
             }
             tc::fence_after();
             const uint32_t sa = tc::smem_u32(base + (size_t)s * C::STAGE_BYTES), sb = sa + C::A_BYTES;
+            const int rows = min(C::R, p.h - (kb0 + kb) / segs_x % bands * C::R);
+            for (int y = 0; y < rows; y++)
 #pragma unroll
-            for (int kk = 0; kk < 4; kk++)
-                tc::mma_bf16<tc::desc_hi(A_ROW), tc::desc_hi(C::B_ROW)>(one, tmem, tc::desc_lo_mn(sa + kk * 16 * A_ROW, A_GROUP),
-                                                                        tc::desc_lo_mn(sb + kk * 16 * C::B_ROW, C::B_GROUP), idesc,
-                                                                        (kb | kk) != 0 ? 1u : 0u);
+                for (int kk = 0; kk < 4; kk++) {
+                    const uint32_t alo = tc::desc_lo_mn(sa + y * C::A_GROUP + kk * 16 * C::A_ROW, C::A_GROUP);
+                    const uint32_t blo = tc::desc_lo_mn(sb + y * C::B_GROUP + kk * 16 * C::B_ROW, C::B_ROW);
+                    tc::mma_bf16<tc::desc_hi(C::A_ROW), tc::desc_hi(C::B_ROW)>(one, tmem, alo, blo, idesc, acc);
+                    if (C::ACCS == 2)
+                        tc::mma_bf16<tc::desc_hi(C::A_ROW), tc::desc_hi(C::B_ROW)>(
+                            one, tmem + C::ACC_COLS, tc::desc_lo_mn(sa + (y + 2) * C::A_GROUP + kk * 16 * C::A_ROW, C::A_GROUP),
+                            blo, idesc, acc);
+                    acc = 1;
+                }
             tc::mma_commit(one, &empty[s]);
         }
         tc::mma_commit(one, &done);
@@ -848,28 +853,170 @@ __global__ void __launch_bounds__(128) wgrad3x3_tc(const __grid_constant__ CUten
     bool got = tc::mbar_wait(&done, 0);
     got = __all_sync(0xffffffffu, got);
     tc::fence_after();
-    // PACK: warp d < 3 holds tap row d of output channels lane; otherwise
-    // accumulator row m is output channel m of tap row blockIdx.z. DXP:
-    // columns [xi BN, (xi + 1) BN) belong to column tap xi
-    if (got && nk > 0 && (!PACK || warp < 3)) {
-        const int m = PACK ? lane : m0 + warp * 32 + lane;
-        const int trow = PACK ? warp : dy + 1;
+    // accumulator row m: output channel m % CO of dY row m / CO of its MMA, tap
+    // row 2 - that; columns [xi BN, (xi + 1) BN) are column tap xi
+    if (got && nk > 0) {
 #pragma unroll 1
-        for (int c = 0; c < C::NB; c += 32) {
-            float v[32];
-            tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-            const int xi = DXP ? c / BN : p.dx + 1, cc = DXP ? c % BN : c;
-            if (m < p.cout) {
-                float* dst = p.dw + ((size_t)m * 9 + trow * 3 + xi) * p.cin + c0 + cc;
-#pragma unroll
-                for (int j = 0; j < 32; j++) atomicAdd(dst + j, v[j]);
+        for (int a = 0; a < C::ACCS; a++) {
+            const int g = a * 2 + warp * 32 / CO;
+            if (g > 2) break;
+            const int m = warp * 32 % CO + lane;
+#pragma unroll 1
+            for (int c = 0; c < C::NB; c += 32) {
+                float v[32];
+                tc::tmem_ld32(tmem + a * C::ACC_COLS + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
+                wgrad_add(p.dw + ((size_t)m * 9 + (2 - g) * 3 + c / BN) * p.cin + c0 + c % BN, v, p.vec);
             }
         }
     }
     tc::fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && (!got || s_fail)) atomicExch(p.err, 1);
-    if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
+    if (warp == 0) tc::tmem_dealloc(tmem, C::ACCS * C::ACC_COLS);
+}
+
+// Weight gradient of layers with 128 output channels or a multiple, in tiles of
+// 128 x 32 channels and all nine taps: three accumulators (one per tap row) of 96
+// columns (column taps as in wgrad3x3_rows). A CTA walks down the rows of 64-pixel
+// columns of the images; the ring holds a row of dY and of X per stage, and a row
+// of dY stays for the three rows of X that meet it, so both tensors cross L2 once
+// per tile: 21 KB a row against 12 MMAs of 56 cycles, which bound it.
+// Boxes for each tap read dY nine times and X three times. 16 images of
+// 128 x 128, 64 -> 128: 68 us, before 150; 128 -> 128: 99 and 203; 384 -> 128: 228
+// and 436; 64 x 64, 128 -> 256: 64 and 131; 256 -> 256: 103 and 193. (For 64 output
+// channels or fewer wgrad3x3_rows fills M with tap rows.)
+struct wgrad_cols_cfg {
+    static constexpr int BN = 32, NB = 96;
+    static constexpr uint32_t A_GROUP = 64u * 128u, A_BYTES = 2u * A_GROUP, B_BYTES = 72u * 64u;
+    static constexpr uint32_t STAGE_BYTES = A_BYTES + 5u * 1024u;  // 1024-byte aligned stages
+    static constexpr int STAGES = 10;
+    static constexpr uint32_t SMEM = STAGES * STAGE_BYTES + 1024u;
+};
+
+__global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUtensorMap tmA,
+                                                     const __grid_constant__ CUtensorMap tmB, wgrad_args p) {
+    using C = wgrad_cols_cfg;
+    extern __shared__ uint8_t smem_dyn[];
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full[C::STAGES], empty[C::STAGES], done;
+    __shared__ uint32_t tmem_base;
+    __shared__ int s_fail;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+
+    const int ntiles = p.cin / C::BN;
+    const int m0 = (int)(blockIdx.y / ntiles) * 128, c0 = (int)(blockIdx.y % ntiles) * C::BN;
+    const int segs_x = p.w / 64;
+    // rows of this CTA, counted down the columns one after another
+    const int row0 = blockIdx.x * p.kpc, row1 = min(row0 + p.kpc, p.total);
+
+    if (warp == 0) tc::tmem_alloc(&tmem_base, 512u);
+    if (threadIdx.x == 32) {
+        for (int s = 0; s < C::STAGES; s++) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        tc::mbar_init(&done, 1);
+        s_fail = 0;
+        tc::mbar_fence_init();
+    }
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+
+    // A run is a CTA's rows within one column. Its stages are the rows from the one
+    // above to the one below it, with X only for its own; the MMAs of a row come
+    // when the next row's stage is there, and leave the previous row's stage free.
+    if (warp == 0 && lane == 0) {
+        int k = 0;  // stages issued
+        bool ok = true;
+        for (int row = row0; ok && row < row1;) {
+            const int col = row / p.h, y0 = row % p.h, y1 = min(y0 + row1 - row, p.h);
+            const int x0 = col % segs_x * 64, im = col / segs_x;
+            for (int y = y0 - 1; y <= y1; y++, k++) {
+                const int s = k % C::STAGES, r = k / C::STAGES;
+                if (r > 0 && !tc::mbar_wait(&empty[s], (r - 1) & 1)) {
+                    ok = false;
+                    break;
+                }
+                const bool own = y >= y0 && y < y1;
+                uint8_t* sa = base + (size_t)s * C::STAGE_BYTES;
+                tc::mbar_expect_tx(&full[s], C::A_BYTES + (own ? C::B_BYTES : 0u));
+                tc::tma_load_4d(sa, &tmA, &full[s], m0, x0, y, im);
+                tc::tma_load_4d(sa + C::A_GROUP, &tmA, &full[s], m0 + 64, x0, y, im);
+                if (own) tc::tma_load_4d(sa + C::A_BYTES, &tmB, &full[s], p.x_coff + c0, x0 - 1, y, im);
+            }
+            row += y1 - y0;
+        }
+        if (!ok) {
+            atomicExch(&s_fail, 1);
+            for (int j = k - C::STAGES < 0 ? 0 : k - C::STAGES; j < k; j++)
+                tc::mbar_wait(&full[j % C::STAGES], (j / C::STAGES) & 1);
+        }
+    } else if (warp == 1) {
+        const uint32_t one = lane == 0;
+        constexpr uint32_t idesc = tc::idesc_bf16_bmn(128, C::NB) | (1u << 15);  // A MN-major too
+        const uint32_t ring = tc::smem_u32(base);
+        bool ok = true;
+        uint32_t acc = 0;  // bit d: the accumulator of tap row d holds sums
+        int k = 0;         // stage of the run's first row, the one above it
+        for (int row = row0; ok && row < row1;) {
+            const int y0 = row % p.h, y1 = min(y0 + row1 - row, p.h);
+            for (int y = y0; y < y1; y++, k++) {
+                // stages k, k + 1, k + 2: dY rows y - 1, y, y + 1
+                for (int j = y == y0 ? 0 : 2; ok && j < 3; j++)
+                    ok = tc::all_lanes(tc::mbar_wait(&full[(k + j) % C::STAGES], ((k + j) / C::STAGES) & 1));
+                if (!ok) break;
+                tc::fence_after();
+                const uint32_t sb = ring + (uint32_t)((k + 1) % C::STAGES) * C::STAGE_BYTES + C::A_BYTES;
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    // tap row d (X a row lower by d - 1): dY row y - (d - 1)
+                    if (y + 1 - d < 0 || y + 1 - d >= p.h) continue;
+                    const uint32_t sa = ring + (uint32_t)((k + 2 - d) % C::STAGES) * C::STAGE_BYTES;
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++) {
+                        tc::mma_bf16<tc::desc_hi(128), tc::desc_hi(64)>(
+                            one, tmem + (uint32_t)(d * C::NB), tc::desc_lo_mn(sa + kk * 16 * 128, C::A_GROUP),
+                            tc::desc_lo_mn(sb + kk * 16 * 64, 64u), idesc, acc >> d & 1u);
+                        acc |= 1u << d;
+                    }
+                }
+                tc::mma_commit(one, &empty[k % C::STAGES]);
+            }
+            if (!ok) break;
+            // the run's last row and the one below it
+            tc::mma_commit(one, &empty[k % C::STAGES]);
+            tc::mma_commit(one, &empty[(k + 1) % C::STAGES]);
+            k += 2;
+            row += y1 - y0;
+        }
+        tc::mma_commit(one, &done);
+        if (!ok) atomicExch(&s_fail, 1);
+    }
+    __syncwarp();
+
+    bool got = tc::mbar_wait(&done, 0);
+    got = __all_sync(0xffffffffu, got);
+    tc::fence_after();
+    // accumulator row m of tap row d: output channel m0 + m; columns
+    // [32 xi, 32 xi + 32): column tap xi
+    const int m = m0 + warp * 32 + lane;
+    if (got && row0 < row1 && m < p.cout) {
+#pragma unroll 1
+        for (int c = 0; c < 3 * C::NB; c += 32) {
+            // an only row at the image's edge has met no dY row of this tap row
+            const int d = c / C::NB, y = row0 % p.h + 1 - d;
+            if (d != 1 && (p.h == 1 || (row1 - row0 == 1 && (y < 0 || y >= p.h)))) continue;
+            float v[32];
+            tc::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
+            wgrad_add(p.dw + ((size_t)m * 9 + c / 32) * p.cin + c0, v, p.vec);
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && (!got || s_fail)) atomicExch(p.err, 1);
+    if (warp == 0) tc::tmem_dealloc(tmem, 512u);
 }
 
 // ------------------------------------------------------------- tensor maps --
@@ -959,23 +1106,68 @@ cudaError_t launch_rows(const CUtensorMap& a, const CUtensorMap& b, const CUtens
     return cudaGetLastError();
 }
 
-template <int BN, bool PACK, bool DXP>
-cudaError_t launch_wgrad(const CUtensorMap& a, const CUtensorMap& b, const wgrad_args& p, int splits, cudaStream_t s) {
-    using C = wgrad_cfg<BN, DXP>;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] { attr = raise_smem(wgrad3x3_tc<BN, PACK, DXP>, C::SMEM); });
-    if (attr != cudaSuccess) return attr;
-    const int mtiles = (p.cout + 127) / 128;
-    dim3 grid((unsigned)splits, (unsigned)(mtiles * (p.cin / BN)), PACK ? 1u : 3u);
-    wgrad3x3_tc<BN, PACK, DXP><<<grid, 128, C::SMEM, s>>>(a, b, p);
-    return cudaGetLastError();
-}
-
 int pick_bn(int c) {
     for (int bn : {256, 128, 64, 32})
         if (c % bn == 0) return bn;
     return 0;
+}
+
+template <int CO, int BN>
+cudaError_t launch_wgrad_rows(const void* dy, const void* x, int x_cstride, wgrad_args p, cudaStream_t s) {
+    using C = wgrad_rows_cfg<CO, BN>;
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [] { attr = raise_smem(wgrad3x3_rows<CO, BN>, C::SMEM); });
+    if (attr != cudaSuccess) return attr;
+    CUtensorMap ma, mb;
+    const CUtensorMapSwizzle swa = CO == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
+    const CUtensorMapSwizzle swb = BN == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
+    const cuuint64_t w = p.w, h = p.h, n = p.n_img, xp = (cuuint64_t)x_cstride * 2;
+    cuuint64_t da[4] = {CO, w, h, n}, sa[3] = {CO * 2, w * CO * 2, h * w * CO * 2};
+    cuuint64_t db[4] = {(cuuint64_t)x_cstride, w, h, n}, sb[3] = {xp, w * xp, h * w * xp};
+    cuuint32_t ba[4] = {CO, 64, C::R + 2, 1}, bb[4] = {BN, 72, C::R, 1};
+    if (!make_map(&ma, dy, 4, da, sa, ba, swa) || !make_map(&mb, x, 4, db, sb, bb, swb)) return cudaErrorInvalidValue;
+    const long long total = (long long)p.n_img * ((p.h + C::R - 1) / C::R) * (p.w / 64);
+    if (total > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+    p.total = (int)total;
+    // every SM full once (two CTAs: twice): partial sums at least as short as
+    // wgrad3x3_tc's
+    const int ntiles = p.cin / BN;
+    const int splits = (int)std::min<long long>(total, std::max(1, sm_count_cached() * C::CTAS * (C::CTAS == 2 ? 2 : 1) / ntiles));
+    p.kpc = (p.total + splits - 1) / splits;
+    dim3 grid((unsigned)((p.total + p.kpc - 1) / p.kpc), (unsigned)ntiles);
+    wgrad3x3_rows<CO, BN><<<grid, 128, C::SMEM, s>>>(ma, mb, p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wgrad_cols(const void* dy, const void* x, int x_cstride, wgrad_args p, cudaStream_t s) {
+    using C = wgrad_cols_cfg;
+    static std::once_flag once;
+    static cudaError_t attr = cudaSuccess;
+    std::call_once(once, [] { attr = raise_smem(wgrad3x3_cols, C::SMEM); });
+    if (attr != cudaSuccess) return attr;
+    CUtensorMap ma, mb;
+    const cuuint64_t w = p.w, h = p.h, n = p.n_img, xp = (cuuint64_t)x_cstride * 2, yp = (cuuint64_t)p.cout * 2;
+    cuuint64_t da[4] = {(cuuint64_t)p.cout, w, h, n}, sa[3] = {yp, w * yp, h * w * yp};
+    cuuint64_t db[4] = {(cuuint64_t)x_cstride, w, h, n}, sb[3] = {xp, w * xp, h * w * xp};
+    cuuint32_t ba[4] = {64, 64, 1, 1}, bb[4] = {32, 72, 1, 1};
+    if (!make_map(&ma, dy, 4, da, sa, ba, CU_TENSOR_MAP_SWIZZLE_128B) || !make_map(&mb, x, 4, db, sb, bb, CU_TENSOR_MAP_SWIZZLE_64B))
+        return cudaErrorInvalidValue;
+    const long long total = (long long)p.n_img * p.h * (p.w / 64);
+    if (total > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
+    p.total = (int)total;
+    // Partial sums of at least two waves of CTAs, and at least 45 over the tiles of
+    // 256 input channels: the rounding error of a sum grows with its length (16
+    // images of 128 x 128, 128 -> 128: 84.6 us and a relative error of 5.8e-6 with
+    // one wave, 99.0 and 2.6e-6 with two, 111 and 1.7e-6 with three).
+    const int mtiles = (p.cout + 127) / 128, tiles = mtiles * (p.cin / C::BN), sms = sm_count_cached();
+    const int least = (45 + mtiles * (p.cin / pick_bn(p.cin)) - 1) / (mtiles * (p.cin / pick_bn(p.cin)));
+    const int waves = std::max(2, (least * tiles + sms - 1) / sms);
+    const int splits = (int)std::min<long long>(total, std::max(1, waves * sms / tiles));
+    p.kpc = (p.total + splits - 1) / splits;
+    dim3 grid((unsigned)((p.total + p.kpc - 1) / p.kpc), (unsigned)tiles);
+    wgrad3x3_cols<<<grid, 128, C::SMEM, s>>>(ma, mb, p);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -1100,31 +1292,6 @@ extern "C" cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cs
     if (w % 64 || cin % 32 || cout <= 0 || cout % 32 || n_img <= 0 || h <= 0) return cudaErrorInvalidValue;
     if (x_coff % 32 || x_cstride % 32 || x_coff + cin > x_cstride) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 63) return cudaErrorMisalignedAddress;
-    const int bn = pick_bn(cin);
-    const size_t P = (size_t)n_img * h * w;
-    // 32 output channels: the three tap rows packed into one launch's M
-    const bool pack = cout == 32;
-    const int a_rows = cout < 128 ? cout : 128;
-    CUtensorMap ma, mb;
-    {
-        // dY NHWC (cout channels): boxes of 32 (packed, 64-byte swizzle) or 64
-        // output channels x 64 pixels, MN-major
-        const cuuint32_t g = pack ? 32u : 64u;
-        cuuint64_t dims[4] = {(cuuint64_t)cout, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n_img};
-        cuuint64_t str[3] = {(cuuint64_t)cout * 2, (cuuint64_t)w * cout * 2, (cuuint64_t)h * w * cout * 2};
-        cuuint32_t box[4] = {g, 64, 1, 1};
-        if (!make_map(&ma, dy, 4, dims, str, box, pack ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))
-            return cudaErrorInvalidValue;
-    }
-    {
-        // X NHWC: boxes of 32 (64-byte swizzle) or 64 channels x 64 pixels
-        const cuuint32_t g = bn == 32 ? 32u : 64u;
-        cuuint64_t dims[4] = {(cuuint64_t)x_cstride, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n_img};
-        cuuint64_t str[3] = {(cuuint64_t)x_cstride * 2, (cuuint64_t)w * x_cstride * 2, (cuuint64_t)h * w * x_cstride * 2};
-        cuuint32_t box[4] = {g, 64, 1, 1};
-        if (!make_map(&mb, x, 4, dims, str, box, g == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))
-            return cudaErrorInvalidValue;
-    }
     wgrad_args p{};
     p.n_img = n_img;
     p.h = h;
@@ -1132,32 +1299,11 @@ extern "C" cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cs
     p.cout = cout;
     p.cin = cin;
     p.x_coff = x_coff;
-    p.total_kb = (int)(P / 64);
-    p.a_rows = a_rows;
-    // about 8 CTAs per SM over the three launches' taps and tiles
-    // input channel tiles of at most 64: the column taps packed into N
-    const bool dxp = bn <= 64;
-    const int mtiles = (cout + 127) / 128;
-    const int per_split = (pack ? 1 : 3) * (dxp ? 1 : 3) * mtiles * (cin / bn);
-    int splits = (152 * 8 / 3 + per_split - 1) / per_split;
-    if (splits > p.total_kb) splits = p.total_kb;
-    if (splits < 1) splits = 1;
-    p.kpc = (p.total_kb + splits - 1) / splits;
-    splits = (p.total_kb + p.kpc - 1) / p.kpc;
     p.dw = dw;
+    p.vec = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
     p.err = err;
-    for (int d = 0; d < (dxp ? 1 : 3); d++) {
-        p.dx = d - 1;
-        cudaError_t e;
-        if (dxp) {
-            if (bn == 64) e = pack ? launch_wgrad<64, true, true>(ma, mb, p, splits, s) : launch_wgrad<64, false, true>(ma, mb, p, splits, s);
-            else e = pack ? launch_wgrad<32, true, true>(ma, mb, p, splits, s) : launch_wgrad<32, false, true>(ma, mb, p, splits, s);
-        } else if (pack) {
-            e = bn == 256 ? launch_wgrad<256, true, false>(ma, mb, p, splits, s) : launch_wgrad<128, true, false>(ma, mb, p, splits, s);
-        } else {
-            e = bn == 256 ? launch_wgrad<256, false, false>(ma, mb, p, splits, s) : launch_wgrad<128, false, false>(ma, mb, p, splits, s);
-        }
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    if (cout > 64) return launch_wgrad_cols(dy, x, x_cstride, p, s);
+    if (cout == 32)
+        return cin % 64 ? launch_wgrad_rows<32, 32>(dy, x, x_cstride, p, s) : launch_wgrad_rows<32, 64>(dy, x, x_cstride, p, s);
+    return cin % 64 ? launch_wgrad_rows<64, 32>(dy, x, x_cstride, p, s) : launch_wgrad_rows<64, 64>(dy, x, x_cstride, p, s);
 }
