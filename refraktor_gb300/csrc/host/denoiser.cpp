@@ -75,7 +75,7 @@ struct workspace {
     bool train = false;
     std::vector<void*> owned;
     bf16 *x, *a1, *cat1, *e1, *d1;
-    float* out;
+    float4* out;  // the network's three channels and padding
     bf16 *p1, *a2, *cat2, *e2, *d2;
     bf16 *p2, *a3, *cat3, *e3, *d3;
     bf16 *p3, *b1, *b2;
@@ -129,7 +129,7 @@ struct rfk_denoiser {
         s->cat1 = s->take<bf16>(P1 * 96);
         s->e1 = s->take<bf16>(P1 * 32);
         s->d1 = s->take<bf16>(P1 * 32);
-        s->out = s->take<float>(P1 * 32);
+        s->out = s->take<float4>(P1);
         s->p1 = s->take<bf16>(P2 * 32);
         s->a2 = s->take<bf16>(P2 * 64);
         s->cat2 = s->take<bf16>(P2 * 192);
@@ -216,7 +216,7 @@ struct rfk_denoiser {
         }
         conv(D1A, s.cat1, H, W, n, 96, 0, s.e1, 32, 0, R, st);
         conv(D1B, s.e1, H, W, n, 32, 0, s.d1, 32, 0, R, st);
-        conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 32, 0, RFK_UNET_F32OUT | A, st);
+        conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 4, 0, RFK_UNET_RGBOUT | A, st);
     }
 
     // Gradients of layer l from dY (dense, cout channels, pre-activation) and
@@ -225,9 +225,7 @@ struct rfk_denoiser {
     void back(workspace& s, int l, const bf16* dy, int n, int h, int w, const bf16* x, int x_cstride, int x_coff, bf16* dx,
               int dx_cstride, int dx_coff, const bf16* mask, cudaStream_t st) {
         const layer& y = L[l];
-        const size_t P = (size_t)n * h * w;
-        cuda_check(rfk_unet_bias_grad(dy, P, y.d.cout, y.bg, st), "bias grad");
-        cuda_check(rfk_unet_wgrad3x3(dy, x, x_cstride, x_coff, n, h, w, y.d.cout, y.d.cin, y.g, d_err, st), "wgrad");
+        cuda_check(rfk_unet_wgrad3x3_bias(dy, x, x_cstride, x_coff, n, h, w, y.d.cout, y.d.cin, y.g, y.bg, d_err, st), "wgrad");
         if (dx)
             cuda_check(rfk_unet_conv3x3(dy, n, h, w, y.d.cout, 0, y.d.cout, y.wb, y.d.cin, nullptr, RFK_UNET_ANY_ORDER, dx, dx_cstride, dx_coff,
                                         mask, y.d.cin, 0, 0, d_err, st),

@@ -15,6 +15,8 @@
 #define RFK_UNET_ANY_ORDER 8  // conv: the f32 sums may be ordered and split as is fastest (inference and input
                               // gradients); without it the order is fixed, so that a training loss is reproducible
 
+#define RFK_UNET_RGBOUT 16  // conv epilogue: store the first four channels as f32 (cstride 4)
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -33,6 +35,9 @@ cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w, int in_cst
 // x_cstride. w must be a multiple of 64, cin and cout of 32.
 cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w, int cout,
                               int cin, float* dw, int* err, cudaStream_t s);
+// The same, and db[n] += sum over pixels of dY[p][n] (db may be null).
+cudaError_t rfk_unet_wgrad3x3_bias(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w, int cout,
+                                   int cin, float* dw, float* db, int* err, cudaStream_t s);
 
 
 // Network input (32 bf16 channels per pixel) of a float4 histogram rendered at `spp` and its
@@ -50,18 +55,16 @@ cudaError_t rfk_unet_up_backward(const void* g, int gcstride, int gcoff, const v
 // Gradient of a skip slice feeding a concatenation and an average pool, times its ReLU derivative.
 cudaError_t rfk_unet_skip_backward(const void* gcat, int cstride, int coff, const void* gpool, const void* cat, int n_img,
                                    int h, int w, int c, void* out, cudaStream_t s);
-// Mean squared error of base + channels 0..2 (f32 output, 32 per pixel) against f32 RGBA targets;
+// Mean squared error of base + output (RFK_UNET_RGBOUT) against f32 RGBA targets;
 // bf16 gradient.
-cudaError_t rfk_unet_mse(const float* out, const float4* base, const float4* target, size_t npx, void* grad, double* loss,
+cudaError_t rfk_unet_mse(const float4* out, const float4* base, const float4* target, size_t npx, void* grad, double* loss,
                          cudaStream_t s);
-// db[c] += sum over pixels of g[p][c].
-cudaError_t rfk_unet_bias_grad(const void* g, size_t npx, int c, float* db, cudaStream_t s);
 // Adam step of one layer (f32 master weights and bias) writing the bf16 forward and input-gradient copies.
 cudaError_t rfk_unet_adam(float* w, float* m, float* v, const float* g, int cout, int cin, int live_out, int live_in,
                           float lr, float b1, float b2, float eps, int step, void* wf, void* wb, float* bias, float* bm,
                           float* bv, const float* bg, cudaStream_t s);
 // base + network output to an image (RFK_HALF3 .. RFK_FLOAT4; alpha as the tonemapper's).
-cudaError_t rfk_unet_to_image(const float* net, const float4* base, const float4* bins, size_t npx, void* out, int format,
+cudaError_t rfk_unet_to_image(const float4* net, const float4* base, const float4* bins, size_t npx, void* out, int format,
                               cudaStream_t s);
 
 #ifdef __cplusplus

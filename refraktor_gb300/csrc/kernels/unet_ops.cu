@@ -164,56 +164,44 @@ __global__ void skip_backward_kernel(const bf16* __restrict__ gcat, int cstride,
     st8(out + (size_t)i * 8, gc);
 }
 
-// Mean squared error of the prediction base + out[0..2] (out f32, cstride 32;
-// the network predicts a correction of the tonemapped low-spp image) against
-// target (f32, 4 per pixel), and its gradient as bf16 (channels 3..31 zero).
-__global__ void mse_kernel(const float* __restrict__ out, const float4* __restrict__ base, const float4* __restrict__ target,
-                           size_t npx, float inv_n, bf16* __restrict__ grad, double* __restrict__ loss) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    if (i < npx) {
-        const float4 t = target[i];
-        const float4 b = base[i];
-        const float* o = out + i * 32;
-        const float d0 = b.x + o[0] - t.x, d1 = b.y + o[1] - t.y, d2 = b.z + o[2] - t.z;
-        l = d0 * d0 + d1 * d1 + d2 * d2;
-        __nv_bfloat162 hh[16];
-        hh[0] = __floats2bfloat162_rn(2.0f * d0 * inv_n, 2.0f * d1 * inv_n);
-        hh[1] = __floats2bfloat162_rn(2.0f * d2 * inv_n, 0.0f);
-#pragma unroll
-        for (int j = 2; j < 16; j++) hh[j] = __floats2bfloat162_rn(0.0f, 0.0f);
-        uint4* g = reinterpret_cast<uint4*>(grad + i * 32);
-#pragma unroll
-        for (int q = 0; q < 4; q++) g[q] = reinterpret_cast<uint4*>(hh)[q];
-    }
-    for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.0f) atomicAdd(loss, (double)l);
-}
-
-// Per-channel sum over pixels (bias gradient): db[c] += sum_p g[p][c]. A
-// thread sums one 8-channel chunk over a strided run of pixels; the block
-// reduces in shared memory and adds once per channel.
-__global__ void bias_grad_kernel(const bf16* __restrict__ g, unsigned npx, int c, float* __restrict__ db) {
-    extern __shared__ float red[];  // [c]
-    const int c8 = c / 8;
-    for (int j = threadIdx.x; j < c; j += blockDim.x) red[j] = 0.0f;
-    __syncthreads();
-    const int q = threadIdx.x % c8;
-    const int lanes = blockDim.x / c8;
-    const int lane = threadIdx.x / c8;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (lane < lanes) {
-        for (unsigned p = blockIdx.x * lanes + lane; p < npx; p += gridDim.x * lanes) {
-            float v[8];
-            ld8(g + (size_t)p * c + q * 8, v);
-#pragma unroll
-            for (int j = 0; j < 8; j++) acc[j] += v[j];
+// Mean squared error of the prediction base + out (the network predicts a
+// correction of the tonemapped low-spp image) against target, all f32, 4 per
+// pixel, and its gradient as bf16 (channels 3..31 zero). A warp takes 32 pixels
+// at a time, so that its stores are 512 contiguous bytes; a block adds its
+// squares once. 16 images of 512 x 512: 72 us; with an atomic per warp, 64-byte
+// strides between the lanes' stores and 32 f32 channels in `out` 321.
+__global__ void __launch_bounds__(256) mse_kernel(const float4* __restrict__ out, const float4* __restrict__ base,
+                                                  const float4* __restrict__ target, size_t npx, float inv_n,
+                                                  uint4* __restrict__ grad, double* __restrict__ loss) {
+    const unsigned lane = threadIdx.x & 31u;
+    double sum = 0.0;
+    for (size_t p0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * 32; p0 < npx; p0 += (size_t)gridDim.x * blockDim.x) {
+        const size_t i = p0 + lane;
+        uint2 g = make_uint2(0u, 0u);
+        if (i < npx) {
+            const float4 t = target[i], b = base[i], o = out[i];
+            const float d0 = b.x + o.x - t.x, d1 = b.y + o.y - t.y, d2 = b.z + o.z - t.z;
+            sum += (double)(d0 * d0 + d1 * d1 + d2 * d2);
+            const __nv_bfloat162 h0 = __floats2bfloat162_rn(2.0f * d0 * inv_n, 2.0f * d1 * inv_n);
+            const __nv_bfloat162 h1 = __floats2bfloat162_rn(2.0f * d2 * inv_n, 0.0f);
+            g = make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
         }
 #pragma unroll
-        for (int j = 0; j < 8; j++) atomicAdd(&red[q * 8 + j], acc[j]);
+        for (unsigned k = 0; k < 4; k++) {
+            // 16-byte piece lane % 4 of pixel 8 k + lane / 4
+            const unsigned px = 8 * k + lane / 4;
+            const unsigned x = __shfl_sync(0xffffffffu, g.x, px), y = __shfl_sync(0xffffffffu, g.y, px);
+            if (p0 + px < npx) grad[(p0 + px) * 4 + lane % 4] = lane % 4 ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(x, y, 0u, 0u);
+        }
     }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    __shared__ double part[8];
+    if (lane == 0) part[threadIdx.x / 32] = sum;
     __syncthreads();
-    for (int j = threadIdx.x; j < c; j += blockDim.x) atomicAdd(db + j, red[j]);
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; k++) sum += part[k];
+        atomicAdd(loss, sum);
+    }
 }
 
 // Adam (Kingma & Ba 2015) on one conv layer's f32 master weights [cout][9][cin]
@@ -264,14 +252,13 @@ __global__ void adam_bias_kernel(float* __restrict__ b, float* __restrict__ m, f
 // Prediction (base + network output) to an image in the tonemapper's formats,
 // clamped to [0, 1]; alpha from the histogram as the tonemapper's.
 template <int CH, bool HALF>
-__global__ void to_image_kernel(const float* __restrict__ net, const float4* __restrict__ base,
+__global__ void to_image_kernel(const float4* __restrict__ net, const float4* __restrict__ base,
                                 const float4* __restrict__ bins, size_t npx, void* out) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npx) return;
-    const float* o = net + i * 32;
-    const float4 b = base[i];
-    float v[4] = {fminf(fmaxf(b.x + o[0], 0.0f), 1.0f), fminf(fmaxf(b.y + o[1], 0.0f), 1.0f),
-                  fminf(fmaxf(b.z + o[2], 0.0f), 1.0f), 0.0f};
+    const float4 o = net[i], b = base[i];
+    float v[4] = {fminf(fmaxf(b.x + o.x, 0.0f), 1.0f), fminf(fmaxf(b.y + o.y, 0.0f), 1.0f),
+                  fminf(fmaxf(b.z + o.z, 0.0f), 1.0f), 0.0f};
     if (CH == 4) {
         const float d = bins[i].w;
         v[3] = d > 0.0f ? fminf(fmaxf(logf(d) * (4.0f / 0.69314718f) / 96.0f, 0.0f), 1.0f) : 0.0f;
@@ -335,21 +322,11 @@ extern "C" cudaError_t rfk_unet_skip_backward(const void* gcat, int cstride, int
     return cudaGetLastError();
 }
 
-extern "C" cudaError_t rfk_unet_mse(const float* out, const float4* base, const float4* target, size_t npx, void* grad,
+extern "C" cudaError_t rfk_unet_mse(const float4* out, const float4* base, const float4* target, size_t npx, void* grad,
                                     double* loss, cudaStream_t s) {
     if (npx == 0) return cudaSuccess;
-    mse_kernel<<<blocks_for(npx), 256, 0, s>>>(out, base, target, npx, 1.0f / (3.0f * (float)npx), static_cast<bf16*>(grad),
-                                                loss);
-    return cudaGetLastError();
-}
-
-extern "C" cudaError_t rfk_unet_bias_grad(const void* g, size_t npx, int c, float* db, cudaStream_t s) {
-    if (c % 8 || c > 2048 || npx == 0 || npx > 0xFFFFFFFFull) return cudaErrorInvalidValue;
-    const unsigned lanes = 256 / (c / 8) > 0 ? 256 / (c / 8) : 1;
-    unsigned bx = (unsigned)((npx + lanes * 64 - 1) / (lanes * 64));
-    if (bx > 152 * 4) bx = 152 * 4;
-    const unsigned threads = (c / 8) > 256 ? (unsigned)(c / 8) : 256;
-    bias_grad_kernel<<<bx, threads, (size_t)c * sizeof(float), s>>>(static_cast<const bf16*>(g), (unsigned)npx, c, db);
+    const unsigned blocks = npx / 256 < 152 * 8 ? blocks_for(npx) : 152 * 8;
+    mse_kernel<<<blocks, 256, 0, s>>>(out, base, target, npx, 1.0f / (3.0f * (float)npx), static_cast<uint4*>(grad), loss);
     return cudaGetLastError();
 }
 
@@ -364,7 +341,7 @@ extern "C" cudaError_t rfk_unet_adam(float* w, float* m, float* v, const float* 
     return cudaGetLastError();
 }
 
-extern "C" cudaError_t rfk_unet_to_image(const float* net, const float4* base, const float4* bins, size_t npx, void* out,
+extern "C" cudaError_t rfk_unet_to_image(const float4* net, const float4* base, const float4* bins, size_t npx, void* out,
                                          int format, cudaStream_t s) {
     if (npx == 0) return cudaSuccess;
     switch (format) {

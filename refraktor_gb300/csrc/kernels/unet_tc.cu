@@ -50,6 +50,7 @@ struct conv_args {
     const float* bias;
     int relu;
     int out_f32;  // store f32 instead of bf16
+    int out_rgb;  // f32: the first four channels only
     int up2;      // store at the 2x2 pixels of a (2h, 2w) output
     const bf16* mask;
     int mask_cstride, mask_coff;
@@ -190,9 +191,14 @@ __device__ __forceinline__ void conv_activate(const conv_args& p, float (&v)[N],
     }
 }
 
-// f32 and accumulating outputs: a lane stores its pixel's N channels.
+// f32 and accumulating outputs: a lane stores its pixel's N channels from ch on.
 template <int N>
-__device__ __forceinline__ void store_direct(const conv_args& p, float (&v)[N], size_t at) {
+__device__ __forceinline__ void store_direct(const conv_args& p, float (&v)[N], size_t pix, int ch) {
+    if (p.out_rgb) {
+        if (ch == 0) static_cast<float4*>(p.out)[pix] = make_float4(v[0], v[1], v[2], v[3]);
+        return;
+    }
+    const size_t at = pix * p.out_cstride + p.out_coff + ch;
     if (p.out_f32) {
         float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.out) + at);
 #pragma unroll
@@ -256,12 +262,13 @@ __device__ __forceinline__ void conv_epilogue(const conv_args& p, uint32_t acc, 
         const size_t pix = ((size_t)img * p.h + (valid ? y : 0)) * p.w + (valid ? x : 0);
 #pragma unroll 1
         for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 16) {
+            if (p.out_rgb && n0 + c) break;
             float v[16];
             tc::tmem_ld16(acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(r * BN + c), v);
             if (!valid) continue;
             conv_bias<16>(p, v, n0 + c);
             conv_activate<16>(p, v, n0 + c, pix, true);
-            store_direct<16>(p, v, pix * p.out_cstride + p.out_coff + n0 + c);
+            store_direct<16>(p, v, pix, n0 + c);
         }
     }
 }
@@ -689,7 +696,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_rows(const __grid_constant__ C
                     tc::named_barrier(1 + group, 128);
                     if (leader) store_row(p, &tmO, tile, p.out_coff + n0, xt, img * p.h + y);
                 } else if (valid) {
-                    store_direct<32>(p, v, pix * p.out_cstride + p.out_coff + n0);
+                    store_direct<32>(p, v, pix, n0);
                 }
             }
             g0 += (uint32_t)rows + 2u;
@@ -711,6 +718,7 @@ struct wgrad_args {
     int kpc;        // stages (wgrad3x3_rows) or rows (wgrad3x3_cols) of a 64-pixel segment per CTA
     int total;      // all of them
     float* dw;      // [cout][9][cin]
+    float* db;      // [cout]: sum of dY (null: not wanted)
     int vec;        // dw is 16-byte aligned
     int* err;
 };
@@ -726,6 +734,41 @@ __device__ __forceinline__ void wgrad_add(float* dst, const float (&v)[32], int 
     } else {
 #pragma unroll
         for (int j = 0; j < 32; j++) atomicAdd(dst + j, v[j]);
+    }
+}
+
+// Bias gradient on the way: two warps that no MMA or copy needs add up the rows of
+// dY while these are in shared memory (those of the first input channel tile), a
+// pass over dY of its own less per layer (16 images of 512 x 512: 690 us of the
+// 15 layers of a step; the weight gradients take 40 us longer in all).
+// One row of 64 pixels x CO channels as TMA left it (swizzled 64- or 128-byte
+// pixel lines), CO / 8 lanes to a pixel, by thread t of 64; acc: this lane's 8 channels.
+template <int CO>
+__device__ __forceinline__ void bias_row(const uint8_t* row, int t, float (&acc)[8]) {
+    constexpr int L = CO / 8, PX = 64 / L;  // lanes per pixel, pixels at a time
+    const int c = t % L, px = t / L, sw = c ^ (CO == 64 ? px & 7 : px >> 1 & 3);
+#pragma unroll
+    for (int i = 0; i < 64 / PX; i++) {
+        const uint4 u = *reinterpret_cast<const uint4*>(row + (px + i * PX) * (CO * 2) + sw * 16);
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float2 f = __bfloat1622float2(h[j]);
+            acc[2 * j] += f.x;
+            acc[2 * j + 1] += f.y;
+        }
+    }
+}
+
+// The warp's sums of its lanes with the same channels, into db[0 .. min(CO, n)).
+template <int CO>
+__device__ __forceinline__ void bias_add(float* db, int n, int lane, float (&acc)[8]) {
+    constexpr int L = CO / 8;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+#pragma unroll
+        for (int o = L; o < 32; o *= 2) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+        if (lane < L && lane * 8 + j < n) atomicAdd(db + lane * 8 + j, acc[j]);
     }
 }
 
@@ -776,12 +819,13 @@ __global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUt
     int nk = p.total - kb0;
     if (nk > p.kpc) nk = p.kpc;
     if (nk < 0) nk = 0;
+    const bool bias = p.db != nullptr && blockIdx.y == 0;
 
     if (warp == 0) tc::tmem_alloc(&tmem_base, C::ACCS * C::ACC_COLS);
     if (threadIdx.x == 32) {
         for (int s = 0; s < C::STAGES; s++) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 1);
+            tc::mbar_init(&empty[s], bias ? 3 : 1);
         }
         tc::mbar_init(&done, 1);
         s_fail = 0;
@@ -847,6 +891,22 @@ __global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUt
         }
         tc::mma_commit(one, &done);
         if (!ok) atomicExch(&s_fail, 1);
+    } else if (warp >= 2 && bias) {
+        const int t = threadIdx.x - 64;
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (int kb = 0; kb < nk; kb++) {
+            const int s = kb % C::STAGES, r = kb / C::STAGES;
+            if (!tc::all_lanes(tc::mbar_wait(&full[s], r & 1))) {
+                if (lane == 0) atomicExch(&s_fail, 1);
+                break;
+            }
+            const uint8_t* sa = base + (size_t)s * C::STAGE_BYTES;
+            for (int y = 1; y <= C::R; y++) bias_row<CO>(sa + y * C::A_GROUP, t, acc);  // rows past the image are zero
+            __syncwarp();
+            if (lane == 0) mbar_arrive_n(&empty[s], 1u);
+        }
+        __syncwarp();
+        bias_add<CO>(p.db, CO, lane, acc);
     }
     __syncwarp();
 
@@ -908,12 +968,13 @@ __global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUt
     const int segs_x = p.w / 64;
     // rows of this CTA, counted down the columns one after another
     const int row0 = blockIdx.x * p.kpc, row1 = min(row0 + p.kpc, p.total);
+    const bool bias = p.db != nullptr && c0 == 0;
 
     if (warp == 0) tc::tmem_alloc(&tmem_base, 512u);
     if (threadIdx.x == 32) {
         for (int s = 0; s < C::STAGES; s++) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 1);
+            tc::mbar_init(&empty[s], bias ? 3 : 1);
         }
         tc::mbar_init(&done, 1);
         s_fail = 0;
@@ -993,6 +1054,31 @@ __global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUt
         }
         tc::mma_commit(one, &done);
         if (!ok) atomicExch(&s_fail, 1);
+    } else if (warp >= 2 && bias) {
+        const int t = threadIdx.x - 64;
+        float lo[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hi[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        bool ok = true;
+        int k = 0;
+        for (int row = row0; ok && row < row1;) {
+            const int y0 = row % p.h, y1 = min(y0 + row1 - row, p.h);
+            for (int y = y0 - 1; y <= y1; y++, k++) {
+                const int s = k % C::STAGES;
+                ok = tc::all_lanes(tc::mbar_wait(&full[s], (k / C::STAGES) & 1));
+                if (!ok) break;
+                const uint8_t* sa = base + (size_t)s * C::STAGE_BYTES;
+                if (y >= y0 && y < y1) {
+                    bias_row<64>(sa, t, lo);
+                    bias_row<64>(sa + C::A_GROUP, t, hi);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(&empty[s], 1u);
+            }
+            row += y1 - y0;
+        }
+        if (!ok && lane == 0) atomicExch(&s_fail, 1);
+        __syncwarp();
+        bias_add<64>(p.db + m0, p.cout - m0, lane, lo);
+        bias_add<64>(p.db + m0 + 64, p.cout - m0 - 64, lane, hi);
     }
     __syncwarp();
 
@@ -1176,10 +1262,12 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
                                         const void* weights, int cout, const float* bias, int flags, void* out,
                                         int out_cstride, int out_coff, const void* mask, int mask_cstride, int mask_coff,
                                         int accumulate, int* err, cudaStream_t s) {
-    if (cin % 32 || in_coff % 32 || in_cstride % 32 || cout % 32 || out_coff % 32 || out_cstride % 32) return cudaErrorInvalidValue;
-    if (mask && (mask_coff % 32 || mask_cstride % 32)) return cudaErrorInvalidValue;
-    if (in_coff + cin > in_cstride || out_coff + cout > out_cstride || n_img <= 0 || h <= 0 || w <= 0)
+    const bool rgb = (flags & RFK_UNET_RGBOUT) != 0;
+    if (cin % 32 || in_coff % 32 || in_cstride % 32 || cout % 32) return cudaErrorInvalidValue;
+    if (rgb ? accumulate || out_coff || out_cstride != 4 : out_coff % 32 || out_cstride % 32 || out_coff + cout > out_cstride)
         return cudaErrorInvalidValue;
+    if (mask && (mask_coff % 32 || mask_cstride % 32)) return cudaErrorInvalidValue;
+    if (in_coff + cin > in_cstride || n_img <= 0 || h <= 0 || w <= 0) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weights) | reinterpret_cast<uintptr_t>(out)) & 63)
         return cudaErrorMisalignedAddress;
     const bool wide_k = cin % 64 == 0 && in_coff % 64 == 0;
@@ -1236,7 +1324,8 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
     p.out_coff = out_coff;
     p.bias = bias;
     p.relu = flags & RFK_UNET_RELU;
-    p.out_f32 = (flags & RFK_UNET_F32OUT) ? 1 : 0;
+    p.out_rgb = rgb;
+    p.out_f32 = rgb || (flags & RFK_UNET_F32OUT);
     p.up2 = up2;
     if (p.up2 && (p.out_f32 || accumulate)) return cudaErrorInvalidValue;
     p.mask = static_cast<const bf16*>(mask);
@@ -1289,6 +1378,11 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
 
 extern "C" cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w,
                                          int cout, int cin, float* dw, int* err, cudaStream_t s) {
+    return rfk_unet_wgrad3x3_bias(dy, x, x_cstride, x_coff, n_img, h, w, cout, cin, dw, nullptr, err, s);
+}
+
+extern "C" cudaError_t rfk_unet_wgrad3x3_bias(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w,
+                                              int cout, int cin, float* dw, float* db, int* err, cudaStream_t s) {
     if (w % 64 || cin % 32 || cout <= 0 || cout % 32 || n_img <= 0 || h <= 0) return cudaErrorInvalidValue;
     if (x_coff % 32 || x_cstride % 32 || x_coff + cin > x_cstride) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 63) return cudaErrorMisalignedAddress;
@@ -1300,6 +1394,7 @@ extern "C" cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cs
     p.cin = cin;
     p.x_coff = x_coff;
     p.dw = dw;
+    p.db = db;
     p.vec = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
     p.err = err;
     if (cout > 64) return launch_wgrad_cols(dy, x, x_cstride, p, s);

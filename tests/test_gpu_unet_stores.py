@@ -51,3 +51,24 @@ def test_conv_stores_only_its_slice(n, h, w, cin, cout, any_order, up):
     assert bool(((got[..., off:off + cout].float() - ref).abs() <= bound).all())
     assert torch.equal(buf[:px, :off], before[:px, :off]) and torch.equal(buf[:px, off + cout:], before[:px, off + cout:])
     assert torch.equal(buf[px:], before[px:])
+
+
+@pytest.mark.parametrize("any_order", [False, True])
+@pytest.mark.parametrize("n,h,w,cin,cout", [(1, 1, 8, 32, 32), (2, 5, 200, 32, 32), (1, 41, 129, 96, 32), (1, 3, 130, 64, 64)])
+def test_conv_rgb_output_is_the_f32_output(n, h, w, cin, cout, any_order):
+    """The first four channels, one float4 per pixel and nothing past them, bit for bit as the full f32 output has them."""
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(w + cin)
+    x = torch.randn(n, h, w, cin, device="cuda", generator=g).to(torch.bfloat16)
+    wt = (torch.randn(cout, 9, cin, device="cuda", generator=g) / np.sqrt(9 * cin)).to(torch.bfloat16)
+    b = torch.randn(cout, device="cuda", generator=g)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = []
+    for flag, cs in ((2, cout), (16, 4)):
+        buf = torch.full((n * h * w * cs + 64,), 7.0, device="cuda")
+        rc = L.rfk_unet_conv3x3(x.data_ptr(), n, h, w, cin, 0, cin, wt.data_ptr(), cout, b.data_ptr(), flag | (8 if any_order else 0),
+                                buf.data_ptr(), cs, 0, None, 0, 0, 0, err.data_ptr(), None)
+        torch.cuda.synchronize()
+        assert rc == 0 and int(err.item()) == 0 and bool((buf[n * h * w * cs:] == 7.0).all())
+        outs.append(buf[:n * h * w * cs].view(n, h, w, cs))
+    assert torch.equal(outs[0][..., :4], outs[1])
