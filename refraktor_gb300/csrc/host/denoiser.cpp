@@ -227,7 +227,7 @@ struct rfk_denoiser {
         const layer& y = L[l];
         cuda_check(rfk_unet_wgrad3x3_bias(dy, x, x_cstride, x_coff, n, h, w, y.d.cout, y.d.cin, y.g, y.bg, d_err, st), "wgrad");
         if (dx)
-            cuda_check(rfk_unet_conv3x3(dy, n, h, w, y.d.cout, 0, y.d.cout, y.wb, y.d.cin, nullptr, RFK_UNET_ANY_ORDER, dx, dx_cstride, dx_coff,
+            cuda_check(rfk_unet_conv3x3(dy, n, h, w, y.d.cout, 0, y.d.cout, y.wb, y.d.cin, nullptr, 0, dx, dx_cstride, dx_coff,
                                         mask, y.d.cin, 0, 0, d_err, st),
                        "dgrad");
     }
