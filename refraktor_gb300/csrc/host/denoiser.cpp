@@ -76,9 +76,9 @@ struct workspace {
     std::vector<void*> owned;
     bf16 *x, *a1, *cat1, *e1, *d1;
     float4* out;  // the network's three channels and padding
-    bf16 *p1, *a2, *cat2, *e2, *d2;
-    bf16 *p2, *a3, *cat3, *e3, *d3;
-    bf16 *p3, *b1, *b2;
+    bf16 *p1, *a2, *cat2, *e2;
+    bf16 *p2, *a3, *cat3, *e3;
+    bf16 *p3, *b1;
     // training only
     bf16 *g_out, *gl1a, *gl1b, *g_cat1;
     bf16 *gl2a, *gl2b, *g_cat2, *g_p1;
@@ -100,6 +100,8 @@ struct workspace {
 
 struct rfk_denoiser {
     layer L[NLAYERS];
+    float* grads = nullptr;  // all layers' g and bg, one after another
+    size_t ngrads = 0;
     int step = 0;
     int* d_err = nullptr;
     double* d_loss = nullptr;
@@ -107,9 +109,9 @@ struct rfk_denoiser {
 
     ~rfk_denoiser() {
         for (auto& l : L)
-            for (void* p : {(void*)l.w, (void*)l.m, (void*)l.v, (void*)l.g, (void*)l.b, (void*)l.bm, (void*)l.bv,
-                            (void*)l.bg, (void*)l.wf, (void*)l.wb})
+            for (void* p : {(void*)l.w, (void*)l.m, (void*)l.v, (void*)l.b, (void*)l.bm, (void*)l.bv, (void*)l.wf, (void*)l.wb})
                 if (p) cudaFree(p);
+        if (grads) cudaFree(grads);
         if (d_err) cudaFree(d_err);
         if (d_loss) cudaFree(d_loss);
     }
@@ -134,15 +136,12 @@ struct rfk_denoiser {
         s->a2 = s->take<bf16>(P2 * 64);
         s->cat2 = s->take<bf16>(P2 * 192);
         s->e2 = s->take<bf16>(P2 * 64);
-        s->d2 = s->take<bf16>(P2 * 64);
         s->p2 = s->take<bf16>(P3 * 64);
         s->a3 = s->take<bf16>(P3 * 128);
         s->cat3 = s->take<bf16>(P3 * 384);
         s->e3 = s->take<bf16>(P3 * 128);
-        s->d3 = s->take<bf16>(P3 * 128);
         s->p3 = s->take<bf16>(P4 * 128);
         s->b1 = s->take<bf16>(P4 * 256);
-        s->b2 = s->take<bf16>(P4 * 256);
         if (train) {
             s->g_out = s->take<bf16>(P1 * 32);
             s->gl1a = s->take<bf16>(P1 * 32);
@@ -173,12 +172,10 @@ struct rfk_denoiser {
                    "conv");
     }
 
-    // Forward pass of the whole network on ws.x; the result in ws.out. For
-    // inference (`infer`) the last convolution of each decoder level and of
-    // the bottleneck writes its output straight into the next level's
-    // concatenation at twice the resolution (the upsampling fused into its
-    // epilogue); training keeps the low-resolution activations, which the
-    // backward pass reads, and upsamples them in a pass of its own.
+    // Forward pass of the whole network on ws.x; the result in ws.out. The last
+    // convolution of each decoder level and of the bottleneck writes its output
+    // straight into the next level's concatenation at twice the resolution (the
+    // upsampling fused into its epilogue). `infer`: sums in any order.
     void forward(workspace& s, cudaStream_t st, bool infer = false) {
         const int n = s.n, H = s.h, W = s.w;
         const int H2 = H / 2, W2 = W / 2, H3 = H / 4, W3 = W / 4, H4 = H / 8, W4 = W / 8;
@@ -194,26 +191,11 @@ struct rfk_denoiser {
         cuda_check(rfk_unet_avgpool(s.cat3, n, H3, W3, 384, 256, 128, s.p3, st), "pool");
         conv(B1, s.p3, H4, W4, n, 128, 0, s.b1, 256, 0, R, st);
         const int U = R | RFK_UNET_UP2;
-        if (infer) {
-            conv(B2, s.b1, H4, W4, n, 256, 0, s.cat3, 384, 0, U, st);
-        } else {
-            conv(B2, s.b1, H4, W4, n, 256, 0, s.b2, 256, 0, R, st);
-            cuda_check(rfk_unet_upsample(s.b2, n, H4, W4, 256, s.cat3, 384, 0, st), "upsample");
-        }
+        conv(B2, s.b1, H4, W4, n, 256, 0, s.cat3, 384, 0, U, st);
         conv(D3A, s.cat3, H3, W3, n, 384, 0, s.e3, 128, 0, R, st);
-        if (infer) {
-            conv(D3B, s.e3, H3, W3, n, 128, 0, s.cat2, 192, 0, U, st);
-        } else {
-            conv(D3B, s.e3, H3, W3, n, 128, 0, s.d3, 128, 0, R, st);
-            cuda_check(rfk_unet_upsample(s.d3, n, H3, W3, 128, s.cat2, 192, 0, st), "upsample");
-        }
+        conv(D3B, s.e3, H3, W3, n, 128, 0, s.cat2, 192, 0, U, st);
         conv(D2A, s.cat2, H2, W2, n, 192, 0, s.e2, 64, 0, R, st);
-        if (infer) {
-            conv(D2B, s.e2, H2, W2, n, 64, 0, s.cat1, 96, 0, U, st);
-        } else {
-            conv(D2B, s.e2, H2, W2, n, 64, 0, s.d2, 64, 0, R, st);
-            cuda_check(rfk_unet_upsample(s.d2, n, H2, W2, 64, s.cat1, 96, 0, st), "upsample");
-        }
+        conv(D2B, s.e2, H2, W2, n, 64, 0, s.cat1, 96, 0, U, st);
         conv(D1A, s.cat1, H, W, n, 96, 0, s.e1, 32, 0, R, st);
         conv(D1B, s.e1, H, W, n, 32, 0, s.d1, 32, 0, R, st);
         conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 4, 0, RFK_UNET_RGBOUT | A, st);
@@ -235,24 +217,21 @@ struct rfk_denoiser {
     void backward(workspace& s, cudaStream_t st) {
         const int n = s.n, H = s.h, W = s.w;
         const int H2 = H / 2, W2 = W / 2, H3 = H / 4, W3 = W / 4, H4 = H / 8, W4 = W / 8;
-        for (auto& y : L) {
-            cuda_check(cudaMemsetAsync(y.g, 0, y.nw() * sizeof(float), st), "zero grads");
-            cuda_check(cudaMemsetAsync(y.bg, 0, y.d.cout * sizeof(float), st), "zero grads");
-        }
+        cuda_check(cudaMemsetAsync(grads, 0, ngrads * sizeof(float), st), "zero grads");
         // level 1, decoder side
         back(s, L_OUT, s.g_out, n, H, W, s.d1, 32, 0, s.gl1a, 32, 0, s.d1, st);     // gl1a = gp_d1
         back(s, D1B, s.gl1a, n, H, W, s.e1, 32, 0, s.gl1b, 32, 0, s.e1, st);        // gl1b = gp_e1
         back(s, D1A, s.gl1b, n, H, W, s.cat1, 96, 0, s.g_cat1, 96, 0, nullptr, st);
         // level 2
-        cuda_check(rfk_unet_up_backward(s.g_cat1, 96, 0, s.d2, n, H2, W2, 64, s.gl2a, st), "up backward");
+        cuda_check(rfk_unet_up_backward(s.g_cat1, 96, 0, s.cat1, n, H2, W2, 64, s.gl2a, st), "up backward");
         back(s, D2B, s.gl2a, n, H2, W2, s.e2, 64, 0, s.gl2b, 64, 0, s.e2, st);
         back(s, D2A, s.gl2b, n, H2, W2, s.cat2, 192, 0, s.g_cat2, 192, 0, nullptr, st);
         // level 3
-        cuda_check(rfk_unet_up_backward(s.g_cat2, 192, 0, s.d3, n, H3, W3, 128, s.gl3a, st), "up backward");
+        cuda_check(rfk_unet_up_backward(s.g_cat2, 192, 0, s.cat2, n, H3, W3, 128, s.gl3a, st), "up backward");
         back(s, D3B, s.gl3a, n, H3, W3, s.e3, 128, 0, s.gl3b, 128, 0, s.e3, st);
         back(s, D3A, s.gl3b, n, H3, W3, s.cat3, 384, 0, s.g_cat3, 384, 0, nullptr, st);
         // bottleneck
-        cuda_check(rfk_unet_up_backward(s.g_cat3, 384, 0, s.b2, n, H4, W4, 256, s.gl4a, st), "up backward");
+        cuda_check(rfk_unet_up_backward(s.g_cat3, 384, 0, s.cat3, n, H4, W4, 256, s.gl4a, st), "up backward");
         back(s, B2, s.gl4a, n, H4, W4, s.b1, 256, 0, s.gl4b, 256, 0, s.b1, st);
         back(s, B1, s.gl4b, n, H4, W4, s.p3, 128, 0, s.g_p3, 128, 0, nullptr, st);
         // encoder
@@ -267,23 +246,21 @@ struct rfk_denoiser {
         back(s, L_IN, s.gl1b, n, H, W, s.x, 32, 0, nullptr, 0, 0, nullptr, st);
     }
 
-    void adam(float lr, cudaStream_t st) {
-        step++;
-        for (auto& y : L)
-            cuda_check(rfk_unet_adam(y.w, y.m, y.v, y.g, y.d.cout, y.d.cin, y.d.live_out, y.d.live_in, lr, 0.9f, 0.999f,
-                                     1e-8f, step, y.wf, y.wb, y.b, y.bm, y.bv, y.bg, st),
-                       "adam");
+    void adam_launch(float lr, int t, cudaStream_t st) {
+        rfk_unet_layer a[NLAYERS];
+        for (int l = 0; l < NLAYERS; l++) {
+            const layer& y = L[l];
+            a[l] = {y.w, y.m, y.v, y.g, y.b, y.bm, y.bv, y.bg, y.wf, y.wb, y.d.cin, y.d.cout, y.d.live_in, y.d.live_out};
+        }
+        cuda_check(rfk_unet_adam(a, NLAYERS, lr, 0.9f, 0.999f, 1e-8f, t, st), "adam");
     }
+
+    void adam(float lr, cudaStream_t st) { adam_launch(lr, ++step, st); }
 
     // Writes the bf16 copies of the current master weights (Adam with lr 0).
     void sync_copies(cudaStream_t st) {
-        for (auto& y : L) {
-            cuda_check(cudaMemsetAsync(y.g, 0, y.nw() * sizeof(float), st), "zero");
-            cuda_check(cudaMemsetAsync(y.bg, 0, y.d.cout * sizeof(float), st), "zero");
-            cuda_check(rfk_unet_adam(y.w, y.m, y.v, y.g, y.d.cout, y.d.cin, y.d.live_out, y.d.live_in, 0.0f, 0.9f, 0.999f,
-                                     1e-8f, 1, y.wf, y.wb, y.b, y.bm, y.bv, y.bg, st),
-                       "weights");
-        }
+        cuda_check(cudaMemsetAsync(grads, 0, ngrads * sizeof(float), st), "zero");
+        adam_launch(0.0f, 1, st);
     }
 
     void check_err(cudaStream_t st) {
@@ -357,11 +334,9 @@ rfk_status rfk_denoiser_create(uint64_t seed, rfk_denoiser** out) {
             y.w = dalloc<float>(nw);
             y.m = dalloc<float>(nw);
             y.v = dalloc<float>(nw);
-            y.g = dalloc<float>(nw);
             y.b = dalloc<float>(y.d.cout);
             y.bm = dalloc<float>(y.d.cout);
             y.bv = dalloc<float>(y.d.cout);
-            y.bg = dalloc<float>(y.d.cout);
             y.wf = dalloc<bf16>(nw);
             y.wb = dalloc<bf16>(nw);
             // He initialisation over the live fan-in; the output layer (a
@@ -375,6 +350,14 @@ rfk_status rfk_denoiser_create(uint64_t seed, rfk_denoiser** out) {
             cuda_check(cudaMemcpy(y.w, w.data(), nw * sizeof(float), cudaMemcpyHostToDevice), "H2D weights");
             for (float* p : {y.m, y.v}) cuda_check(cudaMemset(p, 0, nw * sizeof(float)), "zero");
             for (float* p : {y.b, y.bm, y.bv}) cuda_check(cudaMemset(p, 0, y.d.cout * sizeof(float)), "zero");
+        }
+        for (auto& y : d->L) d->ngrads += y.nw() + y.d.cout;  // multiples of 4 floats: 16-byte aligned parts
+        d->grads = dalloc<float>(d->ngrads);
+        float* at = d->grads;
+        for (auto& y : d->L) {
+            y.g = at;
+            y.bg = at += y.nw();
+            at += y.d.cout;
         }
         d->d_err = dalloc<int>(1);
         d->d_loss = dalloc<double>(1);

@@ -17,6 +17,19 @@
                               // the signs of the gradients: other roundings move the next loss by up to 1e-4)
 #define RFK_UNET_RGBOUT 16  // conv epilogue: store the first four channels as f32 (cstride 4)
 
+#define RFK_UNET_MAX_LAYERS 24
+
+// A layer's f32 master weights [cout][9][cin] and bias with their Adam moments and
+// gradients, and its bf16 copies wf [cout][9][cin] and wb [cin][9][cout].
+struct rfk_unet_layer {
+    float *w, *m, *v;
+    const float* g;
+    float *b, *bm, *bv;
+    const float* bg;
+    void *wf, *wb;
+    int cin, cout, live_in, live_out;
+};
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -39,18 +52,15 @@ cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cstride, int 
 cudaError_t rfk_unet_wgrad3x3_bias(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w, int cout,
                                    int cin, float* dw, float* db, int* err, cudaStream_t s);
 
-
 // Network input (32 bf16 channels per pixel) of a float4 histogram rendered at `spp` and its
 // tonemapped image `base` (float4).
 cudaError_t rfk_unet_features(const float4* bins, const float4* base, size_t npx, float spp, void* out, cudaStream_t s);
 // 2x2 average pool of a channel slice into a dense [n][h/2][w/2][c] tensor.
 cudaError_t rfk_unet_avgpool(const void* in, int n_img, int h, int w, int cstride, int coff, int c, void* out,
                              cudaStream_t s);
-// Nearest 2x upsample of a dense [n][h][w][c] tensor into a channel slice.
-cudaError_t rfk_unet_upsample(const void* in, int n_img, int h, int w, int c, void* out, int cstride, int coff,
-                              cudaStream_t s);
-// Gradient through the upsample (2x2 sums of a slice of g) times (act > 0); act and out [n][h][w][c].
-cudaError_t rfk_unet_up_backward(const void* g, int gcstride, int gcoff, const void* act, int n_img, int h, int w, int c,
+// Gradient through the upsample (2x2 sums of a slice of g) times (cat > 0), the upsampled activation
+// in the same slice of the [n][2h][2w] concatenation; out [n][h][w][c].
+cudaError_t rfk_unet_up_backward(const void* g, int gcstride, int gcoff, const void* cat, int n_img, int h, int w, int c,
                                  void* out, cudaStream_t s);
 // Gradient of a skip slice feeding a concatenation and an average pool, times its ReLU derivative.
 cudaError_t rfk_unet_skip_backward(const void* gcat, int cstride, int coff, const void* gpool, const void* cat, int n_img,
@@ -59,10 +69,8 @@ cudaError_t rfk_unet_skip_backward(const void* gcat, int cstride, int coff, cons
 // bf16 gradient.
 cudaError_t rfk_unet_mse(const float4* out, const float4* base, const float4* target, size_t npx, void* grad, double* loss,
                          cudaStream_t s);
-// Adam step of one layer (f32 master weights and bias) writing the bf16 forward and input-gradient copies.
-cudaError_t rfk_unet_adam(float* w, float* m, float* v, const float* g, int cout, int cin, int live_out, int live_in,
-                          float lr, float b1, float b2, float eps, int step, void* wf, void* wb, float* bias, float* bm,
-                          float* bv, const float* bg, cudaStream_t s);
+// Adam step of all layers, writing the bf16 forward and input-gradient copies.
+cudaError_t rfk_unet_adam(const rfk_unet_layer* layers, int n, float lr, float b1, float b2, float eps, int step, cudaStream_t s);
 // base + network output to an image (RFK_HALF3 .. RFK_FLOAT4; alpha as the tonemapper's).
 cudaError_t rfk_unet_to_image(const float4* net, const float4* base, const float4* bins, size_t npx, void* out, int format,
                               cudaStream_t s);
