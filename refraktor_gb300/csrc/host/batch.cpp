@@ -151,9 +151,8 @@ struct rfk_batch {
         }
         cuda_check(cudaMemsetAsync(d_bins, 0, total_px * sizeof(float4), s), "clear histograms");
         cuda_check(cudaMemsetAsync(d_uc, 0, nu * kUnitWords * sizeof(unsigned long long), s), "clear unit counters");
-        cuda_check(rfk_launch_clear_counters(d_counters, s), "clear counters");
+        cuda_check(rfk_launch_clear_counters(d_counters, kCounterWords + 1, s), "clear counters and queue");
         n++;
-        cuda_check(cudaMemsetAsync(d_counters + kCounterWords, 0, sizeof(unsigned long long), s), "clear queue");
         {
             dev_batch_args a{};
             a.units = d_units;

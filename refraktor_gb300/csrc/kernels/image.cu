@@ -415,13 +415,10 @@ void launch_convert(const __half* in, void* out, unsigned w, unsigned h, int fli
     else convert_kernel<CIN, COUT, BYTES, false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, out, w, h, flip_y, swap);
 }
 
-__global__ void clear_counters_kernel(unsigned long long* c) {
-    c[0] = 0;
-    c[1] = 0;
-    c[2] = ~0ull;
-    c[3] = 0;
-    c[4] = 0;
-    c[5] = 0;
+// Counters of a render (rfk_counters: 0, the earliest start the largest value) and
+// `n` words in all.
+__global__ void clear_counters_kernel(unsigned long long* c, unsigned n) {
+    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) c[i] = i == 2 ? ~0ull : 0ull;
 }
 
 de_table de_make_table() {
@@ -563,8 +560,8 @@ cudaError_t rfk_launch_convert(const void* in, int in_channels, void* out, int o
     return cudaGetLastError();
 }
 
-cudaError_t rfk_launch_clear_counters(unsigned long long* c, cudaStream_t s) {
-    clear_counters_kernel<<<1, 1, 0, s>>>(c);
+cudaError_t rfk_launch_clear_counters(unsigned long long* c, unsigned n, cudaStream_t s) {
+    clear_counters_kernel<<<1, 128, 0, s>>>(c, n);
     return cudaGetLastError();
 }
 
