@@ -473,28 +473,26 @@ __device__ __forceinline__ void rfk_block_sort(float4* __restrict__ chains, cons
 }
 #endif
 
-// Batched renders of union kernels (RFK_SHARED) assign xforms by strata instead of
-// picking one per chain and sorting. A pass has one slot per chain of the block, N
-// in all: slot i runs the xform whose share of [0, 1) holds (i + u) / N, u uniform
-// and new for every pass, so the slots of one xform are one run by construction,
-// and takes the chain at place (mul * i + add) mod N, which stays at its place: mul
-// is odd, so the places of a pass are a permutation, and neither needs moving or
-// staging. As add is uniform, a chain's (i + u) / N is uniform in [0, 1) and
-// independent from pass to pass: each chain picks xforms independently with the
-// weights' chances, as in the chaos game. Only the joint law of a block's chains
-// differs: an xform's count in a pass is rounded to a whole number instead of
-// random, and as mul is random the distance of two chains' slots changes every pass.
+// Batched renders assign xforms by strata instead of picking one per chain and
+// sorting. A pass has one slot per chain of the block, N in all: slot i runs the
+// xform whose share of [0, 1) holds (i + u) / N, u uniform and new for every
+// pass, so the slots of one xform are one run by construction, and takes the
+// chain at place (mul * i + add) mod N, which stays at its place: mul is odd, so
+// the places of a pass are a permutation, and neither needs moving or staging.
+// As add is uniform, a chain's (i + u) / N is uniform in [0, 1) and independent
+// from pass to pass: each chain picks xforms independently with the weights'
+// chances, as in the chaos game. Only the joint law of a block's chains differs:
+// an xform's count in a pass is rounded to a whole number instead of random, and
+// as mul is random the distance of two chains' slots changes every pass.
 // A pass then costs a chain one load and one store of its state and a block one
 // barrier, with no matching of lanes, shared atomics, scan and scatter (64
-// aligned flames: 55.4 ms of rfk_bin_batch, 62.3 with picks and the sort).
-// The other kernels keep picks and sort: chaos rows pick by the previous xform, a
-// chain count that is no power of two has other multipliers, and flames of one
-// structure (animation frames, 36.2 ms against 44.7 for 16 at 1280 x 720) keep the
-// trajectories that their seeds have had, and with them each image's noise, which a
-// union kernel's seeds lost to its shared function.
+// aligned flames: 55.4 ms of rfk_bin_batch, 62.3 with picks and the sort; 16
+// frames of an animation at 1280 x 720: 36.2 and 44.7).
+// With chaos rows the pick depends on the previous xform, and a chain count
+// that is no power of two has other multipliers: both keep the sort.
 #define RFK_CHAINS (RFK_BLOCK * RFK_CPT)
 #define RFK_STRATA \
-    (RFK_SHARED && RFK_SORT == 2 && !RFK_CHAOS && RFK_NX <= 32 && RFK_BLOCK % 32 == 0 && (RFK_CHAINS & (RFK_CHAINS - 1)) == 0)
+    (RFK_SORT == 2 && !RFK_CHAOS && RFK_NX <= 32 && RFK_BLOCK % 32 == 0 && (RFK_CHAINS & (RFK_CHAINS - 1)) == 0)
 #if RFK_STRATA
 #define RFK_SPLIT 0x80u
 struct rfk_strata {

@@ -1,6 +1,6 @@
 """The xform picks of batched renders: every chain picks independently with the
-weights' chances, whatever the kernel and launch shape (stratified assignment in
-union kernels with a power-of-two number of chains, pick and sort in others).
+weights' chances, whatever the launch shape (stratified assignment of a
+power-of-two number of chains, pick and sort of others).
 
 Three maps x / 8 + t (t = -0.25, 0, 0.25) put a chain into a strip of the image
 that names its last two xforms. The counts are held against the products of the
@@ -28,23 +28,18 @@ def _strips(density):
     return [col[r[0]:r[-1] + 1].sum() for r in runs]
 
 
-@pytest.mark.parametrize("union", [True, False])
 @pytest.mark.parametrize("block,cpt,sort", [(256, 8, 2), (256, 1, 2), (128, 4, 2), (32, 1, 2), (96, 8, 2), (256, 8, 1), (256, 1, -1)])
 @pytest.mark.parametrize("weights", [(0.5, 0.3, 0.2), (0.9, 0.0, 0.1), (0.0, 0.35, 0.65), (0.7, 0.3, 0.0), (0.004, 0.496, 0.5),
                                      (0.0, 0.0, 0.0)])
-def test_batch_picks_follow_the_weights(db, weights, block, cpt, sort, union):
+def test_batch_picks_follow_the_weights(db, weights, block, cpt, sort):
     g = syn.plain_flame(0)
-    # a union kernel's flame: variations of weight 0 beside the linear one
-    others = ["bubble", "cylinder", "disc", "exponential", "horseshoe", "polar", "sinusoidal", "spherical", "swirl"]
-    variations = {"linear": 1.0, **({v: 0.0 for v in others} if union else {})}
     g["xforms"] = [{"weight": wt, "color": 0.5, "color_speed": 0.5, "opacity": 1.0,
                     "vchain": [{"transform": [0.125, 0, 0, 0.125, tx, 0], "mod_x": 0, "mod_y": 0, "mod_scale": 1,
-                                "mod_rotate": 0, "variations": variations}]}
+                                "mod_rotate": 0, "variations": {"linear": 1.0}}]}
                    for wt, tx in zip(weights, (-0.25, 0.0, 0.25))]
     g.pop("final_xform", None)
     g.update(center_x=0.0, center_y=0.0, rotate=0.0, scale=16.0)  # about 1000 pixels a unit
     f = lr.flame.from_json(db, g)
-    assert ("#define RFK_SHARED 1" in lr.generate_source(db, f)) == union
     k = lr.flame_compiler().get_flame_kernel(db, f, block=block, chains_per_thread=cpt, sort=sort, flush=4)
     b = lr.batch(k, [lr.batch_unit(W, H, SPP, segment=0, t=0.0)], 4, out_format=-1, seed=7)
     b.set_samples(f.pack_samples(4, W, H))
