@@ -305,8 +305,6 @@ generated_flame generate_flame_code(const flamedb& db, const flame& f) {
         s << "    return rfk_xf_" << g.num_xforms << "(pt, col, P, rng);\n}\n\n";
     }
     s << "RFK_FN void rfk_precalc(PT* P, Rng& rng) {\n    (void)P; (void)rng;\n" << em.precalc.str() << "}\n";
-    // whether a variation draws random bits: else no lane needs any at hand
-    s << "#define RFK_USES_BITS " << (s.str().find("RNG_BIT()") != std::string::npos ? 1 : 0) << "\n";
     g.source = s.str();
     return g;
 }

@@ -9,7 +9,6 @@
 //   all of them with RFK_SX_STRIDE, RFK_SX_VARS, rfk_sx_src[], rfk_sx_weight[]
 //   R rfk_final(V2& p, R& c, const float* P, Rng& rng)              (if RFK_HAS_FINAL)
 //   void rfk_precalc(float* P, Rng& rng)                             (variation precalc)
-//   RFK_USES_BITS (1: a variation draws random bits)
 // and the launch shape: RFK_BLOCK (threads per block), RFK_CPT (chains per
 // thread), RFK_FLUSH (0 = one red.global.add.v4.f32 per draw, 1 = warp-
 // aggregated red for lanes that hit the same pixel, 2 = warp-aggregated into a
@@ -308,10 +307,10 @@ __device__ __forceinline__ int rfk_pick(float u, const float* __restrict__ P, un
 }
 
 // Moves one chain through xform k: apply, bad-value reset, final xform on a
-// copy, screen projection (`origin`: the affine's c and f, with the jitter).
-// Returns the draw (pixel index or -1) and its RGBA contribution.
+// copy, screen projection. Returns the draw (pixel index or -1) and its RGBA
+// contribution.
 __device__ __forceinline__ int rfk_move(int k, float& x, float& y, float& c, Rng& rng, const float* __restrict__ P,
-                                        float2 origin, unsigned w, unsigned h, float4& contrib, unsigned& hit) {
+                                        unsigned w, unsigned h, float4& contrib, unsigned& hit) {
     V2 p = fl_vec2(x, y);
     R col = c;
     R op = rfk_apply_xform(k, p, col, P, rng);
@@ -326,9 +325,9 @@ __device__ __forceinline__ int rfk_move(int k, float& x, float& y, float& c, Rng
 #if RFK_HAS_FINAL
     rfk_final(p, col, P, rng);
 #endif
-    // screen-space affine: a, d, b, e at P[0..3], and `origin`
-    float sx = fmaf(P[0], p.x, fmaf(P[2], p.y, origin.x));
-    float sy = fmaf(P[1], p.x, fmaf(P[3], p.y, origin.y));
+    // screen-space affine (a,d,b,e,c,f at P[0..5])
+    float sx = fmaf(P[0], p.x, fmaf(P[2], p.y, P[4]));
+    float sy = fmaf(P[1], p.x, fmaf(P[3], p.y, P[5]));
     sx = truncf(sx);
     sy = truncf(sy);
     hit = 0;
@@ -360,7 +359,7 @@ __device__ __forceinline__ int rfk_step(float& x, float& y, float& c, unsigned& 
 #if RFK_CHAOS
     last = (unsigned)k;
 #endif
-    return rfk_move(k, x, y, c, rng, P, make_float2(P[4], P[5]), w, h, contrib, hit);
+    return rfk_move(k, x, y, c, rng, P, w, h, contrib, hit);
 }
 
 #if RFK_SORT
@@ -470,93 +469,6 @@ __device__ __forceinline__ void rfk_block_sort(float4* __restrict__ chains, cons
         chains[pos] = make_float4(v[q].x, v[q].y, v[q].z, __int_as_float((int)kbq));
     }
     __syncthreads();
-}
-#endif
-
-// Batched renders assign xforms by strata instead of picking one per chain and
-// sorting. A pass has one slot per chain of the block, N in all: slot i runs the
-// xform whose share of [0, 1) holds (i + u) / N, u uniform and new for every
-// pass, so the slots of one xform are one run by construction, and takes the
-// chain at place (mul * i + add) mod N, which stays at its place: mul is odd, so
-// the places of a pass are a permutation, and neither needs moving or staging.
-// As add is uniform, a chain's (i + u) / N is uniform in [0, 1) and independent
-// from pass to pass: each chain picks xforms independently with the weights'
-// chances, as in the chaos game. Only the joint law of a block's chains differs:
-// an xform's count in a pass is rounded to a whole number instead of random, and
-// as mul is random the distance of two chains' slots changes every pass.
-// A pass then costs a chain one load and one store of its state and a block one
-// barrier, with no matching of lanes, shared atomics, scan and scatter (64
-// aligned flames: 55.4 ms of rfk_bin_batch, 62.3 with picks and the sort; 16
-// frames of an animation at 1280 x 720: 36.2 and 44.7).
-// With chaos rows the pick depends on the previous xform, and a chain count
-// that is no power of two has other multipliers: both keep the sort.
-#define RFK_CHAINS (RFK_BLOCK * RFK_CPT)
-#define RFK_STRATA \
-    (RFK_SORT == 2 && !RFK_CHAOS && RFK_NX <= 32 && RFK_BLOCK % 32 == 0 && (RFK_CHAINS & (RFK_CHAINS - 1)) == 0)
-#if RFK_STRATA
-#define RFK_SPLIT 0x80u
-struct rfk_strata {
-    float cum[RFK_NX];                        // chance of an xform before k
-    unsigned start[2][RFK_NX + 1];            // first slot of xform k's run, by pass parity; [RFK_NX]: all slots
-    unsigned mul[2], add[2];                  // the permutation
-    float2 origin[32];                        // of the screen affine, with a jitter of each lane's own
-    unsigned char first[2][RFK_CHAINS / 32];  // xform of the first of each 32 slots; RFK_SPLIT: not that of all
-};
-
-// One warp: the xforms' chances, as rfk_pick draws them from the alias table.
-// A chance of 0 leaves `cum` unchanged bit for bit, and its run empty.
-__device__ __forceinline__ void rfk_strata_chances(rfk_strata& st, const float* __restrict__ P) {
-    const unsigned lane = threadIdx.x & 31u;
-    float p = 0.0f;
-    for (unsigned e = 0; e < RFK_NX; e++) {
-        const float keep = fminf(fmaxf(P[RFK_OFF_ALIAS + 2 * e], 0.0f), 1.0f);
-        if (e == lane) p += keep;
-        if ((unsigned)__float_as_int(P[RFK_OFF_ALIAS + 2 * e + 1]) == lane) p += 1.0f - keep;
-    }
-    float before = 0.0f, sum = 0.0f;
-    for (unsigned e = 0; e < RFK_NX; e++) {
-        const float pe = __shfl_sync(0xffffffffu, p, (int)e);
-        if (e < lane) before += pe;
-        sum += pe;
-    }
-    if (lane < RFK_NX) st.cum[lane] = before == sum ? 1.0f : before / sum;
-    __syncwarp();
-}
-
-// One warp: runs and permutation of pass `pass`.
-__device__ __forceinline__ void rfk_strata_pass(rfk_strata& st, unsigned call_id, unsigned long long pass,
-                                                unsigned seed, unsigned salt) {
-    const unsigned lane = threadIdx.x & 31u, set = (unsigned)pass & 1u;
-    Rng r;
-    r.start(blockIdx.x, call_id, pass, seed, salt ^ 0x85EBCA6Bu);
-    const unsigned mul = (r.next() >> 8) | 1u, add = r.next() >> 8;
-    const float u = rfk_u01f(r.next());
-    if (lane < RFK_NX) {
-        const float c = st.cum[lane];
-        const int at = (int)ceilf(fmaf(c, (float)RFK_CHAINS, -u));
-        st.start[set][lane] = c >= 1.0f ? RFK_CHAINS : (unsigned)min(max(at, 0), RFK_CHAINS);
-    }
-    if (lane == 0) {
-        st.start[set][RFK_NX] = RFK_CHAINS;
-        st.mul[set] = mul;
-        st.add[set] = add;
-    }
-    __syncwarp();
-    for (unsigned g = lane; g < RFK_CHAINS / 32; g += 32) {
-        unsigned k = 0;
-        for (unsigned e = 1; e < RFK_NX; e++) k += st.start[set][e] <= 32u * g ? 1u : 0u;
-        st.first[set][g] = (unsigned char)(k | (st.start[set][k + 1] < 32u * g + 32u ? RFK_SPLIT : 0u));
-    }
-}
-
-// Xform of slot i. Runs only end before slot i or at RFK_CHAINS > i.
-__device__ __forceinline__ int rfk_strata_xform(const rfk_strata& st, unsigned set, unsigned i) {
-    unsigned k = st.first[set][i / 32];
-    if (k & RFK_SPLIT) {
-        k &= RFK_SPLIT - 1u;
-        while (i >= st.start[set][k + 1]) k++;
-    }
-    return (int)k;
 }
 #endif
 
@@ -856,12 +768,7 @@ struct rfk_pass_smem {
 #if RFK_SORT == 1
     unsigned counts[RFK_BLOCK / 32][32];
 #elif RFK_SORT == 2
-    union {
-        unsigned counts[2][RFK_NX * (RFK_BLOCK / 32)];  // ping-pong sets, one per pass parity
-#if RFK_STRATA
-        rfk_strata strata;  // rfk_bin_batch
-#endif
-    };
+    unsigned counts[2][RFK_NX * (RFK_BLOCK / 32)];  // ping-pong sets, one per pass parity
 #endif
 #if RFK_FLUSH == 2 || RFK_FLUSH == 3
     rfk_cache cache;
@@ -1019,7 +926,7 @@ __device__ __forceinline__ void rfk_move_slot(int q, unsigned chain, rfk_pass_sm
     rng.start_lazy(chain, call_id, pass, seed, salt);
     rng.give_bits(last >> 8);
     last &= 0xFFu;
-    idx = rfk_move((int)last, x, y, c, rng, P, make_float2(P[4], P[5]), w, h, v, hit);
+    idx = rfk_move((int)last, x, y, c, rng, P, w, h, v, hit);
 #else
     rng.start(chain, call_id, pass, seed, salt);
     idx = rfk_step(x, y, c, last, rng, P, w, h, v, hit);
@@ -1031,56 +938,6 @@ __device__ __forceinline__ void rfk_move_slot(int q, unsigned chain, rfk_pass_sm
         my_draws += (idx >= 0) ? 1u : 0u;
     }
 }
-
-#if RFK_STRATA
-// The pass of rfk_bin_batch: this thread's slots, without a barrier at either
-// end. One warp of the block, in turn, prepares the next pass's runs, in the set
-// that this pass does not read. A variation's random bits come from a lane's
-// stream, 8 a chain, as those that the sorted passes have left of their picks.
-__device__ __forceinline__ void rfk_strata_moves(rfk_pass_smem& sm, const float* P, float4* bins, unsigned w, unsigned h,
-                                                 unsigned chain0, unsigned cstride, unsigned lane_stream, unsigned call_id,
-                                                 unsigned long long pass, unsigned seed, unsigned salt, bool draw,
-                                                 unsigned age, unsigned& my_hits, unsigned& my_draws) {
-    (void)age;
-    (void)lane_stream;
-    const unsigned set = (unsigned)pass & 1u;
-    if (threadIdx.x / 32 == (unsigned)pass % (RFK_BLOCK / 32)) rfk_strata_pass(sm.strata, call_id, pass + 1, seed, salt);
-    const unsigned step = RFK_BLOCK * sm.strata.mul[set];
-    unsigned place = threadIdx.x * sm.strata.mul[set] + sm.strata.add[set];
-    const float2 origin = sm.strata.origin[threadIdx.x % 32];
-#if RFK_USES_BITS
-    Rng br;
-    br.start(lane_stream, call_id, pass, seed, salt ^ 0x9E3779B9u);
-    unsigned bits = br.next(), more = br.next();
-    static_assert(RFK_CPT <= 8, "64 bits a lane and pass");
-#endif
-#pragma unroll 1
-    for (int q = 0; q < RFK_CPT; q++, place += step) {
-        float4* at = &sm.chains[place & (RFK_CHAINS - 1)];
-        const float4 s = *at;
-        float x = s.x, y = s.y, c = s.z;
-        float4 v;
-        unsigned hit;
-        Rng rng;
-        rng.start_lazy(chain0 + (unsigned)q * cstride, call_id, pass, seed, salt);
-#if RFK_USES_BITS
-        rng.give_bits(bits);
-        bits = __funnelshift_r(bits, more, 8);
-        more >>= 8;
-#endif
-        const int k = rfk_strata_xform(sm.strata, set, (unsigned)q * RFK_BLOCK + threadIdx.x);
-        const int idx = rfk_move(k, x, y, c, rng, P, origin, w, h, v, hit);
-        *at = make_float4(x, y, c, 0.0f);
-        if (draw) {
-            const bool disc = RFK_DISC(age, q);
-            (void)disc;
-            rfk_flush(bins, idx, v RFK_CACHE_ARG);
-            my_hits += hit;
-            my_draws += (idx >= 0) ? 1u : 0u;
-        }
-    }
-}
-#endif
 
 // Block totals of the check interval: warp sums, then shared atomics. Ends
 // with a barrier after which s_hits / s_draws hold the block's sums and the
@@ -1395,28 +1252,16 @@ struct rfk_batch_args {
 // Antialiasing jitter ~ gauss(1/3 px) of the screen affine (as each temporal
 // sample of the single-flame path has one), drawn afresh at the start of an
 // item and at every quality check, so that a small unit worked on by few
-// blocks still averages over many jitters; one for each lane of the warps (a
-// 96 x 64 unit at 160 spp differs less between two seeds, and a move reads no
-// screen offset: 53.7 ms of rfk_bin_batch for 64 aligned flames, 54.1 with one
-// jitter), or with picks and the sort one for the block. The first warp's threads call it. Philox
-// stream (item, lane, call_id : block pass) of a key of its own, unique per draw.
-__device__ __forceinline__ void rfk_batch_jitter(rfk_pass_smem& sm, float* P, const float* __restrict__ base,
-                                                 unsigned long long item, unsigned call_id, unsigned long long pass,
-                                                 unsigned seed, unsigned salt) {
-#if !RFK_STRATA
-    if (threadIdx.x != 0) return;
-#endif
+// blocks still averages over many jitters. Philox stream (item, 0xFFFF,
+// call_id : block pass), unique per draw.
+__device__ __forceinline__ void rfk_batch_jitter(float* P, const float* __restrict__ base, unsigned long long item,
+                                                 unsigned call_id, unsigned long long pass, unsigned seed,
+                                                 unsigned salt) {
     Rng jr;
-    jr.start((unsigned)item, threadIdx.x, ((unsigned long long)call_id << 32) | (unsigned)pass, seed, salt ^ 0xC2B2AE35u);
+    jr.start((unsigned)item, 0xFFFFu, ((unsigned long long)call_id << 32) | (unsigned)pass, seed, salt);
     const V2 j = jr.gauss(1.0f / 3.0f);
-#if RFK_STRATA
-    (void)P;
-    sm.strata.origin[threadIdx.x] = make_float2(base[4] + j.x, base[5] + j.y);
-#else
-    (void)sm;
     P[4] = base[4] + j.x;
     P[5] = base[5] + j.y;
-#endif
 }
 
 extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
@@ -1478,13 +1323,7 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
         const rfk_unit U = a.units[u];
         rfk_load_params(P, U.params, RFK_BLOCK);
         __syncthreads();
-#if RFK_STRATA
-        if (threadIdx.x < 32) {
-            rfk_strata_chances(sm.strata, P);
-            rfk_strata_pass(sm.strata, call_id, pass, a.seed, a.salt);
-        }
-#endif
-        if (threadIdx.x < 32) rfk_batch_jitter(sm, P, U.params, item, call_id, pass, a.seed, a.salt);
+        if (threadIdx.x == 0) rfk_batch_jitter(P, U.params, item, call_id, pass, a.seed, a.salt);
         __syncthreads();
         unsigned warm = 0;
         if (u != cur) {
@@ -1521,17 +1360,11 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
 #pragma unroll 1
             for (unsigned it = 0; it < n; it++) {
                 const bool draw = done + it >= warm;
-#if RFK_STRATA
-                rfk_strata_moves(sm, P, U.bins, U.w, U.h, chain0, cstride, lane_stream, call_id, pass, a.seed, a.salt,
-                                 draw, age, my_hits, my_draws);
-                __syncthreads();
-#else
                 rfk_pick_sort(sm, P, lane_stream, call_id, pass, a.seed, a.salt);
 #pragma unroll 1
                 for (int q = 0; q < RFK_CPT; q++)
                     rfk_move_slot(q, chain0 + (unsigned)q * cstride, sm, P, U.bins, U.w, U.h, call_id, pass, a.seed,
                                   a.salt, draw, RFK_DISC(age, q), my_hits, my_draws);
-#endif
                 pass++;
 #if RFK_FLUSH == 4
                 if (draw) {
@@ -1555,10 +1388,10 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
                     if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
                 }
                 s_bail = bail;
+                // a new jitter for the next interval: the other threads wait at
+                // the barrier below and read P only after it
+                if (!bail && done < total) rfk_batch_jitter(P, U.params, item, call_id, pass, a.seed, a.salt);
             }
-            // a new jitter for the next interval: the other warps wait at the
-            // barrier below and read it only after that
-            if (threadIdx.x < 32 && done < total) rfk_batch_jitter(sm, P, U.params, item, call_id, pass, a.seed, a.salt);
             __syncthreads();
             ended = s_bail;
             if (ended) break;
