@@ -142,8 +142,8 @@ struct emitter {
             }
         }
         // and values with the same readers share a branch (64 aligned flames:
-        // 54.1 ms of rfk_bin_batch, 55.4 with a branch each; a loop over the live
-        // bits with a switch instead of a test for each variation: 62.4)
+        // 63.6 ms of rfk_bin_batch, 63.8 with a branch each; a loop over the live
+        // bits with a switch instead of a test for each variation is 13% slower)
         unsigned open = 0;  // readers of the values in the branch being written
         std::ostringstream decl, eval;
         for (auto& cn : db.common_closure(direct)) {
