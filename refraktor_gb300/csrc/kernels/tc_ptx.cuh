@@ -213,6 +213,17 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&a)[32], uint32_t (&b)[32
     for (int i = 0; i < 32; i++) asm volatile("" : "+r"(a[i]), "+r"(b[i]), "+r"(c[i]));
 }
 
+// Clears 32 consecutive columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
+    __syncwarp();
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+        "%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+        "r"(0u)
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // 16 consecutive f32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
