@@ -165,10 +165,10 @@ struct rfk_denoiser {
     }
 
     void conv(int l, const bf16* in, int h, int w, int n, int in_cstride, int in_coff, void* out, int out_cstride,
-              int out_coff, int flags, cudaStream_t st) {
+              int out_coff, int flags, cudaStream_t st, void* pool = nullptr) {
         const layer& y = L[l];
-        cuda_check(rfk_unet_conv3x3(in, n, h, w, in_cstride, in_coff, y.d.cin, y.wf, y.d.cout, y.b, flags, out, out_cstride,
-                                    out_coff, nullptr, 0, 0, 0, d_err, st),
+        cuda_check(rfk_unet_conv3x3_pool(in, n, h, w, in_cstride, in_coff, y.d.cin, y.wf, y.d.cout, y.b, flags, out, out_cstride,
+                                         out_coff, nullptr, 0, 0, 0, pool, d_err, st),
                    "conv");
     }
 
@@ -181,8 +181,7 @@ struct rfk_denoiser {
         const int H2 = H / 2, W2 = W / 2, H3 = H / 4, W3 = W / 4, H4 = H / 8, W4 = W / 8;
         const int A = infer ? RFK_UNET_ANY_ORDER : 0, R = RFK_UNET_RELU | A;
         conv(L_IN, s.x, H, W, n, 32, 0, s.a1, 32, 0, R, st);
-        conv(E1B, s.a1, H, W, n, 32, 0, s.cat1, 96, 64, R, st);
-        cuda_check(rfk_unet_avgpool(s.cat1, n, H, W, 96, 64, 32, s.p1, st), "pool");
+        conv(E1B, s.a1, H, W, n, 32, 0, s.cat1, 96, 64, RFK_UNET_RELU, st, s.p1);  // and its pool
         conv(E2A, s.p1, H2, W2, n, 32, 0, s.a2, 64, 0, R, st);
         conv(E2B, s.a2, H2, W2, n, 64, 0, s.cat2, 192, 128, R, st);
         cuda_check(rfk_unet_avgpool(s.cat2, n, H2, W2, 192, 128, 64, s.p2, st), "pool");

@@ -43,6 +43,13 @@ cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w, int in_cst
                              int out_coff, const void* mask, int mask_cstride, int mask_coff, int accumulate, int* err,
                              cudaStream_t s);
 
+// The same, and the 2x2 average pool of the output as a dense [n][h/2][w/2][cout] tensor (pool may be
+// null): for 32 dense input channels in the fixed order, bf16 outputs and even h and w.
+cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, int w, int in_cstride, int in_coff, int cin,
+                                  const void* weights, int cout, const float* bias, int flags, void* out, int out_cstride,
+                                  int out_coff, const void* mask, int mask_cstride, int mask_coff, int accumulate, void* pool,
+                                  int* err, cudaStream_t s);
+
 // dW[cout][9][cin] (f32) += sum over pixels of dY[p][n] * X[p + tap][c], on tcgen05. dy: dY as
 // dense NHWC bf16 (cout channels); x: X as NHWC bf16, channels x_coff .. x_coff + cin of
 // x_cstride. w must be a multiple of 64, cin and cout of 32.

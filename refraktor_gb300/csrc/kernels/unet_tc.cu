@@ -56,7 +56,8 @@ struct conv_args {
     int mask_cstride, mask_coff;
     int accumulate;
     int tma_out;  // bf16 output through shared memory and TMA stores
-    int band;     // conv3x3_rows: output rows per task
+    int band;     // conv3x3_rows, conv3x3_walk: output rows per task
+    bf16* pool;   // conv3x3_walk: the output's 2x2 average pool too, dense (null: not wanted)
     int* err;
 };
 
@@ -905,6 +906,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
         const uint32_t lane_acc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(k * 256);
         int in = 0, out = 0;  // input rows of earlier tasks, output rows so far
         bool ok = true;
+        float above[32];      // the pair's sum in an even row, for the pool
         for (int t = first + k * step; ok && t < ntasks; t += 2 * step) {
             const int xt = t % p.tiles_x, y0 = ((t / p.tiles_x) % bands) * p.band, img = t / (p.tiles_x * bands);
             const int rows = min(p.band, p.h - y0);
@@ -918,7 +920,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
                     break;
                 }
                 tc::fence_after();
-                float v[2][32];
+                float v[2][32];  // the pair's pixels
                 const uint32_t acc = lane_acc + (uint32_t)(out % C::SLOTS) * 64u;
 #pragma unroll
                 for (int a = 0; a < 2; a++) tc::tmem_ld32(acc + a * 32u, v[a]);
@@ -941,6 +943,22 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
                         stage_bf16<64, 32>(tile, pair, a * 32, v[a]);
                     } else {
                         stage_bf16<32, 32>(tile + a * (C::OUT_TILE / 2), pair, 0, v[a]);
+                    }
+                }
+                if (p.pool) {
+                    // as avgpool_kernel adds the stored values (bands start at even rows);
+                    // 1080p: 87 us, 62 and 43 in two passes
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const float2 l = __bfloat1622float2(__floats2bfloat162_rn(v[0][j], v[0][j + 1]));
+                        const float2 r = __bfloat1622float2(__floats2bfloat162_rn(v[1][j], v[1][j + 1]));
+                        above[j] = q & 1 ? 0.25f * ((above[j] + l.x) + r.x) : l.x + r.x;
+                        above[j + 1] = q & 1 ? 0.25f * ((above[j + 1] + l.y) + r.y) : l.y + r.y;
+                    }
+                    if ((q & 1) && valid) {
+                        bf16* dst = p.pool + (((size_t)img * (p.h / 2) + y / 2) * (p.w / 2) + x / 2) * p.cout + n0;
+#pragma unroll
+                        for (int g = 0; g < 32; g += 16) store_bf16x16(dst + g, reinterpret_cast<float(&)[16]>(above[g]));
                     }
                 }
                 if (p.tma_out) {
@@ -1488,7 +1506,8 @@ cudaError_t launch_walk(const void* in, const void* weights, conv_args p, cudaSt
     if (strips * p.h > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     long long best = -1;
     for (long long nb = 1; nb <= 16 * ctas / strips + 8 && nb <= (p.h + 1) / 2; nb++) {
-        const int band = (int)((p.h + nb - 1) / nb);
+        int band = (int)((p.h + nb - 1) / nb);
+        if (p.pool) band = (band + 1) / 2 * 2;
         if (p.h % band == 1 || band < 2) continue;
         const long long tasks = strips * ((p.h + band - 1) / band), cost = (tasks + 2 * ctas - 1) / (2 * ctas) * (band + 2);
         if (best < 0 || cost < best) {
@@ -1572,6 +1591,14 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
                                         const void* weights, int cout, const float* bias, int flags, void* out,
                                         int out_cstride, int out_coff, const void* mask, int mask_cstride, int mask_coff,
                                         int accumulate, int* err, cudaStream_t s) {
+    return rfk_unet_conv3x3_pool(in, n_img, h, w, in_cstride, in_coff, cin, weights, cout, bias, flags, out, out_cstride, out_coff,
+                                 mask, mask_cstride, mask_coff, accumulate, nullptr, err, s);
+}
+
+extern "C" cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, int w, int in_cstride, int in_coff, int cin,
+                                             const void* weights, int cout, const float* bias, int flags, void* out,
+                                             int out_cstride, int out_coff, const void* mask, int mask_cstride, int mask_coff,
+                                             int accumulate, void* pool, int* err, cudaStream_t s) {
     const bool rgb = (flags & RFK_UNET_RGBOUT) != 0;
     if (cin % 32 || in_coff % 32 || in_cstride % 32 || cout % 32) return cudaErrorInvalidValue;
     if (rgb ? accumulate || out_coff || out_cstride != 4 : out_coff % 32 || out_cstride % 32 || out_coff + cout > out_cstride)
@@ -1599,6 +1626,7 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
     // would be of 32 output channels (any order: no faster than conv3x3_rows, 62 us
     // both for a 1080p image; 32 f32 channels out: 259 us against 250)
     const bool walk = !any && !up2 && !accumulate && !(flags & RFK_UNET_F32OUT) && cin == 32 && in_cstride == 32 && w % 2 == 0 && h >= 2 && pick_bn(cout) == 32;
+    if (pool && (!walk || h % 2)) return cudaErrorInvalidValue;
     const int bn = rows ? 32 : pick_bn(cout);
     // tap reuse: 32 output channels (4 rows per tile) load each input channel
     // block once for all nine taps (MODE 2, 32-channel K blocks so that three
@@ -1648,6 +1676,7 @@ extern "C" cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w,
     p.accumulate = accumulate;
     p.err = err;
     p.tma_out = !p.out_f32 && !accumulate;
+    p.pool = static_cast<bf16*>(pool);
     if (walk) return launch_walk(in, weights, p, s);
     CUtensorMap mo{};
     if (p.tma_out) {

@@ -52,3 +52,30 @@ def test_pairs_are_single_pixels_bit_for_bit(n, h, w, cout, out):
     if out == "slice":
         rows = results[0][:n * h * w * cs].view(-1, cs)
         assert bool((rows[:, :32] == 7.0).all()) and bool((rows[:, 32 + cout:] == 7.0).all())
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 2, 2), (1, 8, 8), (2, 68, 300), (5, 248, 512), (12, 300, 514)])
+def test_pool_in_the_epilogue_is_the_pool_of_the_output(n, h, w):
+    L = _lib.lib()
+    L.rfk_unet_conv3x3_pool.restype = L.rfk_unet_avgpool.restype = C.c_int
+    L.rfk_unet_conv3x3_pool.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_int,
+                                        C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_int,
+                                        C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]
+    L.rfk_unet_avgpool.argtypes = [C.c_void_p] + [C.c_int] * 6 + [C.c_void_p] * 2
+    g = torch.Generator(device="cuda").manual_seed(n + 7 * h + w)
+    x = torch.randn(n, h, w, 32, device="cuda", generator=g).to(torch.bfloat16)
+    wt = (torch.randn(32, 9, 32, device="cuda", generator=g) / np.sqrt(288)).to(torch.bfloat16)
+    b = torch.randn(32, device="cuda", generator=g)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    y = torch.zeros(n, h, w, 96, device="cuda", dtype=torch.bfloat16)
+    px = n * h * w // 4 * 32
+    pools = [torch.full((px + 256,), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    assert L.rfk_unet_conv3x3_pool(x.data_ptr(), n, h, w, 32, 0, 32, wt.data_ptr(), 32, b.data_ptr(), 1, y.data_ptr(), 96, 64,
+                                   None, 0, 0, 0, pools[0].data_ptr(), err.data_ptr(), None) == 0
+    assert L.rfk_unet_avgpool(y.data_ptr(), n, h, w, 96, 64, 32, pools[1].data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    assert torch.equal(pools[0].view(torch.int16), pools[1].view(torch.int16))
+    # refused: odd heights, other layouts
+    assert L.rfk_unet_conv3x3_pool(y.data_ptr(), n, h, w, 96, 0, 32, wt.data_ptr(), 32, b.data_ptr(), 1, x.data_ptr(), 32, 0, None, 0,
+                                   0, 0, pools[0].data_ptr(), err.data_ptr(), None) != 0
