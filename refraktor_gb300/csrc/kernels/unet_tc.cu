@@ -714,10 +714,10 @@ __global__ void __launch_bounds__(320, 1) conv3x3_rows(const __grid_constant__ C
 // conv3x3_walk: 32 dense input channels, tiles of 32 output channels.
 struct walk_cfg {
     static constexpr uint32_t A_ROW = 136u * 128u;  // 136 pixel pairs of an input row, from x0 - 2 on
-    static constexpr uint32_t B_TILE = 32u * 64u, B_GROUP = 6u * B_TILE, RES = 4u * B_GROUP;
-    static constexpr int SLOTS = 4;                 // accumulators of 128 x 64 per strip
+    static constexpr uint32_t B_TILE = 32u * 64u, RES = 9u * B_TILE;
+    static constexpr int SLOTS = 4;                 // accumulators of 128 x 32 per strip and pixel of a pair
     static constexpr int DONE = 16;                 // barriers of a strip's input rows
-    static constexpr int STAGES = 6;
+    static constexpr int STAGES = 7;
     static constexpr uint32_t OUT_TILE = 128u * 64u * 2u;  // two per strip
     static constexpr uint32_t SMEM = RES + STAGES * A_ROW + 4u * OUT_TILE + 1024u;
 };
@@ -725,22 +725,22 @@ struct walk_cfg {
 // Row-streaming convolution of 32 input channels whose sums keep the order of
 // conv3x3_tc's, tap after tap. A 32-channel layer moves 64 bytes per pixel each way,
 // and TMA boxes of 64-byte rows get half the memory rate of 128-byte ones, so the
-// tensors are taken as images of w / 2 pixel pairs with 64 channels: M is 128
-// pairs, N the two pixels of an output pair, and K runs over the four pixels that
-// their column taps read, left to right (the right one of the pair before, both of
-// the pair, the left one of the pair after), with weights of 0 where a pixel is no
-// neighbour of the other. That is 24 products per 18 that count, and an output still
-// adds its taps in their order.
-// The three tap rows lie in N too, but they meet in one accumulator per output row:
-// input row i is tap row 2 of output row i - 2, tap row 1 of i - 1 and tap row 0 of
-// i, whose accumulators are neighbours in a ring of four (192 columns; 64 or 128
-// at a band's ends, in two parts at the ring's). MMAs of different input rows overlap
-// in accumulators but not in their base, which no rule orders: the next row of a
-// strip is issued when the one before is done. Two strips in turn, each with an
-// accumulator ring and an epilogue group of its own, hide that wait. The epilogue
-// clears an accumulator that it has read.
-// 16 images of 512 x 512, 32 -> 32 channels: 107 us, conv3x3_tc 138; with a mask 165
-// and 289; 32 -> 96: 304 and 423.
+// tensors are taken as images of w / 2 pixel pairs with 64 channels: M is 128 pairs,
+// the left and the right pixels have accumulators of their own, and a column tap
+// reads the half line (the right one of the pair before, both of the pair, the left
+// one of the pair after) that holds its pixel. (One accumulator for both pixels and
+// weights of 0 for the pixels that a tap row does not reach make 8 MMAs of N 192 of
+// the 12 of N 96, 109 us instead of 130, but 0 times an infinity is not 0.)
+// As in conv3x3_rows the three tap rows lie in N, but they meet in one accumulator
+// per output row: input row i is tap row 2 of output row i - 2, tap row 1 of i - 1
+// and tap row 0 of i, whose accumulators are neighbours in a ring of four (96
+// columns; 32 or 64 at a band's ends, in two parts at the ring's). MMAs of different
+// input rows overlap in accumulators but not in their base, which no rule orders: the
+// next row of a strip is issued when the one before is done. Two strips in turn, each
+// with accumulator rings and an epilogue group of its own, hide that wait in part.
+// The epilogue clears an accumulator that it has read.
+// 16 images of 512 x 512, 32 -> 32 channels: 130 us, conv3x3_tc 138; with a mask 179
+// and 289; 32 -> 96: 369 and 423.
 __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                                                        const __grid_constant__ CUtensorMap tmO, conv_args p) {
     using C = walk_cfg;
@@ -800,15 +800,9 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
     if (warp == 8) {
         if (lane == 0) {
             tc::mbar_expect_tx(&wbar, C::RES);
-            // pixel u of the four, tap rows stacked as [dy 2 | dy 1 | dy 0], each for the
-            // left and the right output pixel; past the weights' end: zeros
-            for (int u = 0; u < 4; u++)
-                for (int dy = 0; dy < 3; dy++)
-                    for (int a = 0; a < 2; a++) {
-                        const int dx = u - a;  // tap column of pixel u for output pixel a
-                        tc::tma_load_2d(res + (uint32_t)u * C::B_GROUP + (uint32_t)((2 - dy) * 2 + a) * C::B_TILE, &tmB, &wbar,
-                                        dx >= 0 && dx < 3 ? (dy * 3 + dx) * 32 : 9 * 32, n0);
-                    }
+            for (int dx = 0; dx < 3; dx++)
+                for (int dy = 0; dy < 3; dy++)  // stacked as [dy 2 | dy 1 | dy 0]
+                    tc::tma_load_2d(res + (uint32_t)(dx * 3 + 2 - dy) * C::B_TILE, &tmB, &wbar, (dy * 3 + dx) * 32, n0);
             int issued = 0;
             bool ok = true;
             strip st[2];
@@ -870,18 +864,20 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
                     // output rows lo .. lo + num - 1, of which `part` up to the ring's end
                     const int lo = max(q.i - 2, 0), num = min(q.i, q.rows - 1) - lo + 1;
                     const int slot = (out[k] + lo) % C::SLOTS, part = min(num, C::SLOTS - slot);
-                    const uint32_t b = b0 + (uint32_t)(lo - (q.i - 2)) * (2 * C::B_TILE >> 4);
+                    const uint32_t b = b0 + (uint32_t)(lo - (q.i - 2)) * (C::B_TILE >> 4);
                     for (int at = 0; at < num; at = at ? num : part) {
                         const int m = at ? num - part : part;
-                        const uint32_t acc = tmem + (uint32_t)(k * 256 + (at ? 0 : slot) * 64);
-                        const uint32_t idesc = tc::idesc_bf16(128, 0) | ((uint32_t)(m * 64 / 8) << 17);
+                        const uint32_t acc = tmem + (uint32_t)(k * 256 + (at ? 0 : slot) * 32);
+                        const uint32_t idesc = tc::idesc_bf16(128, 0) | ((uint32_t)(m * 32 / 8) << 17);
 #pragma unroll
-                        for (int u = 0; u < 4; u++)
+                        for (int a = 0; a < 2; a++)
 #pragma unroll
-                            for (int kk = 0; kk < 2; kk++)
-                                // pixel u: the right half of line 0, line 1, the left half of line 2
-                                tc::mma_bf16<AHI, BHI>(one, acc, a0 + (uint32_t)((64 + u * 64 + kk * 32) >> 4),
-                                                       b + (uint32_t)((u * C::B_GROUP + at * 2 * C::B_TILE + kk * 32) >> 4), idesc, 1u);
+                            for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+                                for (int kk = 0; kk < 2; kk++)
+                                    // half lines from the right one of line 0 on
+                                    tc::mma_bf16<AHI, BHI>(one, acc + a * 128u, a0 + (uint32_t)((64 + (a + dx) * 64 + kk * 32) >> 4),
+                                                           b + (uint32_t)(((at + dx * 3) * C::B_TILE + kk * 32) >> 4), idesc, 1u);
                     }
                     tc::mma_commit(one, &empty[s]);
                     tc::mma_commit(one, &done[k][in[k] % C::DONE]);
@@ -921,11 +917,11 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
                 }
                 tc::fence_after();
                 float v[2][32];  // the pair's pixels
-                const uint32_t acc = lane_acc + (uint32_t)(out % C::SLOTS) * 64u;
+                const uint32_t acc = lane_acc + (uint32_t)(out % C::SLOTS) * 32u;
 #pragma unroll
-                for (int a = 0; a < 2; a++) tc::tmem_ld32(acc + a * 32u, v[a]);
+                for (int a = 0; a < 2; a++) tc::tmem_ld32(acc + a * 128u, v[a]);
 #pragma unroll
-                for (int a = 0; a < 2; a++) tc::tmem_zero32(acc + a * 32u);
+                for (int a = 0; a < 2; a++) tc::tmem_zero32(acc + a * 128u);
                 tc::fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&slot_empty[k][out % C::SLOTS]);
@@ -947,7 +943,7 @@ __global__ void __launch_bounds__(320, 1) conv3x3_walk(const __grid_constant__ C
                 }
                 if (p.pool) {
                     // as avgpool_kernel adds the stored values (bands start at even rows);
-                    // 1080p: 87 us, 62 and 43 in two passes
+                    // 1080p: 98 us, 62 and 43 in two passes
 #pragma unroll
                     for (int j = 0; j < 32; j += 2) {
                         const float2 l = __bfloat1622float2(__floats2bfloat162_rn(v[0][j], v[0][j + 1]));
@@ -1623,8 +1619,8 @@ extern "C" cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, i
     const bool rows = any && cout <= 96 && h >= 2 && (cout != 64 || cin > 64 || up2) &&
                       (wide_k ? rows_cfg<64, 1>::stages(cin / 64) : rows_cfg<32, 1>::stages(cin / 32)) >= rows_cfg<32, 1>::MIN_STAGES;
     // 32 dense input channels in the fixed order: conv3x3_walk, if the tiles below
-    // would be of 32 output channels (any order: no faster than conv3x3_rows, 62 us
-    // both for a 1080p image; 32 f32 channels out: 259 us against 250)
+    // would be of 32 output channels (any order: no faster than conv3x3_rows, 74 us
+    // and 66 for a 1080p image; 32 f32 channels out: slower than the tiles)
     const bool walk = !any && !up2 && !accumulate && !(flags & RFK_UNET_F32OUT) && cin == 32 && in_cstride == 32 && w % 2 == 0 && h >= 2 && pick_bn(cout) == 32;
     if (pool && (!walk || h % 2)) return cudaErrorInvalidValue;
     const int bn = rows ? 32 : pick_bn(cout);
