@@ -15,7 +15,8 @@
 // tcgen05.commit; eight epilogue warps read the accumulator rows from TMEM
 // (two per lane quarter) and apply the epilogue: bias, ReLU, a
 // ReLU-derivative mask, then bf16 rows by TMA store, or f32 or accumulating
-// stores. conv3x3_rows streams image rows through narrow layers.
+// stores. conv3x3_rows streams image rows through narrow layers, conv3x3_walk
+// pixel pairs through layers of 32 input channels.
 // The input gradient of a conv is the same kernel on the output gradient with
 // the weights transposed and the taps flipped ([cin][9][cout]).
 //
