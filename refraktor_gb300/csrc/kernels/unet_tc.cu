@@ -1622,7 +1622,8 @@ extern "C" cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, i
     // 32 dense input channels in the fixed order: conv3x3_walk, if the tiles below
     // would be of 32 output channels (any order: no faster than conv3x3_rows, 74 us
     // and 66 for a 1080p image; 32 f32 channels out: slower than the tiles)
-    const bool walk = !any && !up2 && !accumulate && !(flags & RFK_UNET_F32OUT) && cin == 32 && in_cstride == 32 && w % 2 == 0 && h >= 2 && pick_bn(cout) == 32;
+    const bool walk = !any && !up2 && !accumulate && !(flags & RFK_UNET_F32OUT) && cin == 32 && in_cstride == 32 && w % 2 == 0 &&
+                      h >= 2 && pick_bn(cout) == 32;
     if (pool && (!walk || h % 2)) return cudaErrorInvalidValue;
     const int bn = rows ? 32 : pick_bn(cout);
     // tap reuse: 32 output channels (4 rows per tile) load each input channel
