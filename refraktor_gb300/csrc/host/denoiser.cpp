@@ -175,13 +175,13 @@ struct rfk_denoiser {
     // Forward pass of the whole network on ws.x; the result in ws.out. The last
     // convolution of each decoder level and of the bottleneck writes its output
     // straight into the next level's concatenation at twice the resolution (the
-    // upsampling fused into its epilogue). `infer`: sums in any order.
-    void forward(workspace& s, cudaStream_t st, bool infer = false) {
+    // upsampling fused into its epilogue).
+    void forward(workspace& s, cudaStream_t st) {
         const int n = s.n, H = s.h, W = s.w;
         const int H2 = H / 2, W2 = W / 2, H3 = H / 4, W3 = W / 4, H4 = H / 8, W4 = W / 8;
-        const int A = infer ? RFK_UNET_ANY_ORDER : 0, R = RFK_UNET_RELU | A;
+        const int R = RFK_UNET_RELU;
         conv(L_IN, s.x, H, W, n, 32, 0, s.a1, 32, 0, R, st);
-        conv(E1B, s.a1, H, W, n, 32, 0, s.cat1, 96, 64, RFK_UNET_RELU, st, s.p1);  // and its pool
+        conv(E1B, s.a1, H, W, n, 32, 0, s.cat1, 96, 64, R, st, s.p1);  // and its pool
         conv(E2A, s.p1, H2, W2, n, 32, 0, s.a2, 64, 0, R, st);
         conv(E2B, s.a2, H2, W2, n, 64, 0, s.cat2, 192, 128, R, st);
         cuda_check(rfk_unet_avgpool(s.cat2, n, H2, W2, 192, 128, 64, s.p2, st), "pool");
@@ -197,7 +197,7 @@ struct rfk_denoiser {
         conv(D2B, s.e2, H2, W2, n, 64, 0, s.cat1, 96, 0, U, st);
         conv(D1A, s.cat1, H, W, n, 96, 0, s.e1, 32, 0, R, st);
         conv(D1B, s.e1, H, W, n, 32, 0, s.d1, 32, 0, R, st);
-        conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 4, 0, RFK_UNET_RGBOUT | A, st);
+        conv(L_OUT, s.d1, H, W, n, 32, 0, s.out, 4, 0, RFK_UNET_RGBOUT, st);
     }
 
     // Gradients of layer l from dY (dense, cout channels, pre-activation) and
@@ -506,7 +506,7 @@ rfk_status rfk_denoise(rfk_denoiser* d, const float* bins, const float* base, ui
         cuda_check(rfk_unet_features(reinterpret_cast<const float4*>(bins), reinterpret_cast<const float4*>(base), P,
                                      (float)spp, s.x, st),
                    "features");
-        d->forward(s, st, true);
+        d->forward(s, st);
         cuda_check(rfk_unet_to_image(s.out, reinterpret_cast<const float4*>(base), reinterpret_cast<const float4*>(bins), P,
                                      out, format, st),
                    "to image");

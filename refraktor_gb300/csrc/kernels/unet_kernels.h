@@ -12,9 +12,6 @@
 #define RFK_UNET_F32OUT 2  // conv epilogue: store f32 instead of bf16
 #define RFK_UNET_UP2 4     // conv epilogue: store each output pixel at its 2x2 pixels of a (2h, 2w) output
                            // (nearest upsampling into the next level's concatenation; bf16, no accumulate)
-#define RFK_UNET_ANY_ORDER 8  // conv: the f32 sums may be ordered and split as is fastest (inference); without it the
-                              // order is fixed, so that training losses are reproducible (Adam's first steps follow
-                              // the signs of the gradients: other roundings move the next loss by up to 1e-4)
 #define RFK_UNET_RGBOUT 16  // conv epilogue: store the first four channels as f32 (cstride 4)
 
 #define RFK_UNET_MAX_LAYERS 24

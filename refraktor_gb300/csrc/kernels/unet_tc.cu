@@ -15,8 +15,7 @@
 // tcgen05.commit; eight epilogue warps read the accumulator rows from TMEM
 // (two per lane quarter) and apply the epilogue: bias, ReLU, a
 // ReLU-derivative mask, then bf16 rows by TMA store, or f32 or accumulating
-// stores. conv3x3_rows streams image rows through narrow layers, conv3x3_walk
-// pixel pairs through layers of 32 input channels.
+// stores. conv3x3_walk streams pixel pairs through layers of 32 input channels.
 // The input gradient of a conv is the same kernel on the output gradient with
 // the weights transposed and the taps flipped ([cin][9][cout]).
 //
@@ -57,7 +56,7 @@ struct conv_args {
     int mask_cstride, mask_coff;
     int accumulate;
     int tma_out;  // bf16 output through shared memory and TMA stores
-    int band;     // conv3x3_rows, conv3x3_walk: output rows per task
+    int band;     // conv3x3_walk: output rows per task
     bf16* pool;   // conv3x3_walk: the output's 2x2 average pool too, dense (null: not wanted)
     int* err;
 };
@@ -106,32 +105,8 @@ struct conv_cfg {
     static_assert(STAGES >= 2, "at least two stages");
 };
 
-// conv3x3_rows: input channel blocks of BK, tiles of 32 output channels whose
-// weights stay in shared memory; a pipeline stage is CPS channel blocks of an input row.
-template <int BK, int CPS>
-struct rows_cfg {
-    static constexpr uint32_t A_ROW = 136u * BK * 2u;  // pixels x0 - 1 .. x0 + 134 of an input row
-    static constexpr uint32_t STAGE_BYTES = CPS * A_ROW;
-    static constexpr uint32_t B_TILE = 32u * BK * 2u;
-    static constexpr int SLOTS = 5;                    // accumulators of 128 x 96 in TMEM
-    static constexpr int MAX_STAGES = 16, MIN_STAGES = 4;
-    static constexpr uint32_t OUT_TILE = 128u * 32u * 2u;  // two per epilogue group
-    static constexpr uint32_t BUDGET = 229376u - 4u * OUT_TILE;
-    static __host__ __device__ constexpr uint32_t res_bytes(int kpt) { return (uint32_t)kpt * 9u * B_TILE; }
-    static __host__ __device__ constexpr int stages(int kpt) {
-        if (res_bytes(kpt) >= BUDGET) return 0;
-        const int n = (int)((BUDGET - res_bytes(kpt)) / STAGE_BYTES);
-        return n > MAX_STAGES ? MAX_STAGES : n;
-    }
-    static_assert(A_ROW % 512u == 0 && B_TILE % 1024u == 0, "tiles must stay swizzle-aligned");
-};
-
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_n(uint64_t* bar, uint32_t n) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(bar)), "r"(n) : "memory");
 }
 
 __device__ __forceinline__ void store_bf16x16(bf16* dst, const float (&v)[16]) {
@@ -497,221 +472,6 @@ __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUt
     if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
 }
 
-// Row-streaming convolution for layers of 32, 64 or 96 output channels. An MMA
-// of such a layer is bound by its A tile: M 128 x K 16 takes 45 cycles at N 32
-// and 56 at N 96 (math: 16 and 48), so the three tap rows go into N: the
-// weights of a column tap lie stacked as [dy 0 | dy 1 | dy 2], 32 output
-// channels each, and the MMAs of an input row leave its three partial products
-// side by side in a TMEM slot of 96 columns. Output row q is dy 0 of input row
-// q - 1, dy 1 of row q and dy 2 of row q + 1, summed in f32 by the epilogue; five
-// slots let two input rows run ahead. A CTA walks down bands of a 128-pixel
-// column, an input row (136 pixels, one stage per channel block) being read
-// once per band and 32 output channels; the tile's weights are loaded once.
-// Two epilogue groups of four warps (one per TMEM lane quarter) take output rows
-// in turn; each output row arrives once at its three slots, the first and last
-// row of a band also for the rows that do not exist.
-template <int BK, int CPS>
-__global__ void __launch_bounds__(320, 1) conv3x3_rows(const __grid_constant__ CUtensorMap tmA,
-                                                       const __grid_constant__ CUtensorMap tmB,
-                                                       const __grid_constant__ CUtensorMap tmO, conv_args p) {
-    using C = rows_cfg<BK, CPS>;
-    extern __shared__ uint8_t smem_dyn[];
-    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full[C::MAX_STAGES], empty[C::MAX_STAGES], slot_full[C::SLOTS], slot_empty[C::SLOTS], wbar;
-    __shared__ uint32_t tmem_base;
-    __shared__ int s_fail;
-    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    const int kpt = p.cin / BK;
-    const uint32_t nst = (uint32_t)C::stages(kpt);
-    uint8_t* const res = base;
-    uint8_t* const outbuf = base + C::res_bytes(kpt);
-    uint8_t* const stages = outbuf + 4 * C::OUT_TILE;
-    // this CTA's 32 output channels, and its tasks among those of the CTAs that share them
-    const int ntn = p.cout / 32, n0 = ((int)blockIdx.x % ntn) * 32;
-    const int bands = (p.h + p.band - 1) / p.band;
-    const int ntasks = p.n_img * bands * p.tiles_x, first = (int)blockIdx.x / ntn;
-    const int step = ((int)gridDim.x - (int)blockIdx.x % ntn + ntn - 1) / ntn;
-
-    if (warp == 0) tc::tmem_alloc(&tmem_base, 512u);
-    if (threadIdx.x == 32) {
-        for (uint32_t s = 0; s < nst; s++) {
-            tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], 1);
-        }
-        for (int s = 0; s < C::SLOTS; s++) {
-            tc::mbar_init(&slot_full[s], 1);
-            tc::mbar_init(&slot_empty[s], 3 * 4);  // three output rows, four warps each
-        }
-        tc::mbar_init(&wbar, 1);
-        s_fail = 0;
-        tc::mbar_fence_init();
-    }
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
-
-    if (warp == kEpiWarps) {
-        if (lane == 0) {
-            // producer: the weights once, then a stage per (input row, channel block)
-            tc::mbar_expect_tx(&wbar, C::res_bytes(kpt));
-            for (int cb = 0; cb < kpt; cb++)
-                for (int dx = 0; dx < 3; dx++)
-                    for (int dy = 0; dy < 3; dy++)
-                        tc::tma_load_2d(res + (uint32_t)((cb * 3 + dx) * 3 + dy) * C::B_TILE, &tmB, &wbar,
-                                        (dy * 3 + dx) * p.cin + cb * BK, n0);
-            uint32_t s = 0, round = 0, issued = 0;
-            bool ok = true;
-            for (int t = first; ok && t < ntasks; t += step) {
-                const int xt = t % p.tiles_x, y0 = ((t / p.tiles_x) % bands) * p.band, img = t / (p.tiles_x * bands);
-                const int rows_in = min(p.band, p.h - y0) + 2;
-                for (int i = 0; ok && i < rows_in; i++)
-                    for (int cb = 0; cb < kpt; cb += CPS) {
-                        if (round > 0 && !tc::mbar_wait(&empty[s], (round - 1) & 1)) {
-                            ok = false;
-                            break;
-                        }
-                        tc::mbar_expect_tx(&full[s], C::STAGE_BYTES);
-#pragma unroll
-                        for (int c = 0; c < CPS; c++)
-                            tc::tma_load_4d(stages + s * C::STAGE_BYTES + (uint32_t)c * C::A_ROW, &tmA, &full[s],
-                                            p.cin_off + (cb + c) * BK, xt * 128 - 1, y0 + i - 1, img);
-                        issued++;
-                        if (++s == nst) {
-                            s = 0;
-                            round++;
-                        }
-                    }
-            }
-            if (!ok) {
-                atomicExch(&s_fail, 1);
-                // let the copies in flight land before the CTA exits (bounded)
-                for (uint32_t q = issued >= nst ? issued - nst : 0; q < issued; q++) tc::mbar_wait(&full[q % nst], (q / nst) & 1);
-            }
-            if (!tc::mbar_wait(&wbar, 0)) atomicExch(&s_fail, 1);
-        }
-    } else if (warp == kEpiWarps + 1) {
-        const uint32_t one = lane == 0;
-        {
-            constexpr uint32_t idesc = tc::idesc_bf16(128, 96), HI = tc::desc_hi(BK * 2);
-            const uint32_t b0 = tc::desc_lo(tc::smem_u32(res));
-            uint32_t s = 0, round = 0, slot = 0, use = 0;  // use: how often the slot ring has gone round
-            bool ok = tc::all_lanes(tc::mbar_wait(&wbar, 0));
-            for (int t = first; ok && t < ntasks; t += step) {
-                const int y0 = ((t / p.tiles_x) % bands) * p.band;
-                const int rows_in = min(p.band, p.h - y0) + 2;
-                for (int i = 0; ok && i < rows_in; i++) {
-                    if (use > 0 && !tc::all_lanes(tc::mbar_wait(&slot_empty[slot], (use - 1) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    tc::fence_after();
-                    const uint32_t acc = tmem + slot * 96u;
-                    for (int cb = 0; cb < kpt; cb += CPS) {
-                        if (!tc::all_lanes(tc::mbar_wait(&full[s], round & 1))) {
-                            ok = false;
-                            break;
-                        }
-                        tc::fence_after();
-                        const uint32_t a0 = tc::desc_lo(tc::smem_u32(stages + s * C::STAGE_BYTES));
-                        const uint32_t bc = b0 + (((uint32_t)cb * 9u * C::B_TILE) >> 4);
-#pragma unroll
-                        for (int c = 0; c < CPS; c++)
-#pragma unroll
-                            for (int dx = 0; dx < 3; dx++)
-#pragma unroll
-                                for (int kk = 0; kk < BK / 16; kk++)
-                                    tc::mma_bf16<HI, HI>(one, acc, a0 + (uint32_t)((c * C::A_ROW + dx * (BK * 2) + kk * 32) >> 4),
-                                                         bc + (uint32_t)(((c * 9 + dx * 3) * C::B_TILE + kk * 32) >> 4), idesc,
-                                                         (cb | c | dx | kk) != 0 ? 1u : 0u);
-                        tc::mma_commit(one, &empty[s]);
-                        if (++s == nst) {
-                            s = 0;
-                            round++;
-                        }
-                    }
-                    tc::mma_commit(one, &slot_full[slot]);  // also on failure: arrives once the issued MMAs are done
-                    if (++slot == C::SLOTS) {
-                        slot = 0;
-                        use++;
-                    }
-                }
-            }
-            if (!ok) atomicExch(&s_fail, 1);
-        }
-    } else {
-        // epilogue: the groups take the CTA's output rows in turn. A group waits
-        // for the last input row of an output row only (the others were committed
-        // before it); a parity tells neighbouring uses of a slot apart, so these
-        // waits may be SLOTS input rows apart at most: 2, or 4 across the end of a
-        // band, as every band has at least two rows.
-        const int quarter = warp & 3, group = warp >> 2;
-        const bool leader = (threadIdx.x & 127) == 0;
-        const int px = quarter * 32 + lane;
-        const uint32_t lane_acc = tmem + ((uint32_t)(quarter * 32) << 16);
-        float bias[32];
-#pragma unroll
-        for (int j = 0; j < 32; j++) bias[j] = p.bias ? __ldg(p.bias + n0 + j) : 0.0f;
-        uint32_t g0 = 0, n = 0, flip = 0;  // input rows and output rows before this band; staged rows of the group
-        bool ok = true;
-        for (int t = first; ok && t < ntasks; t += step) {
-            const int xt = t % p.tiles_x, y0 = ((t / p.tiles_x) % bands) * p.band, img = t / (p.tiles_x * bands);
-            const int rows = min(p.band, p.h - y0);
-            const int x = xt * 128 + px;
-            const bool valid = x < p.w;
-            for (int q = (int)((n ^ (uint32_t)group) & 1u); q < rows; q += 2) {
-                const uint32_t g = g0 + (uint32_t)q;
-                const uint32_t s0 = g % C::SLOTS, s1 = (g + 1) % C::SLOTS, s2 = (g + 2) % C::SLOTS;
-                ok = tc::named_barrier_all(1 + group, 128,
-                                           __all_sync(0xffffffffu, tc::mbar_wait(&slot_full[s2], ((g + 2) / C::SLOTS) & 1)));
-                if (!ok) {
-                    if (lane == 0) atomicExch(&s_fail, 1);
-                    break;
-                }
-                tc::fence_after();
-                uint32_t d0[32], d1[32], d2[32];
-                tc::tmem_ld32_start(lane_acc + s0 * 96u, d0);
-                tc::tmem_ld32_start(lane_acc + s1 * 96u + 32u, d1);
-                tc::tmem_ld32_start(lane_acc + s2 * 96u + 64u, d2);
-                tc::tmem_ld_wait(d0, d1, d2);
-                tc::fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    const uint32_t lo = q == 0 ? 1u : 0u, hi = q == rows - 1 ? 1u : 0u;
-                    mbar_arrive_n(&slot_empty[s0], 1u + 2u * lo);
-                    mbar_arrive_n(&slot_empty[s1], 1u + lo + hi);
-                    mbar_arrive_n(&slot_empty[s2], 1u + 2u * hi);
-                }
-                float v[32];
-#pragma unroll
-                for (int j = 0; j < 32; j++)
-                    v[j] = ((__uint_as_float(d0[j]) + __uint_as_float(d1[j])) + __uint_as_float(d2[j])) + bias[j];
-                const int y = y0 + q;
-                const size_t pix = ((size_t)img * p.h + y) * p.w + (valid ? x : 0);
-                conv_activate<32>(p, v, n0, pix, valid);
-                if (p.tma_out) {
-                    // two staging tiles per group: the store before last has read this one
-                    uint8_t* const tile = outbuf + (2 * group + (int)(flip++ & 1u)) * C::OUT_TILE;
-                    stage_bf16<32, 32>(tile, px, 0, v);
-                    tc::fence_async();
-                    if (leader) tc::tma_store_wait_read<0>();
-                    tc::named_barrier(1 + group, 128);
-                    if (leader) store_row(p, &tmO, tile, p.out_coff + n0, xt, img * p.h + y);
-                } else if (valid) {
-                    store_direct<32>(p, v, pix, n0);
-                }
-            }
-            g0 += (uint32_t)rows + 2u;
-            n += (uint32_t)rows;
-        }
-        if (leader) tc::tma_store_wait<0>();
-    }
-    tc::fence_before();
-    __syncthreads();
-    if (threadIdx.x == 0 && s_fail) atomicExch(p.err, 1);
-    if (warp == 0) tc::tmem_dealloc(tmem, 512u);
-}
-
 // conv3x3_walk: 32 dense input channels, tiles of 32 output channels.
 struct walk_cfg {
     static constexpr uint32_t A_ROW = 136u * 128u;  // 136 pixel pairs of an input row, from x0 - 2 on
@@ -732,9 +492,10 @@ struct walk_cfg {
 // one of the pair after) that holds its pixel. (One accumulator for both pixels and
 // weights of 0 for the pixels that a tap row does not reach make 8 MMAs of N 192 of
 // the 12 of N 96, 109 us instead of 130, but 0 times an infinity is not 0.)
-// As in conv3x3_rows the three tap rows lie in N, but they meet in one accumulator
-// per output row: input row i is tap row 2 of output row i - 2, tap row 1 of i - 1
-// and tap row 0 of i, whose accumulators are neighbours in a ring of four (96
+// An MMA is bound by its A tile (M 128 x K 16 takes 45 cycles at N 32 and 56 at N 96),
+// so the three tap rows lie in N, and they meet in one accumulator per output row:
+// input row i is tap row 2 of output row i - 2, tap row 1 of i - 1 and tap row 0 of i,
+// whose accumulators are neighbours in a ring of four (96
 // columns; 32 or 64 at a band's ends, in two parts at the ring's). MMAs of different
 // input rows overlap in accumulators but not in their base, which no rule orders: the
 // next row of a strip is issued when the one before is done. Two strips in turn, each
@@ -1178,7 +939,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUt
             const uint8_t* sa = base + (size_t)s * C::STAGE_BYTES;
             for (int y = 1; y <= C::R; y++) bias_row<CO>(sa + y * C::A_GROUP, t, acc);  // rows past the image are zero
             __syncwarp();
-            if (lane == 0) mbar_arrive_n(&empty[s], 1u);
+            if (lane == 0) mbar_arrive(&empty[s]);
         }
         __syncwarp();
         bias_add<CO>(p.db, CO, lane, acc);
@@ -1346,7 +1107,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUt
                     bias_row<64>(sa + C::A_GROUP, t, hi);
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive_n(&empty[s], 1u);
+                if (lane == 0) mbar_arrive(&empty[s]);
             }
             row += y1 - y0;
         }
@@ -1435,35 +1196,6 @@ cudaError_t launch_conv(const CUtensorMap& a, const CUtensorMap& b, const CUtens
     if (tiles > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     const int grid = (int)std::min<long long>(tiles, sm_count_cached());
     conv3x3_tc<BK, BN, MODE><<<grid, 32 * (kEpiWarps + 2), C::SMEM, s>>>(a, b, o, p);
-    return cudaGetLastError();
-}
-
-template <int BK, int CPS>
-cudaError_t launch_rows(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& o, conv_args p, cudaStream_t s) {
-    using C = rows_cfg<BK, CPS>;
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] { attr = raise_smem(conv3x3_rows<BK, CPS>, C::BUDGET + 4u * C::OUT_TILE + 1024u); });
-    if (attr != cudaSuccess) return attr;
-    const int ntn = p.cout / 32, sms = sm_count_cached(), kpt = p.cin / BK;
-    // rows per band: the least rows of the busiest CTA, each band's two halo rows
-    // included; no band of one row
-    const long long strips = (long long)p.n_img * p.tiles_x, ctas = std::max(1, sms / ntn);
-    if (strips * p.h > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
-    long long best = -1;
-    for (long long nb = 1; nb <= 4 * ctas / strips + 4 && nb <= (p.h + 1) / 2; nb++) {
-        const int band = (int)((p.h + nb - 1) / nb);
-        if (p.h % band == 1 || band < 2) continue;
-        const long long tasks = strips * ((p.h + band - 1) / band), cost = (tasks + ctas - 1) / ctas * (band + 2);
-        if (best < 0 || cost < best) {
-            best = cost;
-            p.band = band;
-        }
-    }
-    const long long tasks = strips * ((p.h + p.band - 1) / p.band);
-    const int grid = (int)std::min<long long>(tasks, ctas) * ntn;
-    const uint32_t smem = C::res_bytes(kpt) + (uint32_t)C::stages(kpt) * C::STAGE_BYTES + 4u * C::OUT_TILE + 1024u;
-    conv3x3_rows<BK, CPS><<<grid, 32 * (kEpiWarps + 2), smem, s>>>(a, b, o, p);
     return cudaGetLastError();
 }
 
@@ -1605,43 +1337,36 @@ extern "C" cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, i
     if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(weights) | reinterpret_cast<uintptr_t>(out)) & 63)
         return cudaErrorMisalignedAddress;
     const bool wide_k = cin % 64 == 0 && in_coff % 64 == 0;
-    // Order of the sums. Without RFK_UNET_ANY_ORDER an accumulator adds its
-    // products in one order, whichever sizes: channel block, tap (32 output
-    // channels), tap row, channel block, column tap (64), or tap, channel block
-    // (128, 256). Another order changes a few bf16 roundings per layer: 1e-5 of a
-    // training loss, nothing in a denoised image (half-float steps are coarser).
-    const bool any = (flags & RFK_UNET_ANY_ORDER) != 0;
-    // Up to 96 output channels with weights that leave room for four input rows
-    // in shared memory: conv3x3_rows (1080p U-Net, against the tiles below: 32 ->
-    // 32 63 / 72 us, 96 -> 32 95 / 174, 32 -> 96 176 / 211, 192 -> 64 100 / 111, 64 -> 64
-    // with up2 56 / 63), except 64 output channels from at most 64 without up2
-    // (32 -> 64 37 / 33).
+    // Order of the sums: an accumulator adds its products in one order, whichever
+    // sizes and whichever kernel: channel block, tap (32 output channels), tap row,
+    // channel block, column tap (64), or tap, channel block (128, 256). So an image
+    // denoised is the image whose loss is computed, bit for bit, and losses are
+    // reproducible. A row-streaming kernel that summed the tap rows in accumulators of
+    // their own took a 1080p denoise from 1.09 to 0.97 ms and moved its half-float
+    // channels by up to 0.007 (3e-4 relative over the image).
     const bool up2 = (flags & RFK_UNET_UP2) != 0;
-    const bool rows = any && cout <= 96 && h >= 2 && (cout != 64 || cin > 64 || up2) &&
-                      (wide_k ? rows_cfg<64, 1>::stages(cin / 64) : rows_cfg<32, 1>::stages(cin / 32)) >= rows_cfg<32, 1>::MIN_STAGES;
-    // 32 dense input channels in the fixed order: conv3x3_walk, if the tiles below
-    // would be of 32 output channels (any order: no faster than conv3x3_rows, 74 us
-    // and 66 for a 1080p image; 32 f32 channels out: slower than the tiles)
-    const bool walk = !any && !up2 && !accumulate && !(flags & RFK_UNET_F32OUT) && cin == 32 && in_cstride == 32 && w % 2 == 0 &&
+    // 32 dense input channels: conv3x3_walk, if the tiles below would be of 32 output
+    // channels (32 f32 channels out: slower than the tiles)
+    const bool walk = !up2 && !accumulate && !(flags & RFK_UNET_F32OUT) && cin == 32 && in_cstride == 32 && w % 2 == 0 &&
                       h >= 2 && pick_bn(cout) == 32;
     if (pool && (!walk || h % 2)) return cudaErrorInvalidValue;
-    const int bn = rows ? 32 : pick_bn(cout);
+    const int bn = pick_bn(cout);
     // tap reuse: 32 output channels (4 rows per tile) load each input channel
     // block once for all nine taps (MODE 2, 32-channel K blocks so that three
     // 52 KB stages fit; it keeps one output tile's weights resident: cout == 32,
     // at most 3 input blocks); 64 (2 rows) once per tap row (MODE 1); 128 (2 rows
-    // sharing each weight tile) once per tap row where the order allows it, 256 (1
+    // sharing each weight tile) once per tap row if there is one channel block, 256 (1
     // row) once per tap (MODE 0: three 32 KB weight tiles and the row leave one stage).
-    const int mode2 = !rows && cout == 32 && cin <= 32 * 3;
+    const int mode2 = cout == 32 && cin <= 32 * 3;
     const int bk = !mode2 && wide_k ? 64 : 32;
-    const int mode = rows ? 1 : mode2 ? 2 : bn <= 64 ? 1 : bn == 128 && (any || cin == bk) ? 1 : 0;
+    const int mode = mode2 ? 2 : bn <= 64 ? 1 : bn == 128 && cin == bk ? 1 : 0;
     CUtensorMap ma, mb;
     const CUtensorMapSwizzle sw = bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     {
         cuuint64_t dims[4] = {(cuuint64_t)in_cstride, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n_img};
         cuuint64_t str[3] = {(cuuint64_t)in_cstride * 2, (cuuint64_t)w * in_cstride * 2, (cuuint64_t)h * w * in_cstride * 2};
-        // image rows and pixel lines of an A box, as rows_cfg and conv_cfg<BK, BN, MODE>
-        const cuuint32_t box_rows = rows || bn == 256 ? 1u : bn == 128 ? 2u : (cuuint32_t)(128 / bn) + (mode == 2 ? 2u : 0u);
+        // image rows and pixel lines of an A box, as conv_cfg<BK, BN, MODE>
+        const cuuint32_t box_rows = bn == 256 ? 1u : bn == 128 ? 2u : (cuuint32_t)(128 / bn) + (mode == 2 ? 2u : 0u);
         cuuint32_t box[4] = {(cuuint32_t)bk, mode ? 136u : 128u, box_rows, 1};
         if (!make_map(&ma, in, 4, dims, str, box, sw)) return cudaErrorInvalidValue;
     }
@@ -1697,10 +1422,6 @@ extern "C" cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, i
             good = make_map(&mo, out, 3, dims, str, box, osw);
         }
         if (!good) return cudaErrorInvalidValue;
-    }
-    if (rows) {
-        if (bk == 64) return launch_rows<64, 1>(ma, mb, mo, p, s);
-        return cin == 96 ? launch_rows<32, 3>(ma, mb, mo, p, s) : launch_rows<32, 1>(ma, mb, mo, p, s);
     }
     if (bk == 64) {
         switch (bn) {
