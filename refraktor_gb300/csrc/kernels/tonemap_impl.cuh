@@ -109,18 +109,20 @@ struct density_counts {
 // (granularity 4: 97 log2 bins, max density) is accumulated in the same pass
 // when `hist` is non-null.
 // Bound by memory once a pixel costs about 100 instructions: with vibrancy 1
-// and gamma >= 1 (the usual genome) the precise build leaves out the three
-// c^(1/gamma) whose weight is 0, and the next pixel's load is in flight while
-// this one is computed. 1920 x 1080 half4 at vibrancy 1: 12.5 us a call, 17.1-18.7
-// with all four powf.
+// and gamma >= 1 (the usual genome) the precise build's short form leaves out the
+// three c^(1/gamma) whose weight is 0, and the next pixel's load is in flight while
+// this one is computed. 1920 x 1080 half4, every pixel lit: 18.5 us a call, 32.9 with
+// all four powf. The other form is bound by these: no load ahead and up to 8 blocks
+// for an SM's 6 (one kernel for both, as the short form: 34.9 us, 640 x 360 8.2 and 6.3).
 struct tonemap_args {
     void* out;
     float gamma, scale_constant, brightness, vibrancy, highlight_power;
 };
 
-// PAIR (fast build): the factor w^(1/gamma) / w by pow_pair; false where a channel's
-// rounding is left open, and nothing is stored.
-template <int C, bool HALF, bool PAIR>
+// SHORT, fast build: the factor w^(1/gamma) / w by pow_pair; false where a channel's
+// rounding is left open, and nothing is stored. SHORT, precise build: vibrancy is 1
+// and gamma 1 or more.
+template <int C, bool HALF, bool SHORT>
 __device__ __forceinline__ bool tonemap_pixel(const tonemap_args& p, size_t i, float4 col, const float2* table, float2 q) {
     if (col.w == 0.0f) {
         pixel_out<C, HALF>::store(p.out, i, 0.0f, 0.0f, 0.0f, 0.0f);
@@ -142,7 +144,7 @@ __device__ __forceinline__ bool tonemap_pixel(const tonemap_args& p, size_t i, f
     col.w *= factor;
     float lr, lgc, lb;
 #ifdef RFK_TONEMAP_FAST
-    if (PAIR) {
+    if (SHORT) {
         float hi, lo;
         if (!pow_pair(col.w, table, q, hi, lo)) return false;
         bool done = scale_pair(col.x, hi, lo, lr);
@@ -165,7 +167,7 @@ __device__ __forceinline__ bool tonemap_pixel(const tonemap_args& p, size_t i, f
 #endif
     if (p.highlight_power >= 0.0f) highlight(lr, lgc, lb, p.highlight_power);
 #ifndef RFK_TONEMAP_FAST
-    if (p.vibrancy == 1.0f && p.gamma >= 1.0f) {
+    if (SHORT) {
         // lerp(c^(1/gamma), l, 1) = l; an infinite channel gives NaN (0) as inf + (inf - inf) does
         lr += col.x - col.x;
         lgc += col.y - col.y;
@@ -191,7 +193,7 @@ __device__ __noinline__ void tonemap_pixel_fp64(tonemap_args p, size_t i, float4
 }
 #endif
 
-// PAIR (fast build): pixels that pow_pair leaves open are put aside, 1 in 120, and
+// SHORT, fast build: pixels that pow_pair leaves open are put aside, 1 in 120, and
 // done by whole warps in FP64 at the block's end; where more come than kOpenPixels (one
 // colour everywhere, densities past pow_pair's range) the rest are done at once.
 // 1366 x 768 float4 with its histogram: 21 us a call, 98 with every power in FP64 (19.5
@@ -203,7 +205,7 @@ constexpr int kBlocksPerSm = 4;
 constexpr int kBlocksPerSm = 6;
 #endif
 
-template <int C, bool HALF, bool PAIR>
+template <int C, bool HALF, bool SHORT>
 __global__ void __launch_bounds__(256, kBlocksPerSm)
     tonemap_kernel(const float4* __restrict__ bins, unsigned size, tonemap_args p, unsigned long long* __restrict__ hist,
                    unsigned long long* __restrict__ max_density, const unsigned long long* __restrict__ q_hits, double q_per_hit
@@ -216,8 +218,8 @@ __global__ void __launch_bounds__(256, kBlocksPerSm)
     float2 *table = nullptr, q = {0.0f, 0.0f};
 #ifdef RFK_TONEMAP_FAST
     __shared__ float2 table_sm[32];
-    __shared__ unsigned open[PAIR ? kOpenPixels : 1], nopen;
-    if (PAIR) {
+    __shared__ unsigned open[SHORT ? kOpenPixels : 1], nopen;
+    if (SHORT) {
         if (threadIdx.x < 32) table_sm[threadIdx.x] = pt.t[threadIdx.x];
         if (threadIdx.x == 0) nopen = 0;
         __syncthreads();
@@ -235,18 +237,18 @@ __global__ void __launch_bounds__(256, kBlocksPerSm)
     float my_max = 0.0f;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    float4 next = i < size ? bins[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 next = SHORT && i < size ? bins[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (; i < size; i += stride) {
-        const float4 col = next;
-        if (i + stride < size) next = bins[i + stride];
+        const float4 col = SHORT ? next : bins[i];
+        if (SHORT && i + stride < size) next = bins[i + stride];
         if (hist) {
             atomicAdd(&counts.bins[density_counts::bin(col.w, log_div)], 1u);
             if (col.w >= 1.0f) my_max = fmaxf(my_max, col.w);
         }
-        const bool done = tonemap_pixel<C, HALF, PAIR>(p, i, col, table, q);
+        const bool done = tonemap_pixel<C, HALF, SHORT>(p, i, col, table, q);
         (void)done;
 #ifdef RFK_TONEMAP_FAST
-        if (PAIR && !done) {
+        if (SHORT && !done) {
             const unsigned at = atomicAdd(&nopen, 1u);
             if (at < kOpenPixels) open[at] = (unsigned)i;
             else tonemap_pixel_fp64<C, HALF>(p, i, col);
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(256, kBlocksPerSm)
 #endif
     }
 #ifdef RFK_TONEMAP_FAST
-    if (PAIR) {
+    if (SHORT) {
         __syncthreads();
         const unsigned n = min(nopen, kOpenPixels);
         for (unsigned k = threadIdx.x; k < n; k += blockDim.x) tonemap_pixel_fp64<C, HALF>(p, open[k], bins[open[k]]);
@@ -263,14 +265,15 @@ __global__ void __launch_bounds__(256, kBlocksPerSm)
     if (hist) counts.flush(my_max, hist, max_density);
 }
 
-template <bool HALF, int C, bool PAIR>
+template <bool HALF, int C, bool SHORT>
 void launch_form(unsigned blocks, unsigned sms, cudaStream_t s, const float4* bins, unsigned size, const tonemap_args& p,
                  unsigned long long* hist, unsigned long long* max_density, const unsigned long long* q_hits, double q_per_hit) {
-    // one wave of persistent blocks at most
-    if (blocks > sms * kBlocksPerSm) blocks = sms * kBlocksPerSm;
-    tonemap_kernel<C, HALF, PAIR><<<blocks, 256, 0, s>>>(bins, size, p, hist, max_density, q_hits, q_per_hit
+    // persistent blocks: one wave at most in the short form
+    const unsigned cap = sms * (SHORT ? kBlocksPerSm : 8);
+    if (blocks > cap) blocks = cap;
+    tonemap_kernel<C, HALF, SHORT><<<blocks, 256, 0, s>>>(bins, size, p, hist, max_density, q_hits, q_per_hit
 #ifdef RFK_TONEMAP_FAST
-                                                          , PAIR ? make_pow_table(p.gamma) : pow_table{}
+                                                          , SHORT ? make_pow_table(p.gamma) : pow_table{}
 #endif
     );
 }
@@ -280,13 +283,18 @@ void launch(unsigned blocks, unsigned sms, cudaStream_t s, const float4* bins, v
             float brightness, float vibrancy, float highlight_power, unsigned long long* hist,
             unsigned long long* max_density, const unsigned long long* q_hits, double q_per_hit) {
     const tonemap_args p{out, gamma, scale_constant, brightness, vibrancy, highlight_power};
-#if defined(RFK_TONEMAP_FAST) && !defined(RFK_TONEMAP_FP64)
-    if (gamma >= kPowPairGamma) {
-        launch_form<HALF, C, true>(blocks, sms, s, bins, size, p, hist, max_density, q_hits, q_per_hit);
-        return;
-    }
+#ifdef RFK_TONEMAP_FP64
+    const bool is_short = false;
+#elif defined(RFK_TONEMAP_FAST)
+    const bool is_short = gamma >= kPowPairGamma;
+#else
+    const bool is_short = vibrancy == 1.0f && gamma >= 1.0f;
 #endif
-    launch_form<HALF, C, false>(blocks, sms, s, bins, size, p, hist, max_density, q_hits, q_per_hit);
+    if (is_short) {
+        launch_form<HALF, C, true>(blocks, sms, s, bins, size, p, hist, max_density, q_hits, q_per_hit);
+    } else {
+        launch_form<HALF, C, false>(blocks, sms, s, bins, size, p, hist, max_density, q_hits, q_per_hit);
+    }
 }
 
 }  // namespace rfk_tm
