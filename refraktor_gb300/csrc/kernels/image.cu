@@ -348,16 +348,22 @@ __global__ void pipe_probe_kernel(float* __restrict__ out, unsigned iters, int p
 // The reference multiplies in double; a half times 255 has at most 19
 // significant bits, so the FP32 product is the same number, and the kernel is
 // left to memory: a thread takes 4 pixels with 8- or 16-byte loads and 4- or
-// 16-byte stores where they are aligned, else one pixel. 3840 x 2160 half4 to
-// uchar3: 16.6 us; 230 us with FP64 and one pixel a thread.
-template <int CIN, int COUT, bool BYTES>
-__device__ __forceinline__ void convert_pixel(const __half* p, void* out, int swap) {
-    float v[4] = {__half2float(p[0]), __half2float(p[1]), __half2float(p[2]), CIN == 4 ? __half2float(p[CIN - 1]) : 1.0f};
+// 16-byte stores where they are aligned (not to float4 or small float3 images), else
+// one pixel. 3840 x 2160 half4 to uchar3: 16.6 us; 230 us with FP64 and one pixel a
+// thread.
+template <int CIN>
+__device__ __forceinline__ void convert_load(const __half* p, int swap, float (&v)[4]) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[c] = c < CIN ? __half2float(p[c]) : 1.0f;
     if (swap) {
         const float t = v[0];
         v[0] = v[2];
         v[2] = t;
     }
+}
+
+template <int COUT, bool BYTES>
+__device__ __forceinline__ void convert_store(void* out, const float (&v)[4]) {
 #pragma unroll
     for (int c = 0; c < COUT; c++) {
         if (BYTES) {
@@ -372,15 +378,25 @@ __device__ __forceinline__ void convert_pixel(const __half* p, void* out, int sw
 template <int CIN, int COUT, bool BYTES, bool VEC>
 __global__ void __launch_bounds__(256) convert_kernel(const __half* __restrict__ in, void* __restrict__ out, unsigned w,
                                                       unsigned h, int flip_y, int swap) {
-    constexpr unsigned PX = VEC ? 4 : 1;
     constexpr unsigned OUT = COUT * (BYTES ? 1 : 4);  // bytes of an output pixel
     const unsigned n = w * h;
+    float v[4];
+    if (!VEC) {
+        const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+        if (i >= n) return;
+        convert_load<CIN>(in + (size_t)i * CIN, swap, v);  // on its way while the row is worked out
+        unsigned o = i;
+        if (flip_y) o = (h - i / w - 1) * w + i % w;
+        convert_store<COUT, BYTES>(static_cast<unsigned char*>(out) + (size_t)o * OUT, v);
+        return;
+    }
+    constexpr unsigned PX = 4;
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * PX;
     if (i >= n) return;
     size_t o = i;  // with flip_y a group of 4 stays within a row (w % 4 == 0)
     if (flip_y) o = (size_t)(h - (unsigned)i / w - 1) * w + (unsigned)i % w;
     unsigned char* dst = static_cast<unsigned char*>(out) + o * OUT;
-    if (VEC && i + PX <= n) {
+    if (i + PX <= n) {
         __align__(16) __half p[PX * CIN];
         if (CIN == 4) {
             const uint4* src = reinterpret_cast<const uint4*>(in + i * CIN);
@@ -393,7 +409,10 @@ __global__ void __launch_bounds__(256) convert_kernel(const __half* __restrict__
         }
         __align__(16) unsigned char r[PX * OUT];
 #pragma unroll
-        for (unsigned k = 0; k < PX; k++) convert_pixel<CIN, COUT, BYTES>(p + k * CIN, r + k * OUT, swap);
+        for (unsigned k = 0; k < PX; k++) {
+            convert_load<CIN>(p + k * CIN, swap, v);
+            convert_store<COUT, BYTES>(r + k * OUT, v);
+        }
         if (OUT == 3) {
 #pragma unroll
             for (int q = 0; q < 3; q++) reinterpret_cast<unsigned*>(dst)[q] = reinterpret_cast<unsigned*>(r)[q];
@@ -403,7 +422,10 @@ __global__ void __launch_bounds__(256) convert_kernel(const __half* __restrict__
         }
         return;
     }
-    for (unsigned k = 0; k < PX && i + k < n; k++) convert_pixel<CIN, COUT, BYTES>(in + (i + k) * CIN, dst + k * OUT, swap);
+    for (unsigned k = 0; k < PX && i + k < n; k++) {
+        convert_load<CIN>(in + (i + k) * CIN, swap, v);
+        convert_store<COUT, BYTES>(dst + k * OUT, v);
+    }
 }
 
 template <int CIN, int COUT, bool BYTES>
@@ -411,8 +433,16 @@ void launch_convert(const __half* in, void* out, unsigned w, unsigned h, int fli
     const size_t n = (size_t)w * h;
     const uintptr_t in_mask = CIN == 4 ? 15 : 7, out_mask = COUT * (BYTES ? 1 : 4) == 3 ? 3 : 15;
     const bool vec = ((uintptr_t)in & in_mask) == 0 && ((uintptr_t)out & out_mask) == 0 && (!flip_y || w % 4 == 0);
-    if (vec) convert_kernel<CIN, COUT, BYTES, true><<<(unsigned)((n + 1023) / 1024), 256, 0, s>>>(in, out, w, h, flip_y, swap);
-    else convert_kernel<CIN, COUT, BYTES, false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, out, w, h, flip_y, swap);
+    // float4: a pixel fills a 16-byte store by itself (1920 x 1080 half4: 10.6 us, 11.4
+    // with 4 pixels a thread); float3: small images lose threads by it (640 x 360 half3:
+    // 2.60 us, 2.75 with 4 pixels; 1280 x 720 5.41 and 4.80)
+    if constexpr (BYTES || COUT == 3) {
+        if (vec && (BYTES || n >= (1u << 19))) {
+            convert_kernel<CIN, COUT, BYTES, true><<<(unsigned)((n + 1023) / 1024), 256, 0, s>>>(in, out, w, h, flip_y, swap);
+            return;
+        }
+    }
+    convert_kernel<CIN, COUT, BYTES, false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, out, w, h, flip_y, swap);
 }
 
 // Counters of a render (rfk_counters: 0, the earliest start the largest value) and
