@@ -965,13 +965,6 @@ __device__ __forceinline__ void rfk_block_totals(unsigned& my_hits, unsigned& my
     (void)hot;
 }
 
-// Whether the `n` passes up to `pass` hold one whose number is a multiple of
-// 16: the bailout checks read the clock and the host's stop flag (pinned host
-// memory, about a microsecond away) only then, and always after 16 or more.
-__device__ __forceinline__ bool rfk_poll(unsigned long long pass, unsigned n) {
-    return n == 0 || (pass >> 4) != ((pass - n) >> 4);
-}
-
 #ifdef RFK_MINB
 #define RFK_BIN_BOUNDS __launch_bounds__(RFK_BLOCK, RFK_MINB)
 #else
@@ -1027,10 +1020,8 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin(rfk_bin_args a) {
             unsigned bail = 0;
             if (a.quality_target && q >= a.quality_target) bail |= RFK_ST_QUALITY;
             if (a.max_passes && pass >= a.max_passes) bail |= RFK_ST_ITERS;
-            if (rfk_poll(pass, n)) {
-                if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
-                if (a.stop && *a.stop) bail |= RFK_ST_STOP;
-            }
+            if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
+            if (a.stop && *a.stop) bail |= RFK_ST_STOP;
             s_bail = bail;
         }
         __syncthreads();
@@ -1165,10 +1156,8 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_tm(rfk_bin_args a) {
             unsigned bail = 0;
             if (done == (T >= 32 ? 0xFFFFFFFFu : ((1u << T) - 1u))) bail |= RFK_ST_QUALITY;
             if (a.max_passes && total >= a.max_passes) bail |= RFK_ST_ITERS;
-            if (rfk_poll(total, n)) {
-                if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
-                if (a.stop && *a.stop) bail |= RFK_ST_STOP;
-            }
+            if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
+            if (a.stop && *a.stop) bail |= RFK_ST_STOP;
             s_bail = bail;
             int nxt = cur;
             if (!bail && ((done >> cur) & 1u || in_slice >= a.slice)) {
@@ -1383,10 +1372,8 @@ extern "C" __global__ void RFK_BIN_BOUNDS rfk_bin_batch(rfk_batch_args a) {
                 s_draws = 0;
                 unsigned bail = 0;
                 if (q >= U.quality_target) bail |= RFK_ST_QUALITY;
-                if (rfk_poll(pass, n)) {
-                    if (a.stop && *a.stop) bail |= RFK_ST_STOP;
-                    if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
-                }
+                if (a.stop && *a.stop) bail |= RFK_ST_STOP;
+                if (a.time_ns && rfk_time() - s_start >= a.time_ns) bail |= RFK_ST_TIME;
                 s_bail = bail;
                 // a new jitter for the next interval: the other threads wait at
                 // the barrier below and read P only after it
