@@ -180,9 +180,12 @@ void rfk_state_destroy(rfk_state* s);
  * samples, the chains start again from the Hammersley points and run
  * warmup_count passes, the counters and the accumulated quality restart at
  * 0, and the histogram is cleared when `clear` is non-zero (kept otherwise,
- * also an adopted one). Nothing is allocated, so the per-frame cost is the
- * sample upload, the preparation and the warm-up launch. Fails with
- * RFK_E_INVALID while a bin call on the state is pending. */
+ * also an adopted one). The samples go through pinned and device memory that
+ * the state keeps from its warm-up on, and takes more of when more of them come
+ * than before (by half at least; work on other streams is not waited for);
+ * nothing else is allocated, so the per-frame cost is the sample upload, the
+ * preparation and the warm-up launch. Fails with RFK_E_INVALID while a bin call
+ * on the state is pending. */
 rfk_status rfk_state_rewarm(rfk_state* s, const double* samples, size_t nsamples, uint32_t seed, uint32_t warmup_count,
                             int clear, void* stream);
 
