@@ -141,20 +141,14 @@ struct emitter {
                 direct.insert(c);
             }
         }
-        // and values with the same readers share a branch (64 aligned flames:
-        // 63.6 ms of rfk_bin_batch, 63.8 with a branch each; a loop over the live
-        // bits with a switch instead of a test for each variation is 13% slower)
-        unsigned open = 0;  // readers of the values in the branch being written
-        std::ostringstream decl, eval;
         for (auto& cn : db.common_closure(direct)) {
             dsl::emit_env cenv;
             cenv.variation = "common." + cn;
-            if (readers[cn] != open) eval << (open ? "    }\n" : "") << "    if (live & " << readers[cn] << "u) {\n";
-            open = readers[cn];
-            decl << "    R c_" << cn << " = R(0);\n";
-            eval << "        c_" << cn << " = " << dsl::emit_expression(db.common_ast(cn), cenv) << ";\n";
+            out << "    R c_" << cn << " = R(0);\n    if (live & " << readers[cn] << "u) c_" << cn << " = "
+                << dsl::emit_expression(db.common_ast(cn), cenv) << ";\n";
         }
-        out << decl.str() << eval.str() << (open ? "    }\n" : "");
+        // a loop over the live bits with a switch, instead of a test for each variation,
+        // is 13% slower
         size_t off = 10;
         for (size_t v = 0; v < names.size(); v++) {
             const auto& def = db.get_variation(names[v]);
