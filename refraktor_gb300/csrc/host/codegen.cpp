@@ -173,18 +173,26 @@ struct emitter {
 
 // A union-of-variations kernel repeats the code of nearly every variation in
 // every xform, more than the instruction cache holds while the warps of a block
-// run different xforms: half of its time goes into instruction fetch. If the
-// standard xforms (one vlink each) hold the variations of their union twice
-// over or more, and 24 bodies at least, they share one function instead, and
-// each xform's parameters are laid out alike in shared memory:
+// run different xforms: half of its time goes into instruction fetch. From 72
+// bodies on (an xform's variations, added up over the standard xforms of one vlink
+// each) these share one function instead, and each xform's parameters are laid out
+// alike in shared memory:
 //   live mask (bit v: the weight of the union's variation v is not 0), colour,
 //   colour speed, opacity, affine (6), then per variation its weight, parameters
 //   and precalculated parameters (0 where the xform lacks it).
-// 64 heterogeneous flames (8 to 14 variations in each of 12 xforms: 62.3 ms of
-// rfk_bin_batch, 72.1 with a function per xform) and the denoiser's sets qualify;
-// a flame of its own, with one to three variations per xform, does not, and keeps
-// a function per xform with compile-time offsets. Returns the union's names,
-// empty if not shared.
+// G iterations/s of rfk_bin with a function per xform and with the shared one
+// (xforms x variations each of a union; 8 chains per thread, and by default):
+//   24 bodies   12 x 2 of 12   91.6 79.7   96.4 88.4     4 x 6 of 6    89.7 86.9   94.9 95.1
+//   42 to 56     6 x 7 of 14   77.7 70.0   78.6 73.5     4 x 14        61.6 59.8   62.2 63.7
+//   64 to 70    16 x 4 of 8    88.6 84.7   91.4 91.0    10 x 7 of 14   71.1 69.6   75.3 72.9
+//   72          12 x 6 of 12   71.6 73.6   74.7 77.6     6 x 12        68.8 68.5   68.4 73.8
+//   80          16 x 5 of 10   75.8 78.4   79.7 81.7     8 x 10        70.5 72.1   72.1 77.5
+//   84 to 112   12 x 7 of 14   57.8 68.0   63.5 70.7    16 x 7 of 14   38.8 67.3   37.4 70.0
+//   168         12 x 14        24.3 57.5   23.7 61.5
+// So 16 or 64 aligned flames of 12 xforms (118 and 158 bodies: 62.1 ms of rfk_bin_batch
+// with the first, 72.1 with a function per xform) and the denoiser's sets share one; a
+// flame of its own, with one to three variations per xform, keeps a function per xform
+// with compile-time offsets. Returns the union's names, empty if not shared.
 std::vector<std::string> shared_layout(const flamedb& db, const flame& f, size_t& stride) {
     std::map<std::string, const vardata*> all;
     size_t bodies = 0;
@@ -195,7 +203,7 @@ std::vector<std::string> shared_layout(const flamedb& db, const flame& f, size_t
             bodies++;
         }
     }
-    if (f.xforms.size() < 2 || all.size() > 32 || bodies < 24 || bodies < 2 * all.size()) return {};
+    if (all.size() > 32 || bodies < 72) return {};  // 32 bits of the mask, so three xforms or more
     stride = 10;
     std::vector<std::string> names;
     for (auto& [vn, vd] : all) {
