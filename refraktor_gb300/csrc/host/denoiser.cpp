@@ -64,7 +64,8 @@ T* dalloc(size_t count) {
 struct layer {
     layer_def d{};
     float *w = nullptr, *m = nullptr, *v = nullptr, *g = nullptr;
-    float *b = nullptr, *bm = nullptr, *bv = nullptr, *bg = nullptr;
+    float *b = nullptr, *bm = nullptr, *bv = nullptr;
+    double* bg = nullptr;
     bf16 *wf = nullptr, *wb = nullptr;
     size_t nw() const { return (size_t)d.cout * 9 * d.cin; }
 };
@@ -100,8 +101,8 @@ struct workspace {
 
 struct rfk_denoiser {
     layer L[NLAYERS];
-    float* grads = nullptr;  // all layers' g and bg, one after another
-    size_t ngrads = 0;
+    float* grads = nullptr;  // all layers' bg (64-bit sums), then their g
+    size_t ngrads = 0;       // in floats
     int step = 0;
     int* d_err = nullptr;
     double* d_loss = nullptr;
@@ -206,7 +207,7 @@ struct rfk_denoiser {
     void back(workspace& s, int l, const bf16* dy, int n, int h, int w, const bf16* x, int x_cstride, int x_coff, bf16* dx,
               int dx_cstride, int dx_coff, const bf16* mask, cudaStream_t st) {
         const layer& y = L[l];
-        cuda_check(rfk_unet_wgrad3x3_bias(dy, x, x_cstride, x_coff, n, h, w, y.d.cout, y.d.cin, y.g, y.bg, d_err, st), "wgrad");
+        cuda_check(rfk_unet_wgrad3x3_bias64(dy, x, x_cstride, x_coff, n, h, w, y.d.cout, y.d.cin, y.g, y.bg, d_err, st), "wgrad");
         if (dx)
             cuda_check(rfk_unet_conv3x3(dy, n, h, w, y.d.cout, 0, y.d.cout, y.wb, y.d.cin, nullptr, 0, dx, dx_cstride, dx_coff,
                                         mask, y.d.cin, 0, 0, d_err, st),
@@ -350,13 +351,16 @@ rfk_status rfk_denoiser_create(uint64_t seed, rfk_denoiser** out) {
             for (float* p : {y.m, y.v}) cuda_check(cudaMemset(p, 0, nw * sizeof(float)), "zero");
             for (float* p : {y.b, y.bm, y.bv}) cuda_check(cudaMemset(p, 0, y.d.cout * sizeof(float)), "zero");
         }
-        for (auto& y : d->L) d->ngrads += y.nw() + y.d.cout;  // multiples of 4 floats: 16-byte aligned parts
+        for (auto& y : d->L) d->ngrads += y.nw() + 2 * y.d.cout;  // multiples of 4 floats: 16-byte aligned parts
         d->grads = dalloc<float>(d->ngrads);
         float* at = d->grads;
         for (auto& y : d->L) {
+            y.bg = reinterpret_cast<double*>(at);
+            at += 2 * y.d.cout;
+        }
+        for (auto& y : d->L) {
             y.g = at;
-            y.bg = at += y.nw();
-            at += y.d.cout;
+            at += y.nw();
         }
         d->d_err = dalloc<int>(1);
         d->d_loss = dalloc<double>(1);
@@ -488,8 +492,9 @@ rfk_status rfk_denoiser_gradients(rfk_denoiser* d, const float* bins, const floa
         for (auto& y : d->L) {
             cuda_check(cudaMemcpy(grads + o, y.g, y.nw() * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
             o += y.nw();
-            cuda_check(cudaMemcpy(grads + o, y.bg, y.d.cout * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
-            o += y.d.cout;
+            std::vector<double> bg(y.d.cout);
+            cuda_check(cudaMemcpy(bg.data(), y.bg, y.d.cout * sizeof(double), cudaMemcpyDeviceToHost), "D2H");
+            for (double v : bg) grads[o++] = (float)v;
         }
     });
 }

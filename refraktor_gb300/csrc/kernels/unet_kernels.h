@@ -22,7 +22,7 @@ struct rfk_unet_layer {
     float *w, *m, *v;
     const float* g;
     float *b, *bm, *bv;
-    const float* bg;
+    const double* bg;
     void *wf, *wb;
     int cin, cout, live_in, live_out;
 };
@@ -55,6 +55,9 @@ cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cstride, int 
 // The same, and db[n] += sum over pixels of dY[p][n] (db may be null).
 cudaError_t rfk_unet_wgrad3x3_bias(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w, int cout,
                                    int cin, float* dw, float* db, int* err, cudaStream_t s);
+// With db in 64 bits: as many partial sums as there are CTAs meet in it.
+cudaError_t rfk_unet_wgrad3x3_bias64(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w, int cout,
+                                     int cin, float* dw, double* db, int* err, cudaStream_t s);
 
 // Network input (32 bf16 channels per pixel) of a float4 histogram rendered at `spp` and its
 // tonemapped image `base` (float4).

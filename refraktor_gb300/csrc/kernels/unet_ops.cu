@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) adam_kernel(const __grid_constant__ adam_
         static_cast<bf16*>(y.wb)[((size_t)ci * 9 + (8 - t)) * y.cout + co] = h;
     } else if (i - n < y.cout) {
         const int c = i - n;
-        y.b[c] = c < y.live_out ? adam_update(p, y.b[c], y.bm[c], y.bv[c], y.bg[c]) : 0.0f;
+        y.b[c] = c < y.live_out ? adam_update(p, y.b[c], y.bm[c], y.bv[c], (float)y.bg[c]) : 0.0f;
     }
 }
 

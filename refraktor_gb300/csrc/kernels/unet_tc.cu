@@ -754,7 +754,8 @@ struct wgrad_args {
     int kpc;        // stages (wgrad3x3_rows) or rows (wgrad3x3_cols) of a 64-pixel segment per CTA
     int total;      // all of them
     float* dw;      // [cout][9][cin]
-    float* db;      // [cout]: sum of dY (null: not wanted)
+    float* db;      // [cout]: sum of dY, in 32 or 64 bits (both null: not wanted)
+    double* db64;
     int vec;        // dw is 16-byte aligned
     int* err;
 };
@@ -776,7 +777,11 @@ __device__ __forceinline__ void wgrad_add(float* dst, const float (&v)[32], int 
 // Bias gradient on the way: two warps that no MMA or copy needs add up the rows of
 // dY while these are in shared memory (those of the first input channel tile), a
 // pass over dY of its own less per layer (16 images of 512 x 512: 690 us of the
-// 15 layers of a step; the weight gradients take 40 us longer in all).
+// 15 layers of a step; the weight gradients take 90 us longer in all).
+// A lane adds four stages' rows in f32 and those sums in 64 bits, and the CTAs add theirs
+// in 64 bits too: hundreds of them meet in a bias. 128 x 512 pixels of 32 channels: an
+// error of 3e-10 of sum |dY|; 6e-9 in f32 alone (50 us less per step of 16 images), 1.5e-9
+// with the pass over dY, whose blocks are few there.
 // One row of 64 pixels x CO channels as TMA left it (swizzled 64- or 128-byte
 // pixel lines), CO / 8 lanes to a pixel, by thread t of 64; acc: this lane's 8 channels.
 template <int CO>
@@ -796,15 +801,29 @@ __device__ __forceinline__ void bias_row(const uint8_t* row, int t, float (&acc)
     }
 }
 
-// The warp's sums of its lanes with the same channels, into db[0 .. min(CO, n)).
+constexpr int kBiasStages = 4;  // of f32 sums
+
+__device__ __forceinline__ void bias_fold(float (&acc)[8], double (&sum)[8]) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        sum[j] += (double)acc[j];
+        acc[j] = 0.0f;
+    }
+}
+
+// The warp's sums of its lanes with the same channels, into channels c0 ..
+// min(c0 + CO, cout) - 1.
 template <int CO>
-__device__ __forceinline__ void bias_add(float* db, int n, int lane, float (&acc)[8]) {
+__device__ __forceinline__ void bias_add(const wgrad_args& p, int c0, int lane, double (&sum)[8]) {
     constexpr int L = CO / 8;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
 #pragma unroll
-        for (int o = L; o < 32; o *= 2) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-        if (lane < L && lane * 8 + j < n) atomicAdd(db + lane * 8 + j, acc[j]);
+        for (int o = L; o < 32; o *= 2) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+        const int c = c0 + lane * 8 + j;
+        if (lane >= L || c >= p.cout) continue;
+        if (p.db64) atomicAdd(p.db64 + c, sum[j]);
+        else atomicAdd(p.db + c, (float)sum[j]);
     }
 }
 
@@ -855,7 +874,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUt
     int nk = p.total - kb0;
     if (nk > p.kpc) nk = p.kpc;
     if (nk < 0) nk = 0;
-    const bool bias = p.db != nullptr && blockIdx.y == 0;
+    const bool bias = (p.db || p.db64) && blockIdx.y == 0;
 
     if (warp == 0) tc::tmem_alloc(&tmem_base, C::ACCS * C::ACC_COLS);
     if (threadIdx.x == 32) {
@@ -930,6 +949,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUt
     } else if (warp >= 2 && bias) {
         const int t = threadIdx.x - 64;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        double sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int kb = 0; kb < nk; kb++) {
             const int s = kb % C::STAGES, r = kb / C::STAGES;
             if (!tc::all_lanes(tc::mbar_wait(&full[s], r & 1))) {
@@ -940,9 +960,11 @@ __global__ void __launch_bounds__(128) wgrad3x3_rows(const __grid_constant__ CUt
             for (int y = 1; y <= C::R; y++) bias_row<CO>(sa + y * C::A_GROUP, t, acc);  // rows past the image are zero
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
+            if (kb % kBiasStages == kBiasStages - 1) bias_fold(acc, sum);
         }
         __syncwarp();
-        bias_add<CO>(p.db, CO, lane, acc);
+        bias_fold(acc, sum);
+        bias_add<CO>(p, 0, lane, sum);
     }
     __syncwarp();
 
@@ -1004,7 +1026,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUt
     const int segs_x = p.w / 64;
     // rows of this CTA, counted down the columns one after another
     const int row0 = blockIdx.x * p.kpc, row1 = min(row0 + p.kpc, p.total);
-    const bool bias = p.db != nullptr && c0 == 0;
+    const bool bias = (p.db || p.db64) && c0 == 0;
 
     if (warp == 0) tc::tmem_alloc(&tmem_base, 512u);
     if (threadIdx.x == 32) {
@@ -1093,6 +1115,7 @@ __global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUt
     } else if (warp >= 2 && bias) {
         const int t = threadIdx.x - 64;
         float lo[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hi[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        double lo_sum[8] = {0, 0, 0, 0, 0, 0, 0, 0}, hi_sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         bool ok = true;
         int k = 0;
         for (int row = row0; ok && row < row1;) {
@@ -1108,13 +1131,19 @@ __global__ void __launch_bounds__(128) wgrad3x3_cols(const __grid_constant__ CUt
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[s]);
+                if (k % kBiasStages == kBiasStages - 1) {
+                    bias_fold(lo, lo_sum);
+                    bias_fold(hi, hi_sum);
+                }
             }
             row += y1 - y0;
         }
         if (!ok && lane == 0) atomicExch(&s_fail, 1);
         __syncwarp();
-        bias_add<64>(p.db + m0, p.cout - m0, lane, lo);
-        bias_add<64>(p.db + m0 + 64, p.cout - m0 - 64, lane, hi);
+        bias_fold(lo, lo_sum);
+        bias_fold(hi, hi_sum);
+        bias_add<64>(p, m0, lane, lo_sum);
+        bias_add<64>(p, m0 + 64, lane, hi_sum);
     }
     __syncwarp();
 
@@ -1274,8 +1303,9 @@ cudaError_t launch_wgrad_rows(const void* dy, const void* x, int x_cstride, wgra
     const long long total = (long long)p.n_img * ((p.h + C::R - 1) / C::R) * (p.w / 64);
     if (total > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     p.total = (int)total;
-    // every SM full once (two CTAs: twice): partial sums at least as short as
-    // wgrad3x3_tc's
+    // every SM full once (two CTAs: twice). The rounding error of a sum grows with its
+    // length: 16 images of 256 x 256, 64 -> 64: 7.0e-6 relative, 8.0e-6 with a box and a
+    // launch per tap.
     const int ntiles = p.cin / BN;
     const int splits = (int)std::min<long long>(total, std::max(1, sm_count_cached() * C::CTAS * (C::CTAS == 2 ? 2 : 1) / ntiles));
     p.kpc = (p.total + splits - 1) / splits;
@@ -1300,10 +1330,12 @@ cudaError_t launch_wgrad_cols(const void* dy, const void* x, int x_cstride, wgra
     const long long total = (long long)p.n_img * p.h * (p.w / 64);
     if (total > 0x7FFFFFFFLL) return cudaErrorInvalidValue;
     p.total = (int)total;
-    // Partial sums of at least two waves of CTAs, and at least 45 over the tiles of
-    // 256 input channels: the rounding error of a sum grows with its length (16
-    // images of 128 x 128, 128 -> 128: 84.6 us and a relative error of 5.8e-6 with
-    // one wave, 99.0 and 2.6e-6 with two, 111 and 1.7e-6 with three).
+    // Partial sums of at least two waves of CTAs: the rounding error of a sum grows
+    // with its length (16 images of 128 x 128, 128 -> 128: 84.6 us and a relative error
+    // of 5.8e-6 with one wave, 99.0 and 2.6e-6 with two, 111 and 1.7e-6 with three; 4.8e-6
+    // with the boxes per tap). And at least the 45 for each 256 input channels that the
+    // boxes per tap had, for at 256 -> 256 (64 x 64) two waves are fewer: 92.8 us and
+    // 2.6e-6, with 45 103.1 and 1.7e-6, with 90 119.5 and 0.9e-6, the boxes 193 and 2.1e-6.
     const int mtiles = (p.cout + 127) / 128, tiles = mtiles * (p.cin / C::BN), sms = sm_count_cached();
     const int least = (45 + mtiles * (p.cin / pick_bn(p.cin)) - 1) / (mtiles * (p.cin / pick_bn(p.cin)));
     const int waves = std::max(2, (least * tiles + sms - 1) / sms);
@@ -1312,6 +1344,29 @@ cudaError_t launch_wgrad_cols(const void* dy, const void* x, int x_cstride, wgra
     dim3 grid((unsigned)((p.total + p.kpc - 1) / p.kpc), (unsigned)tiles);
     wgrad3x3_cols<<<grid, 128, C::SMEM, s>>>(ma, mb, p);
     return cudaGetLastError();
+}
+
+cudaError_t launch_wgrad(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w, int cout, int cin,
+                         float* dw, float* db, double* db64, int* err, cudaStream_t s) {
+    if (w % 64 || cin % 32 || cout <= 0 || cout % 32 || n_img <= 0 || h <= 0) return cudaErrorInvalidValue;
+    if (x_coff % 32 || x_cstride % 32 || x_coff + cin > x_cstride) return cudaErrorInvalidValue;
+    if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 63) return cudaErrorMisalignedAddress;
+    wgrad_args p{};
+    p.n_img = n_img;
+    p.h = h;
+    p.w = w;
+    p.cout = cout;
+    p.cin = cin;
+    p.x_coff = x_coff;
+    p.dw = dw;
+    p.db = db;
+    p.db64 = db64;
+    p.vec = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
+    p.err = err;
+    if (cout > 64) return launch_wgrad_cols(dy, x, x_cstride, p, s);
+    if (cout == 32)
+        return cin % 64 ? launch_wgrad_rows<32, 32>(dy, x, x_cstride, p, s) : launch_wgrad_rows<32, 64>(dy, x, x_cstride, p, s);
+    return cin % 64 ? launch_wgrad_rows<64, 32>(dy, x, x_cstride, p, s) : launch_wgrad_rows<64, 64>(dy, x, x_cstride, p, s);
 }
 
 }  // namespace
@@ -1441,27 +1496,15 @@ extern "C" cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, i
 
 extern "C" cudaError_t rfk_unet_wgrad3x3(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w,
                                          int cout, int cin, float* dw, int* err, cudaStream_t s) {
-    return rfk_unet_wgrad3x3_bias(dy, x, x_cstride, x_coff, n_img, h, w, cout, cin, dw, nullptr, err, s);
+    return launch_wgrad(dy, x, x_cstride, x_coff, n_img, h, w, cout, cin, dw, nullptr, nullptr, err, s);
 }
 
 extern "C" cudaError_t rfk_unet_wgrad3x3_bias(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w,
                                               int cout, int cin, float* dw, float* db, int* err, cudaStream_t s) {
-    if (w % 64 || cin % 32 || cout <= 0 || cout % 32 || n_img <= 0 || h <= 0) return cudaErrorInvalidValue;
-    if (x_coff % 32 || x_cstride % 32 || x_coff + cin > x_cstride) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x)) & 63) return cudaErrorMisalignedAddress;
-    wgrad_args p{};
-    p.n_img = n_img;
-    p.h = h;
-    p.w = w;
-    p.cout = cout;
-    p.cin = cin;
-    p.x_coff = x_coff;
-    p.dw = dw;
-    p.db = db;
-    p.vec = (reinterpret_cast<uintptr_t>(dw) & 15) == 0;
-    p.err = err;
-    if (cout > 64) return launch_wgrad_cols(dy, x, x_cstride, p, s);
-    if (cout == 32)
-        return cin % 64 ? launch_wgrad_rows<32, 32>(dy, x, x_cstride, p, s) : launch_wgrad_rows<32, 64>(dy, x, x_cstride, p, s);
-    return cin % 64 ? launch_wgrad_rows<64, 32>(dy, x, x_cstride, p, s) : launch_wgrad_rows<64, 64>(dy, x, x_cstride, p, s);
+    return launch_wgrad(dy, x, x_cstride, x_coff, n_img, h, w, cout, cin, dw, db, nullptr, err, s);
+}
+
+extern "C" cudaError_t rfk_unet_wgrad3x3_bias64(const void* dy, const void* x, int x_cstride, int x_coff, int n_img, int h, int w,
+                                                int cout, int cin, float* dw, double* db, int* err, cudaStream_t s) {
+    return launch_wgrad(dy, x, x_cstride, x_coff, n_img, h, w, cout, cin, dw, nullptr, db, err, s);
 }

@@ -47,3 +47,23 @@ def test_whole_numbers_are_exact_round_the_ring(n, h, w, cin, cout):
     assert int(err.item()) == 0
     assert torch.equal(dw.double(), _taps(dy.double(), x.double()))
     assert torch.equal(db.double(), dy.double().sum((0, 1, 2)))
+
+
+@pytest.mark.parametrize("n,h,w,cout", [(4, 256, 256, 32), (2, 511, 256, 64), (3, 345, 256, 128), (3, 345, 256, 96)])
+def test_bias_sums_past_24_bits_are_exact(n, h, w, cout):
+    """Sums of about 3.4e7 whole numbers in steps of 1: exact in 64 bits, not in f32."""
+    L = lr.lib()
+    L.rfk_unet_wgrad3x3_bias64.restype = C.c_int
+    L.rfk_unet_wgrad3x3_bias64.argtypes = [C.c_void_p, C.c_void_p] + [C.c_int] * 7 + [C.c_void_p] * 4
+    g = torch.Generator(device="cuda").manual_seed(cout + h)
+    dy = torch.randint(0, 256, (n, h, w, cout), device="cuda", generator=g).bfloat16()
+    x = torch.zeros((n, h, w, 32), device="cuda", dtype=torch.bfloat16)
+    dw, db = torch.zeros(cout, 9, 32, device="cuda"), torch.full((cout + 2,), 0.5, device="cuda", dtype=torch.float64)
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert L.rfk_unet_wgrad3x3_bias64(dy.data_ptr(), x.data_ptr(), 32, 0, n, h, w, cout, 32, dw.data_ptr(), db.data_ptr(),
+                                      err.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and not dw.any()
+    want = dy.double().sum((0, 1, 2))
+    assert float(want.min()) > 2 ** 24
+    assert torch.equal(db[:cout], want + 0.5) and bool((db[cout:] == 0.5).all())
