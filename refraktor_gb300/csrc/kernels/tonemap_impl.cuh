@@ -168,10 +168,12 @@ __device__ __forceinline__ bool tonemap_pixel(const tonemap_args& p, size_t i, f
     if (p.highlight_power >= 0.0f) highlight(lr, lgc, lb, p.highlight_power);
 #ifndef RFK_TONEMAP_FAST
     if (SHORT) {
-        // lerp(c^(1/gamma), l, 1) = l; an infinite channel gives NaN (0) as inf + (inf - inf) does
-        lr += col.x - col.x;
-        lgc += col.y - col.y;
-        lb += col.z - col.z;
+        // lerp(c^(1/gamma), l, 1) = l, and NaN (0) where c^(1/gamma) is infinite or NaN: for an
+        // infinite c, and a negative one unless gamma is 1 (a highlight lifts its l above 0)
+        const float negative = inv_gamma_f < 1.0f ? nanf("") : 0.0f;
+        lr += col.x < 0.0f ? negative : col.x - col.x;
+        lgc += col.y < 0.0f ? negative : col.y - col.y;
+        lb += col.z < 0.0f ? negative : col.z - col.z;
     } else
 #endif
     {
