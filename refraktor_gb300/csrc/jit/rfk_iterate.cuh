@@ -555,12 +555,12 @@ __device__ __forceinline__ void rfk_cache_add(rfk_cache& cc, float4* __restrict_
 // copy, channel), added with integer shared-memory atomics: on GB300 these
 // take 0.87x the time of the chain step with float shared-memory atomics on
 // the 1080p bench genome. A copy sums the draws of RFK_BLOCK * RFK_CPT /
-// RFK_HOT_COPIES chains over at most RFK_MAX_CHECK + RFK_DISC_PASSES passes
-// between flushes, each channel at most 1 (a draw with opacity above 1, which
-// only a spline overshoot gives, goes out as a red.v4), so the shift below,
-// which keeps RFK_MAX_CHECK passes under 2^31, keeps every sum under 2^32. One quantum is 2^-17 at the bench's launch shape: 7.6e-6 per
-// draw against colour contributions of up to the opacity; an opacity of 1 is
-// exact.
+// RFK_HOT_COPIES chains over at most RFK_MAX_CHECK passes between flushes (a
+// rebuild flushes, once a cycle), each channel at most 1 (a draw with opacity above
+// 1, which only a spline overshoot gives, goes out as a red.v4), so the shift below
+// keeps every sum under 2^31. One quantum is 2^-17 at the bench's launch shape:
+// 7.6e-6 per draw against colour contributions of up to the opacity; an opacity of
+// 1 is exact.
 #define RFK_HOT_MAX 64
 #define RFK_HOT_BUCKETS 128  // two ways each
 #define RFK_HOT_COPIES 4

@@ -95,7 +95,8 @@ struct conv_cfg {
     // output staging: two tiles of 128 pixels x OC channels
     static constexpr int OC = BN % 64 == 0 ? 64 : 32;
     static constexpr uint32_t OUT_TILE = 128u * OC * 2u;
-    // one persistent CTA per SM: as many stages as fit in ~208 KB, at most 8
+    // one persistent CTA per SM: as many stages as fit in 224 KB with the weights and
+    // the output tiles, at most 8
     static constexpr uint32_t BUDGET = 229376u - 2u * OUT_TILE;
     static constexpr int STAGES = ((BUDGET - B_RES) / STAGE_BYTES > 8) ? 8 : (int)((BUDGET - B_RES) / STAGE_BYTES);
     static constexpr uint32_t SMEM = B_RES + STAGES * STAGE_BYTES + 2u * OUT_TILE + 1024u;
@@ -291,8 +292,9 @@ __device__ __forceinline__ void conv_epilogue_tma(const conv_args& p, const CUte
 // output channels) t = blockIdx.x, blockIdx.x + gridDim.x, ...
 // Warps 0-7: epilogue (warp w reads TMEM lane quarter w % 4, column half
 // w / 4), warp 8 lane 0: TMA producer over a ring of stages that runs across
-// tiles, warp 9 lane 0: MMA issuer. Two TMEM accumulators: the MMAs of tile
-// i + 1 run while the epilogue drains tile i (acc_full / acc_empty barriers).
+// tiles, warp 9: MMA issuer (the whole warp, see tc::mma_bf16). Two TMEM
+// accumulators: the MMAs of tile i + 1 run while the epilogue drains tile i
+// (acc_full / acc_empty barriers).
 template <int BK, int BN, int MODE>
 __global__ void __launch_bounds__(320, 1) conv3x3_tc(const __grid_constant__ CUtensorMap tmA,
                                                      const __grid_constant__ CUtensorMap tmB,
