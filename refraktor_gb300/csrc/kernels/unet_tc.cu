@@ -779,11 +779,11 @@ __device__ __forceinline__ void wgrad_add(float* dst, const float (&v)[32], int 
 // Bias gradient on the way: two warps that no MMA or copy needs add up the rows of
 // dY while these are in shared memory (those of the first input channel tile), a
 // pass over dY of its own less per layer (16 images of 512 x 512: 690 us of the
-// 15 layers of a step; the weight gradients take 90 us longer in all).
-// A lane adds four stages' rows in f32 and those sums in 64 bits, and the CTAs add theirs
+// 15 layers of a step; the weight gradients take 50 us longer in all).
+// A lane adds 16 stages' rows in f32 and those sums in 64 bits, and the CTAs add theirs
 // in 64 bits too: hundreds of them meet in a bias. 128 x 512 pixels of 32 channels: an
-// error of 3e-10 of sum |dY|; 6e-9 in f32 alone (50 us less per step of 16 images), 1.5e-9
-// with the pass over dY, whose blocks are few there.
+// error of 3e-10 of sum |dY|; 6e-9 in f32 alone, 1.5e-9 with the pass over dY, whose
+// blocks are few there.
 // One row of 64 pixels x CO channels as TMA left it (swizzled 64- or 128-byte
 // pixel lines), CO / 8 lanes to a pixel, by thread t of 64; acc: this lane's 8 channels.
 template <int CO>
@@ -803,7 +803,7 @@ __device__ __forceinline__ void bias_row(const uint8_t* row, int t, float (&acc)
     }
 }
 
-constexpr int kBiasStages = 4;  // of f32 sums
+constexpr int kBiasStages = 16;  // of f32 sums (4: the folds hold wgrad3x3_cols up, 45 us a step)
 
 __device__ __forceinline__ void bias_fold(float (&acc)[8], double (&sum)[8]) {
 #pragma unroll
