@@ -41,7 +41,7 @@ cudaError_t rfk_unet_conv3x3(const void* in, int n_img, int h, int w, int in_cst
                              cudaStream_t s);
 
 // The same, and the 2x2 average pool of the output as a dense [n][h/2][w/2][cout] tensor (pool may be
-// null): for 32 dense input channels in the fixed order, bf16 outputs and even h and w.
+// null): for 32 dense input channels, bf16 outputs and even h and w.
 cudaError_t rfk_unet_conv3x3_pool(const void* in, int n_img, int h, int w, int in_cstride, int in_coff, int cin,
                                   const void* weights, int cout, const float* bias, int flags, void* out, int out_cstride,
                                   int out_coff, const void* mask, int mask_cstride, int mask_coff, int accumulate, void* pool,
